@@ -12,7 +12,8 @@ class QuantumCircuit:
     """Gate list applied in order by ``update_quantum_state`` (cppsim circuit.cpp:46-57).
 
     ``mode="gate_by_gate"`` launches one kernel per gate (the reference's method);
-    ``mode="staged"`` applies several gates per HBM pass with the same per-gate arithmetic;
+    ``mode="staged"`` applies several gates per HBM pass, each with its own arithmetic (specialised passes
+    write one-qubit gates as rotations and diagonals: equal up to rounding);
     ``mode="staged_fused"`` first composes runs of gates into k-qubit dense blocks in FP64 (k chosen
     per circuit by timing, or forced with ``set_fusion``), then stages them.
     """

@@ -2,7 +2,7 @@
 // executors.  QS_EXEC_GATE_BY_GATE launches one kernel per gate, the reference's method
 // (QuantumCircuit::update_quantum_state, circuit.cpp:46-57, dispatching each gate to its csim
 // kernel).  QS_EXEC_STAGED hands the list to the pass scheduler (staged.cpp), which applies several
-// gates per HBM pass with the same per-gate arithmetic.
+// gates per HBM pass.
 #include "circuit.hpp"
 
 #include <cmath>
@@ -199,6 +199,8 @@ std::vector<GateRec> dm_vector_gates(const std::vector<GateRec>& G, UINT n) {
             for (UINT t : g.targets) s.targets.push_back(t);
             for (UINT t : g.targets) s.targets.push_back(t + n);
             s.matrix = depolarizing_superoperator(k, g.prob);
+            s.depol = (int)k;
+            s.prob = g.prob;
             out.push_back(s);
             continue;
         }
@@ -423,7 +425,7 @@ QS_API int qs_circuit_update_density_matrix(qs_circuit_t circuit, void* rho, QS_
     if (!c->dm_vec) {
         auto v = std::make_shared<Circuit>();
         v->n = 2 * c->n;
-        v->gates = qs::dm_vector_gates(c->gates, c->n);
+        v->gates = qs::dm_vector_gates(qs::merge_depolarizing(c->gates), c->n);
         v->fusion_k = c->fusion_k;
         c->dm_vec = v;
     }

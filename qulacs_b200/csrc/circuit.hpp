@@ -22,6 +22,13 @@ struct GateRec {
     std::vector<UINT> pauli_ids;
     double angle = 0.;
     double prob = 0.;
+    int depol = 0;            // a depolarizing channel of `prob` on 1 or 2 qubits as a superoperator (dm_vector_gates)
+    // rotation_form's gates carry their parameters in extended precision, so that each reaches the device
+    // rounded once: an RY's (cosine, sine), a one-qubit DIAGONAL's two entries
+    bool extended = false;
+    bool free_phase = false;  // a diagonal whose phase is a parameter: never treated as a fixed sign or identity
+    long double xc = 0.L, xs = 0.L;
+    std::complex<long double> xd[2];
 
     std::vector<UINT> qubits() const;                      // targets then controls
     std::vector<std::complex<double>> dense_matrix() const;  // on targets only
@@ -32,14 +39,16 @@ struct StagedPlan;  // staged.cpp
 struct Circuit {
     UINT n = 0;
     std::vector<GateRec> gates;
-    // cached staged schedule (built on first staged run for a given dim)
+    // cached staged schedule (built on first staged run for a given dim) of the gates in rotation form
     std::shared_ptr<StagedPlan> plan;
+    std::vector<GateRec> rgates;
     // cached fused complex64 plan (fused_c64.cu)
     std::shared_ptr<void> fused;
     ITYPE fused_dim = 0;
     // FP64-fused gate list and its staged schedule (QS_EXEC_STAGED_FUSED, staged.cu)
     int fusion_k = -1;              // forced block size, or -1: the autotuner chooses
     int fused_k = -1;               // block size of fgates (valid while fplan is set)
+    size_t fused_count = 0;         // gates after the fusion
     int fused_tile_bits = 12;       // tile qubits of fplan's passes
     std::vector<GateRec> fgates;
     std::shared_ptr<StagedPlan> fplan;
@@ -72,6 +81,7 @@ struct Circuit {
         bgates.clear();
         bk = -1;
         plan.reset();
+        rgates.clear();
         fused.reset();
         fused_dim = 0;
         fplan.reset();
@@ -110,5 +120,14 @@ int batch_update_fused_c64(Circuit* const* cs, void* const* states, UINT count, 
 // kb-qubit block matrix U (2^kb x 2^kb, row-major); and the greedy k-qubit fusion of a gate list.
 void apply_gate_to_block(std::vector<std::complex<double>>& U, int kb, const GateRec& g, const std::vector<int>& pos);
 std::vector<GateRec> fuse_gates(const std::vector<GateRec>& G, int k);
+// fusion.cpp: each run of one-qubit unitaries on a qubit as a diagonal and a real rotation, the rotation's
+// second diagonal carried forward (through controls, CZ and other diagonals) into the next run.
+std::vector<GateRec> rotation_form(const std::vector<GateRec>& G);
+// fusion.cpp: the gate list that the staged executors run at block size k; *blocks: gates after the fusion
+// (fuse_gates' count).
+std::vector<GateRec> executor_gates(const std::vector<GateRec>& G, int k, size_t* blocks = nullptr);
+// fusion.cpp: one-qubit depolarizing channels of a density-matrix circuit carried forward past one-qubit
+// unitaries and merged.
+std::vector<GateRec> merge_depolarizing(const std::vector<GateRec>& G);
 
 }  // namespace qs

@@ -4,11 +4,19 @@
 // The generic pass kernel (k_staged_pass, staged.cu) interprets each phase's op list: per op it loads
 // the op record and its matrix from memory, branches through a 128-case switch, and returns its 16
 // amplitudes to the registers the switch fixed, which costs register moves at every op boundary and an
-// instruction footprint larger than the instruction cache.  Here every tile qubit, phase bit, Gray-code
-// address offset and matrix entry is a compile-time constant: the phases become straight-line code,
-// matrix entries are read as constant-bank operands, and the compiler allocates registers across op
-// boundaries.  The arithmetic of each op is the generic kernel's (same fma sequence, same order), and
-// the tile load/store, HBM-direct first/last phases and 16-byte swizzle are the same.
+// instruction footprint larger than the instruction cache.  Here every tile qubit, phase bit, address offset
+// and register index is a compile-time constant: a phase is the straight-line code of its program
+// (phase_program.hpp), and gate parameters are constant-bank operands.
+//
+// What bounds it: a pass needs one read and one write of the state, 16 bytes through shared memory each
+// way per amplitude and inner phase, and the program's FP64 instructions.  The layered circuit at 30 qubits
+// (16 passes, 77 phases, 1296 FP64 instructions per amplitude) has 84 ms of HBM, ~60 ms of shared memory
+// and 75 ms of FP64 time and runs in 139 ms; with one matrix per gate (2400 instructions) it took 212 ms.
+//  * One 16-amplitude coset per thread, so 256 threads and 2 CTAs per SM for a 2^12-amplitude tile
+//    (128 registers): 141 ms, against 159 ms for 128 threads with two cosets each and 3 CTAs per SM
+//    (12 warps, and the coset loop turned parameters into separate constant loads).
+//  * Lanes run over tile bits whose swizzle vectors are independent (lane_order): the density-matrix
+//    circuit of 12 qubits went from 3.6 to 3.1 ms.
 //
 // NVRTC is opened at run time (libnvrtc.so.12); the compiled cubin is loaded with cudaLibraryLoadData,
 // which makes it available to every device context.  Kernels are cached by source text for the life of
@@ -30,6 +38,7 @@
 
 #include "../../include/qulacs_b200.h"
 #include "codegen.hpp"
+#include "phase_program.hpp"
 #include "staged.hpp"
 
 namespace qs {
@@ -119,136 +128,63 @@ __device__ __forceinline__ D2 ldp(const D2* p) {
     asm volatile("ld.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
     return v;
 }
-__device__ __forceinline__ unsigned swz(unsigned u) { return u ^ (((u >> 4) ^ (u >> 7) ^ (u >> 10)) & 7u); }
+__device__ __forceinline__ unsigned swz(unsigned u) { return u ^ (((u >> 3) ^ (u >> 5) ^ (u >> 6) ^ (u >> 8)) & 7u); }
 __device__ __forceinline__ u64 ins0(u64 i, unsigned q) { return ((i >> q) << (q + 1)) | (i & ((1ULL << q) - 1ULL)); }
 
-template <int B> __device__ __forceinline__ void r_dense1(D2 (&r)[16], D2 m0, D2 m1, D2 m2, D2 m3) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << B))) {
-            const D2 x = r[j], y = r[j | (1 << B)];
-            r[j] = cfma(m1, y, cmul(m0, x));
-            r[j | (1 << B)] = cfma(m3, y, cmul(m2, x));
-        }
+// Register steps (phase_program.hpp).  A pair (x, y): the amplitudes where the step's qubit is 0 and 1.
+__device__ __forceinline__ void ry_tan(D2& x, D2& y, double t) {
+    const D2 X = x;
+    x = mk(fma(t, y.x, X.x), fma(t, y.y, X.y));
+    y = mk(fma(-t, X.x, y.x), fma(-t, X.y, y.y));
 }
-template <int B> __device__ __forceinline__ void r_diag1(D2 (&r)[16], D2 d0, D2 d1) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = cmul((j & (1 << B)) ? d1 : d0, r[j]);
+__device__ __forceinline__ void ry_cot(D2& x, D2& y, double u) {
+    const D2 X = x;
+    x = mk(fma(u, X.x, y.x), fma(u, X.y, y.y));
+    y = mk(fma(u, y.x, -X.x), fma(u, y.y, -X.y));
 }
-template <int B> __device__ __forceinline__ void r_rx(D2 (&r)[16], double c, double s) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << B))) {
-            const D2 x = r[j], y = r[j | (1 << B)];
-            r[j] = mk(fma(c, x.x, -s * y.y), fma(c, x.y, s * y.x));
-            r[j | (1 << B)] = mk(fma(c, y.x, -s * x.y), fma(c, y.y, s * x.x));
-        }
+__device__ __forceinline__ void ry_full(D2& x, D2& y, double c, double s) {
+    const D2 X = x;
+    x = mk(fma(c, X.x, s * y.x), fma(c, X.y, s * y.y));
+    y = mk(fma(c, y.x, -s * X.x), fma(c, y.y, -s * X.y));
 }
-template <int B> __device__ __forceinline__ void r_ry(D2 (&r)[16], double c, double s) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << B))) {
-            const D2 x = r[j], y = r[j | (1 << B)];
-            r[j] = mk(fma(c, x.x, s * y.x), fma(c, x.y, s * y.y));
-            r[j | (1 << B)] = mk(fma(c, y.x, -s * x.x), fma(c, y.y, -s * x.y));
-        }
+__device__ __forceinline__ void rx_tan(D2& x, D2& y, double t) {
+    const D2 X = x;
+    x = mk(fma(-t, y.y, X.x), fma(t, y.x, X.y));
+    y = mk(fma(-t, X.y, y.x), fma(t, X.x, y.y));
 }
-template <int C, int T> __device__ __forceinline__ void r_cnot(D2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << C)) && !(j & (1 << T))) {
-            const D2 t = r[j];
-            r[j] = r[j | (1 << T)];
-            r[j | (1 << T)] = t;
-        }
+__device__ __forceinline__ void rx_cot(D2& x, D2& y, double u) {
+    const D2 X = x;
+    x = mk(fma(u, X.x, -y.y), fma(u, X.y, y.x));
+    y = mk(fma(u, y.x, -X.y), fma(u, y.y, X.x));
 }
-template <int A, int B> __device__ __forceinline__ void r_cz(D2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << A)) && (j & (1 << B))) r[j] = mk(-r[j].x, -r[j].y);
+__device__ __forceinline__ void rx_full(D2& x, D2& y, double c, double s) {
+    const D2 X = x;
+    x = mk(fma(c, X.x, -s * y.y), fma(c, X.y, s * y.x));
+    y = mk(fma(c, y.x, -s * X.y), fma(c, y.y, s * X.x));
 }
-template <int A, int B> __device__ __forceinline__ void r_swap(D2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << A)) && !(j & (1 << B))) {
-            const int k = j ^ (1 << A) ^ (1 << B);
-            const D2 t = r[j];
-            r[j] = r[k];
-            r[k] = t;
-        }
+__device__ __forceinline__ void dense1(D2& x, D2& y, D2 m0, D2 m1, D2 m2, D2 m3) {
+    const D2 X = x;
+    x = cfma(m1, y, cmul(m0, X));
+    y = cfma(m3, y, cmul(m2, X));
 }
-template <int A, int B> __device__ __forceinline__ void r_dense2(D2 (&r)[16], const D2 (&p)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A)) && !(j & (1 << B))) {
-            const int o[4] = {j, j | (1 << A), j | (1 << B), j | (1 << A) | (1 << B)};
-            D2 v[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) v[x] = r[o[x]];
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                D2 acc = cmul(p[y * 4], v[0]);
-#pragma unroll
-                for (int x = 1; x < 4; ++x) acc = cfma(p[y * 4 + x], v[x], acc);
-                r[o[y]] = acc;
-            }
-        }
+// One row of a 4 x 4 matrix; the entries are read at their use (volatile), so one row's are live at a time.
+__device__ __forceinline__ D2 row4(const D2* p, D2 a, D2 b, D2 c, D2 d) {
+    return cfma(ldp(p + 3), d, cfma(ldp(p + 2), c, cfma(ldp(p + 1), b, cmul(ldp(p), a))));
 }
-// r_dense2 with the matrix read from a parameter block at each use (volatile loads: only the entries
-// of the row being computed are live).
-template <int A, int B> __device__ __forceinline__ void r_dense2p(D2 (&r)[16], const D2* p) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A)) && !(j & (1 << B))) {
-            const int o[4] = {j, j | (1 << A), j | (1 << B), j | (1 << A) | (1 << B)};
-            D2 v[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) v[x] = r[o[x]];
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                D2 acc = cmul(ldp(p + y * 4), v[0]);
-#pragma unroll
-                for (int x = 1; x < 4; ++x) acc = cfma(ldp(p + y * 4 + x), v[x], acc);
-                r[o[y]] = acc;
-            }
-        }
+__device__ __forceinline__ void dense2(D2& a, D2& b, D2& c, D2& d, const D2* p) {
+    const D2 A = row4(p, a, b, c, d), B = row4(p + 4, a, b, c, d), C = row4(p + 8, a, b, c, d);
+    d = row4(p + 12, a, b, c, d);
+    a = A; b = B; c = C;
 }
-template <int A, int B> __device__ __forceinline__ void r_csel1(D2 (&r)[16], D2 m0, D2 m1, D2 m2, D2 m3, D2 n0, D2 n1,
-                                                                D2 n2, D2 n3) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A))) {
-            const D2 x = r[j], y = r[j | (1 << A)];
-            const bool hi = (j >> B) & 1;
-            r[j] = cfma(hi ? n1 : m1, y, cmul(hi ? n0 : m0, x));
-            r[j | (1 << A)] = cfma(hi ? n3 : m3, y, cmul(hi ? n2 : m2, x));
-        }
+// One-qubit depolarizing channel, scaled by 1 / (1 - q / 2): populations (x, y) mix, coherences shrink.
+__device__ __forceinline__ void mix2(D2& x, D2& y, double t) {
+    const D2 X = x;
+    x = mk(fma(t, y.x, X.x), fma(t, y.y, X.y));
+    y = mk(fma(t, X.x, y.x), fma(t, X.y, y.y));
 }
-template <int A, int B> __device__ __forceinline__ void r_d1_in(D2 (&r)[16], D2 m0, D2 m1, D2 m2, D2 m3) {
-    D2 o[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A))) {
-            const int k = j ^ (1 << A) ^ (1 << B);
-            const D2 x = r[j], y = r[k];
-            o[j] = cfma(m1, y, cmul(m0, x));
-            o[j | (1 << A)] = cfma(m3, y, cmul(m2, x));
-        }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = o[j];
-}
-template <int A, int B> __device__ __forceinline__ void r_d1_out(D2 (&r)[16], D2 m0, D2 m1, D2 m2, D2 m3) {
-    D2 o[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A))) {
-            const D2 x = r[j], y = r[j | (1 << A)];
-            o[j] = cfma(m1, y, cmul(m0, x));
-            o[j ^ (1 << A) ^ (1 << B)] = cfma(m3, y, cmul(m2, x));
-        }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = o[j];
-}
+__device__ __forceinline__ void rscale(D2& x, double k) { x = mk(k * x.x, k * x.y); }
+__device__ __forceinline__ D2 sum4(D2 a, D2 b, D2 c, D2 d) { return mk((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y)); }
+__device__ __forceinline__ void axpy(D2& x, double t, D2 s) { x = mk(fma(t, s.x, x.x), fma(t, s.y, x.y)); }
 )";
 
 // An exact C++17 hexadecimal literal of a double.
@@ -259,13 +195,27 @@ std::string lit(double v) {
 }
 // Gate parameters of a generated kernel: written into the source as literals, or (when `bank` is set)
 // referenced as P.v[i] of the kernel's __grid_constant__ parameter block and collected into `bank`, so
-// the kernel depends only on the pass's structure and is shared by circuits that differ in angles.
+// the kernel depends only on the pass's structure and is shared by circuits that differ in angles.  A
+// reference is a constant-bank operand of the instruction that uses it.
 struct ParamSink {
     std::vector<double2>* bank = nullptr;
+    long half = -1;  // entry whose second double is free
     std::string d2(const double2& v) {
         if (!bank) return "mk(" + lit(v.x) + ", " + lit(v.y) + ")";
         bank->push_back(v);
-        return "ldp(&P.v[" + std::to_string(bank->size() - 1) + "])";
+        return "P.v[z + " + std::to_string(bank->size() - 1) + "]";
+    }
+    std::string d1(double v) {
+        if (!bank) return lit(v);
+        if (half >= 0) {
+            (*bank)[half].y = v;
+            const std::string r = "P.v[z + " + std::to_string(half) + "].y";
+            half = -1;
+            return r;
+        }
+        half = (long)bank->size();
+        bank->push_back(make_double2(v, 0.));
+        return "P.v[z + " + std::to_string(half) + "].x";
     }
 };
 
@@ -277,55 +227,120 @@ std::string u64hex(ITYPE v) {
 
 int gray_bit(int g) { return (g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3; }
 
-unsigned swz_host(unsigned u) { return u ^ (((u >> 4) ^ (u >> 7) ^ (u >> 10)) & 7u); }
+unsigned swz_host(unsigned u) { return QS_SWZ(u); }
 
-void emit_op(std::ostringstream& o, const StOp& op, const double2* pool, ParamSink& ps) {
-    const double2* p = pool + op.param;
-    const int a = op.a, b = op.b;
-    auto d2 = [&](const double2& v) { return ps.d2(v); };
-    switch (op.kind) {
-        case ST_DENSE1:
-            o << "      r_dense1<" << a << ">(r, " << d2(p[0]) << ", " << d2(p[1]) << ", " << d2(p[2]) << ", " << d2(p[3])
-              << ");\n";
+// One step of a phase program on the registers r0..r15.
+void emit_step(std::ostringstream& o, const ProgStep& s, ParamSink& ps) {
+    auto reg = [](int j) { return "r[" + std::to_string(j) + "]"; };
+    // registers by the values of the step's qubits: at(k) for base register b, k = packed qubit values
+    auto coset = [&](int b, int k) {
+        int j = b;
+        for (int i = 0; i < s.nq; ++i)
+            if (((k >> i) & 1) != step_bit(s, i, j)) j ^= s.v[i];
+        return j;
+    };
+    auto bases = [&]() {  // one register of each coset of the step's qubits: all its qubits 0
+        std::vector<int> out;
+        for (int j = 0; j < 16; ++j) {
+            bool zero = true;
+            for (int i = 0; i < s.nq; ++i) zero = zero && !step_bit(s, i, j);
+            if (zero) out.push_back(j);
+        }
+        return out;
+    };
+    switch (s.kind) {
+        case SP_DIAG:
+            for (int j = 0; j < 16; ++j)
+                if ((s.mask >> j) & 1) o << "      " << reg(j) << " = cmul(" << ps.d2(s.par[j]) << ", " << reg(j) << ");\n";
             break;
-        case ST_DIAG1: o << "      r_diag1<" << a << ">(r, " << d2(p[0]) << ", " << d2(p[1]) << ");\n"; break;
-        case ST_RX:
-        case ST_RY:
-            o << "      { const D2 cs = " << d2(p[0]) << "; r_" << (op.kind == ST_RX ? "rx" : "ry") << "<" << a
-              << ">(r, cs.x, cs.y); }\n";
+        case SP_SIGN:
+            for (int j = 0; j < 16; ++j)
+                if ((s.mask >> j) & 1) o << "      " << reg(j) << " = mk(-" << reg(j) << ".x, -" << reg(j) << ".y);\n";
             break;
-        case ST_CNOT: o << "      r_cnot<" << a << ", " << b << ">(r);\n"; break;
-        case ST_CZ: o << "      r_cz<" << a << ", " << b << ">(r);\n"; break;
-        case ST_SWAP: o << "      r_swap<" << a << ", " << b << ">(r);\n"; break;
-        case ST_DENSE2: {
-            if (ps.bank) {  // the 16 entries as one run of the parameter block, read row by row
-                const size_t first = ps.bank->size();
-                for (int i = 0; i < 16; ++i) ps.bank->push_back(p[i]);
-                o << "      r_dense2p<" << a << ", " << b << ">(r, &P.v[" << first << "]);\n";
-                break;
+        case SP_CNOT:
+        case SP_SWAP:
+        case SP_X:  // moves between registers: names, once the compiler has unrolled them
+            for (int j = 0; j < 16; ++j) {
+                const int b0 = step_bit(s, 0, j), b1 = s.nq > 1 ? step_bit(s, 1, j) : 0;
+                const bool first = s.kind == SP_CNOT ? b0 && !b1 : s.kind == SP_SWAP ? b0 && !b1 : !b0;
+                const int k = s.kind == SP_CNOT ? j ^ s.v[1] : s.kind == SP_SWAP ? j ^ s.v[0] ^ s.v[1] : j ^ s.v[0];
+                if (first) o << "      { const D2 t = " << reg(j) << "; " << reg(j) << " = " << reg(k) << "; " << reg(k) << " = t; }\n";
             }
-            o << "      { const D2 m[16] = {";
-            for (int i = 0; i < 16; ++i) o << (i ? ", " : "") << d2(p[i]);
-            o << "}; r_dense2<" << a << ", " << b << ">(r, m); }\n";
+            break;
+        case SP_SCALE: {
+            const std::string z = s.form ? ps.d2(s.par[0]) : ps.d1(s.par[0].x);
+            for (int j = 0; j < 16; ++j) {
+                if (s.form) o << "      " << reg(j) << " = cmul(" << z << ", " << reg(j) << ");\n";
+                else o << "      rscale(" << reg(j) << ", " << z << ");\n";
+            }
             break;
         }
-        case ST_CSEL1:
-            o << "      r_csel1<" << a << ", " << b << ">(r";
-            for (int i = 0; i < 8; ++i) o << ", " << d2(p[i]);
-            o << ");\n";
+        case SP_ROT: {
+            static const char* names[] = {"ry_tan", "ry_cot", "ry_full", "rx_tan", "rx_cot", "rx_full"};
+            const bool full = s.form == RF_Y_FULL || s.form == RF_X_FULL;
+            std::string args = ps.d1(s.par[0].x);
+            if (full) args += ", " + ps.d1(s.par[0].y);
+            for (int j : bases())
+                o << "      " << names[s.form] << "(" << reg(j) << ", " << reg(coset(j, 1)) << ", " << args << ");\n";
             break;
-        case ST_D1_IN:
-        case ST_D1_OUT:
-            o << "      r_d1_" << (op.kind == ST_D1_IN ? "in" : "out") << "<" << a << ", " << b << ">(r, " << d2(p[0])
-              << ", " << d2(p[1]) << ", " << d2(p[2]) << ", " << d2(p[3]) << ");\n";
+        }
+        case SP_DENSE1: {
+            std::string args;
+            for (int i = 0; i < 4; ++i) args += ", " + ps.d2(s.par[i]);
+            for (int j : bases()) o << "      dense1(" << reg(j) << ", " << reg(coset(j, 1)) << args << ");\n";
             break;
-        default: o << "      /* unknown op */\n"; break;
+        }
+        case SP_DENSE2: {
+            std::string m;
+            if (ps.bank) {  // one run of the parameter block
+                m = "&P.v[" + std::to_string(ps.bank->size()) + "]";
+                for (int i = 0; i < 16; ++i) ps.bank->push_back(s.par[i]);
+            } else {
+                o << "      { const D2 m[16] = {";
+                for (int i = 0; i < 16; ++i) o << (i ? ", " : "") << ps.d2(s.par[i]);
+                o << "};\n";
+                m = "m";
+            }
+            for (int j : bases())
+                o << "      dense2(" << reg(j) << ", " << reg(coset(j, 1)) << ", " << reg(coset(j, 2)) << ", "
+                  << reg(coset(j, 3)) << ", " << m << ");\n";
+            if (!ps.bank) o << "      }\n";
+            break;
+        }
+        case SP_DEPOL1: {  // qubits: column, row
+            const std::string t = ps.d1(s.par[0].x), k = ps.d1(s.par[0].y);
+            for (int j : bases())
+                o << "      mix2(" << reg(j) << ", " << reg(coset(j, 3)) << ", " << t << "); rscale(" << reg(coset(j, 1))
+                  << ", " << k << "); rscale(" << reg(coset(j, 2)) << ", " << k << ");\n";
+            break;
+        }
+        case SP_DEPOL2: {  // qubits: columns 0, 1, rows 0, 1; populations: equal column and row
+            const int b = bases()[0];
+            const std::string t = ps.d1(s.par[0].x), k = s.form ? ps.d1(s.par[0].y) : std::string();
+            const int pop[4] = {coset(b, 0), coset(b, 5), coset(b, 10), coset(b, 15)};
+            o << "      { const D2 S = sum4(" << reg(pop[0]) << ", " << reg(pop[1]) << ", " << reg(pop[2]) << ", "
+              << reg(pop[3]) << ");\n";
+            if (s.form)
+                for (int j = 0; j < 16; ++j) o << "      rscale(" << reg(j) << ", " << k << ");\n";
+            for (int j : pop) o << "      axpy(" << reg(j) << ", " << t << ", S);\n";
+            o << "      }\n";
+            break;
+        }
     }
 }
 
-// Largest parameter block passed to a kernel (within the classic 4 KB kernel-parameter space, with
-// room for the state pointer); a pass with more parameters gets them as literals instead.
-constexpr size_t kMaxParamBytes = 4000;
+// Largest parameter block passed to a kernel (the kernel-parameter space is 32764 bytes; the state
+// pointer is in it too); a pass with more parameters gets them as literals instead.
+constexpr size_t kMaxParamBytes = 32000;
+
+// One coset per thread (up to 256 threads); two where a pass holds a two-qubit matrix, whose 16 products
+// per output do not fit beside the coset in 128 registers (184 bytes of spill).
+int spec_threads(const PassDesc& d) {
+    for (int ph = 0; ph < d.nphases; ++ph)
+        for (const ProgStep& s : d.programs[ph].steps)
+            if (s.kind == SP_DENSE2) return 128;
+    return d.m >= 12 ? 256 : 128;
+}
 
 // CUDA C of one pass; mirrors staged_tile (staged.cu) with every schedule quantity a constant.  With
 // `params`, gate parameters come from the kernel's parameter block (their values appended to *params);
@@ -334,39 +349,54 @@ std::string pass_source(const PassDesc& d, std::vector<double2>* params) {
     const int m = d.m;
     const unsigned tsize = 1u << m, ncos = tsize >> kPhaseBits;
     const bool hbm_first = d.io & 1, hbm_last = (d.io >> 1) & 1;
-    const int rows = 1 << (m - 7);  // tile rows of kStThreads amplitudes
+    const int threads = spec_threads(d), tb = __builtin_ctz(threads);
+    const int rows = 1 << (m - tb);  // tile rows of `threads` amplitudes
     ParamSink ps;
     ps.bank = params;
     std::ostringstream o;  // kernel body (the parameter block's size is known once it is written)
     o << ") {\n";
     o << "  extern __shared__ D2 tile[];\n  char* tb = reinterpret_cast<char*>(tile);\n";
     o << "  const unsigned tid = threadIdx.x;\n  u64 base = blockIdx.x;\n";
+    // Parameters are read at P.v[z + i] with z zero but different, to the compiler, in each round of the coset
+    // loop: they stay inside it (hoisted, all of a phase's would be live at once) and uniform over the warp.
+    if (params) o << "  const unsigned zero = blockDim.z - 1u;\n";
     for (int j = 0; j < m; ++j) o << "  base = ins0(base, " << d.q[j] << "u);\n";
     if (!hbm_first || !hbm_last) {
         o << "  u64 lo = 0;\n";
-        for (int j = 0; j < 7 && j < m; ++j) o << "  lo |= (u64)((tid >> " << j << ") & 1u) << " << d.q[j] << ";\n";
+        for (int j = 0; j < tb && j < m; ++j) o << "  lo |= (u64)((tid >> " << j << ") & 1u) << " << d.q[j] << ";\n";
     }
     if (!hbm_first) {
         o << "  {\n";
         for (int k = 0; k < rows; ++k) {
             ITYPE hi = 0;
-            for (int j = 7; j < m; ++j)
-                if ((k >> (j - 7)) & 1) hi |= 1ULL << d.q[j];
+            for (int j = tb; j < m; ++j)
+                if ((k >> (j - tb)) & 1) hi |= 1ULL << d.q[j];
             o << "    asm volatile(\"cp.async.cg.shared.global [%0], [%1], 16;\" :: \"r\"((unsigned)__cvta_generic_to_shared("
-              << "tile + swz(tid + " << k * kStThreads << "u))), \"l\"(s + (base | lo | " << u64hex(hi) << ")) : \"memory\");\n";
+              << "tile + swz(tid + " << k * threads << "u))), \"l\"(s + (base | lo | " << u64hex(hi) << ")) : \"memory\");\n";
         }
         o << "    asm volatile(\"cp.async.commit_group;\\ncp.async.wait_group 0;\" ::: \"memory\");\n    __syncthreads();\n  }\n";
     }
-    const int np = (int)d.phases.size();
+    const int np = d.nphases;
     for (int ph = 0; ph < np; ++ph) {
         const StPhase& P = d.phases[ph];
         const bool from_hbm = hbm_first && ph == 0, to_hbm = hbm_last && ph == np - 1;
         o << "  // phase " << ph << ": tile bits " << (int)P.bits[0] << "," << (int)P.bits[1] << "," << (int)P.bits[2] << ","
-          << (int)P.bits[3] << ", " << P.op_count << " ops\n";
-        o << "#pragma unroll 1\n  for (unsigned c = tid; c < " << ncos << "u; c += " << kStThreads << "u) {\n";
-        o << "    unsigned u0 = c;\n";
-        for (int p = 0; p < 4; ++p) o << "    u0 = (unsigned)ins0(u0, " << (int)P.bits[p] << "u);\n";
+          << (int)P.bits[3] << ", " << d.programs[ph].steps.size() << " steps\n";
+        const unsigned rounds = (ncos + threads - 1) / threads;
+        o << "#pragma unroll 1\n  for (unsigned it = 0; it < " << rounds << "u; ++it) {\n    const unsigned c = tid + it * "
+          << threads << "u;\n";
+        if (ncos < (unsigned)threads) o << "    if (c >= " << ncos << "u) break;\n";
+        const std::vector<int> order(P.order, P.order + (m - kPhaseBits));
+        o << "    const unsigned u0 = 0u";
+        for (size_t k = 0; k < order.size();) {  // runs of consecutive bits
+            size_t e = k + 1;
+            while (e < order.size() && order[e] == order[e - 1] + 1) ++e;
+            o << " | ((c >> " << k << ") & " << ((1u << (e - k)) - 1u) << "u) << " << order[k];
+            k = e;
+        }
+        o << ";\n";
         o << "    D2 r[16];\n";
+        if (params) o << "    const unsigned z = zero & it;\n";
         if (from_hbm || to_hbm) {
             o << "    u64 g0 = base;\n";
             for (int j = 0; j < m; ++j) o << "    g0 |= (u64)((u0 >> " << j << ") & 1u) << " << d.q[j] << ";\n";
@@ -386,19 +416,21 @@ std::string pass_source(const PassDesc& d, std::vector<double2>* params) {
             }
             o << "    }\n";
         }
-        for (uint32_t i = 0; i < P.op_count; ++i) emit_op(o, d.ops[P.op_begin + i], d.pool, ps);
+        for (const ProgStep& s : d.programs[ph].steps) emit_step(o, s, ps);
+        int at[16];  // the register that holds coset index i
+        for (int j = 0; j < 16; ++j) at[d.programs[ph].out[j]] = j;
         if (to_hbm) {
             o << "    { u64 gi = g0;\n";
             for (int g = 0; g < 16; ++g) {
                 if (g) o << "      gi ^= " << u64hex(1ULL << d.q[P.bits[gray_bit(g)]]) << ";\n";
-                o << "      stcs(s + gi, r[" << (g ^ (g >> 1)) << "]);\n";
+                o << "      stcs(s + gi, r[" << at[g ^ (g >> 1)] << "]);\n";
             }
             o << "    }\n";
         } else {
             o << "    { unsigned a = swz(u0) << 4;\n";
             for (int g = 0; g < 16; ++g) {
                 if (g) o << "      a ^= " << (swz_host(1u << P.bits[gray_bit(g)]) << 4) << "u;\n";
-                o << "      *reinterpret_cast<D2*>(tb + a) = r[" << (g ^ (g >> 1)) << "];\n";
+                o << "      *reinterpret_cast<D2*>(tb + a) = r[" << at[g ^ (g >> 1)] << "];\n";
             }
             o << "    }\n";
         }
@@ -411,17 +443,17 @@ std::string pass_source(const PassDesc& d, std::vector<double2>* params) {
         const int batch = rows < 16 ? rows : 16;
         o << "#pragma unroll 1\n  for (unsigned k0 = 0; k0 < " << rows << "u; k0 += " << batch << "u) {\n";
         o << "    D2 v[" << batch << "];\n#pragma unroll\n    for (unsigned k = 0; k < " << batch
-          << "u; ++k) v[k] = tile[swz(tid + (k0 + k) * " << kStThreads << "u)];\n";
+          << "u; ++k) v[k] = tile[swz(tid + (k0 + k) * " << threads << "u)];\n";
         o << "#pragma unroll\n    for (unsigned k = 0; k < " << batch << "u; ++k) {\n      const unsigned row = k0 + k;\n"
           << "      u64 hi = 0;\n";
-        for (int j = 7; j < m; ++j) o << "      hi |= (u64)((row >> " << j - 7 << ") & 1u) << " << d.q[j] << ";\n";
+        for (int j = tb; j < m; ++j) o << "      hi |= (u64)((row >> " << j - tb << ") & 1u) << " << d.q[j] << ";\n";
         o << "      stcs(s + (base | lo | hi), v[k]);\n    }\n  }\n";
     }
     o << "}\n";
     std::ostringstream h;
     h << kPrelude;
     if (params) h << "struct PassParams { D2 v[" << std::max<size_t>(1, params->size()) << "]; };\n";
-    h << "extern \"C\" __global__ void __launch_bounds__(" << kStThreads << ", 3) k_pass_spec(D2* __restrict__ s";
+    h << "extern \"C\" __global__ void __launch_bounds__(" << threads << ", " << (threads == 256 ? 2 : m >= 12 ? 3 : 4) << ") k_pass_spec(D2* __restrict__ s";
     if (params) h << ", const __grid_constant__ PassParams P";
     return h.str() + o.str();
 }
@@ -430,6 +462,7 @@ struct Compiled {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t kernel = nullptr;
     bool has_params = false;  // takes a parameter block after the state pointer
+    int threads = 256;
     std::set<int> smem_set;  // devices on which the dynamic shared-memory limit is raised
 };
 
@@ -528,7 +561,7 @@ int launch_nvrtc_kernel(void* handle, dim3 grid, dim3 block, void** args, size_t
 }
 
 int specialized_pass_kernel(const PassDesc& d, void** kernel, std::vector<double2>* params, double* compile_ms) {
-    if (d.m < 7 || d.m > kTileBits || d.phases.empty())
+    if (d.m < 7 || d.m > kTileBits || d.nphases == 0)
         return set_error(QS_ERR_NOT_SUPPORTED, "specialised passes need 7..12 tile qubits and a phase");
     params->clear();
     std::string src = pass_source(d, params);
@@ -539,7 +572,8 @@ int specialized_pass_kernel(const PassDesc& d, void** kernel, std::vector<double
     }
     const int rc = nvrtc_kernel(src, "k_pass_spec", kernel, compile_ms);
     if (rc != QS_OK) return rc;
-    static_cast<Compiled*>(*kernel)->has_params = !params->empty();  // a property of the source
+    static_cast<Compiled*>(*kernel)->has_params = !params->empty();  // properties of the source
+    static_cast<Compiled*>(*kernel)->threads = spec_threads(d);
     return QS_OK;
 }
 
@@ -547,7 +581,7 @@ int launch_specialized_pass(void* handle, double2* state, const double2* params,
     Compiled* C = static_cast<Compiled*>(handle);
     if (C->has_params && !params) return set_error(QS_ERR_INVALID_ARGUMENT, "specialised pass: no parameter block");
     void* args[] = {&state, const_cast<double2*>(params)};  // the parameter block is copied at launch
-    return launch_nvrtc_kernel(handle, dim3((unsigned)tiles), dim3(kStThreads), args, sizeof(double2) << m,
+    return launch_nvrtc_kernel(handle, dim3((unsigned)tiles), dim3(C->threads), args, sizeof(double2) << m,
         sizeof(double2) << kTileBits, st, "k_pass_spec");
 }
 

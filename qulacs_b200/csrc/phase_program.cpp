@@ -1,0 +1,406 @@
+// Builds phase programs (phase_program.hpp) from a pass's ops.
+#include "phase_program.hpp"
+
+#include <algorithm>
+#include <cmath>
+#include <complex>
+#include <cstring>
+
+namespace qs {
+
+// Parameters are multiplied up in extended precision and rounded once.
+using ld = long double;
+using cl = std::complex<long double>;
+
+namespace {
+
+cl mulc(const cl& x, const cl& y) {
+    return cl(x.real() * y.real() - x.imag() * y.imag(), x.real() * y.imag() + x.imag() * y.real());
+}
+double2 rounded(const cl& z) { return make_double2((double)z.real(), (double)z.imag()); }
+// hi + lo of a parameter pair
+cl joined(const double2& hi, const double2& lo) { return cl((ld)hi.x + lo.x, (ld)hi.y + lo.y); }
+
+struct Node {
+    bool diag = false;
+    // diagonal factors: functionals of the register index (1 or 2 of them) and the 16 values
+    int nf = 0;
+    uint8_t g[2] = {};
+    uint8_t a = 0;      // affine part of g[0]
+    bool sign = false;  // values +-1
+    bool free = false;  // one functional, free phase: counts as a factor whatever its value
+    cl val[16];
+    ProgStep step;      // other nodes: in the algebra of X^v (v in vs) and Z^f (f in fs)
+    int nv = 0, ns = 0;
+    uint8_t vs[4], fs[4];
+    bool rot = false;
+    int waits = 0;      // earlier nodes that do not commute with this one and have not run
+    bool done = false;
+};
+
+int par4(unsigned x) { return __builtin_popcount(x & 15u) & 1; }
+
+// X^v Z^f strings of a rotation: RY is Y = X^v Z^f, RX is X^v.
+bool commute(const Node& a, const Node& b) {
+    if (a.diag && b.diag) return true;
+    if (a.diag || b.diag) {
+        const Node& d = a.diag ? a : b;
+        const Node& o = a.diag ? b : a;
+        for (int i = 0; i < d.nf; ++i)
+            for (int k = 0; k < o.nv; ++k)
+                if (par4(d.g[i] & o.vs[k])) return false;
+        return true;
+    }
+    if (a.rot && b.rot)  // two strings
+        return par4((a.ns ? a.fs[0] : 0) & b.vs[0]) == par4((b.ns ? b.fs[0] : 0) & a.vs[0]);
+    for (int i = 0; i < a.ns; ++i)
+        for (int k = 0; k < b.nv; ++k)
+            if (par4(a.fs[i] & b.vs[k])) return false;
+    for (int i = 0; i < b.ns; ++i)
+        for (int k = 0; k < a.nv; ++k)
+            if (par4(b.fs[i] & a.vs[k])) return false;
+    return true;
+}
+
+struct PassScalar {
+    cl value = 1.;
+    bool any = false;      // something was deferred (whatever its value: the kernel depends on structure only)
+    bool complex = false;
+    double bits = 0.;      // log2 of the growth deferred so far
+};
+
+struct Builder {
+    uint8_t F[4] = {1, 2, 4, 8}, V[4] = {1, 2, 4, 8}, A[4] = {};
+    std::vector<Node> nodes;
+    PassScalar& S;
+    const bool move;  // CNOT, SWAP and X are steps; the map stays the identity
+    Builder(PassScalar& s, bool m) : S(s), move(m) {}
+
+    // qubit i of the node's step is register bit b; x, z: whether the node moves and reads it
+    void set_qubit(Node& n, int i, int b, bool x = true, bool z = true) {
+        ProgStep& p = n.step;
+        p.v[i] = V[b];
+        p.f[i] = F[b];
+        p.a[i] = A[b];
+        p.nq = (uint8_t)std::max<int>(p.nq, i + 1);
+        if (x) n.vs[n.nv++] = V[b];
+        if (z) n.fs[n.ns++] = F[b];
+    }
+    void push(Node n) { nodes.push_back(std::move(n)); }
+
+    // `free`: the phases are parameters, so the step is the same whatever their values
+    void diag1(int b, cl d0, cl d1, bool free = false) {
+        Node n;
+        n.diag = true;
+        n.nf = 1;
+        n.g[0] = F[b];
+        n.a = A[b];
+        const double m0 = (double)std::norm(d0), m1 = (double)std::norm(d1);
+        const bool ok = m0 > 0.25 && m0 < 4. && m1 > 0.25 && m1 < 4.;
+        n.free = free;
+        if (d0 == d1 && ok && (!free || d0 != cl(1.))) {  // a scalar
+            if (d0 != cl(1.)) scalar(d0, free);
+            return;
+        }
+        if (ok) {  // the factor of bit value 0 joins the pass's scalar
+            if (d0 != cl(1.)) scalar(d0, free);
+            const cl r = d1 == -d0 ? cl(-1.) : d0 == cl(1.) ? d1 : d1 / d0;
+            n.sign = !free && r == cl(-1.);
+            for (int j = 0; j < 16; ++j) n.val[j] = (par4(F[b] & j) ^ A[b]) ? r : cl(1.);
+        } else {  // projections and the like
+            for (int j = 0; j < 16; ++j) n.val[j] = (par4(F[b] & j) ^ A[b]) ? d1 : d0;
+        }
+        push(n);
+    }
+    void scalar(cl z, bool free = false) {
+        S.any = true;
+        S.complex = S.complex || free || z.imag() != 0.;
+        S.value = mulc(S.value, z);
+    }
+    void cz(int a, int b) {
+        Node n;
+        n.diag = n.sign = true;
+        n.nf = 2;
+        n.g[0] = F[a];
+        n.g[1] = F[b];
+        for (int j = 0; j < 16; ++j)
+            n.val[j] = ((par4(F[a] & j) ^ A[a]) && (par4(F[b] & j) ^ A[b])) ? cl(-1.) : cl(1.);
+        push(n);
+    }
+    // csim's RY {c, s; -s, c} (x = false) or RX {c, i s; i s, c}
+    void rot(int b, ld c, ld s, bool x) {
+        Node n;
+        n.rot = true;
+        n.step.kind = SP_ROT;
+        set_qubit(n, 0, b, true, !x);
+        const double bits = -std::log2(std::max((double)std::abs(c), 1e-300));
+        const uint8_t base = x ? RF_X_TAN : RF_Y_TAN;
+        if (bits <= 20. && S.bits + bits <= kMaxDeferredBits) {
+            n.step.form = base;
+            n.step.par.push_back(make_double2((double)(s / c), 0.));
+            scalar(c);
+            S.bits += bits;
+        } else if (S.bits + 1. <= kMaxDeferredBits) {  // nearly a flip: the sine is near 1
+            n.step.form = base + 1;
+            n.step.par.push_back(make_double2((double)(c / s), 0.));
+            scalar(s);
+            S.bits += 1.;
+        } else {
+            n.step.form = base + 2;
+            n.step.par.push_back(make_double2((double)c, (double)s));
+        }
+        push(n);
+    }
+    void flip(int b) {
+        if (move) return perm(SP_X, b, -1);
+        A[b] ^= 1;
+    }
+    void perm(StepKind kind, int a, int b) {
+        Node n;
+        n.step.kind = kind;
+        set_qubit(n, 0, a, kind != SP_CNOT, kind != SP_X);
+        if (b >= 0) set_qubit(n, 1, b, true, kind == SP_SWAP);
+        push(n);
+    }
+    void cnot(int c, int t) {
+        if (move) return perm(SP_CNOT, c, t);
+        F[t] ^= F[c];
+        A[t] ^= A[c];
+        V[c] ^= V[t];
+    }
+    void swap(int a, int b) {
+        if (move) return perm(SP_SWAP, a, b);
+        std::swap(F[a], F[b]);
+        std::swap(V[a], V[b]);
+        std::swap(A[a], A[b]);
+    }
+    void dense1(int b, const double2* m) {
+        cl u[4];
+        for (int i = 0; i < 4; ++i) u[i] = cl(m[i].x, m[i].y);
+        if (u[1] == cl(0.) && u[2] == cl(0.)) return diag1(b, u[0], u[3]);
+        if (u[0] == cl(0.) && u[3] == cl(0.)) {
+            flip(b);
+            return diag1(b, u[1], u[2]);
+        }
+        Node n;
+        n.step.kind = SP_DENSE1;
+        set_qubit(n, 0, b);
+        n.step.par.assign(m, m + 4);
+        push(n);
+    }
+    void dense2(int a, int b, const double2* m) {
+        Node n;
+        n.step.kind = SP_DENSE2;
+        set_qubit(n, 0, a);
+        set_qubit(n, 1, b);
+        n.step.par.assign(m, m + 16);
+        push(n);
+    }
+    // depolarizing channel of strength q (rho -> (1 - q) rho + q I / 2^k tr): column bits, then row bits
+    void depol(const int* bits, int k, ld q) {
+        Node n;
+        n.step.kind = k == 1 ? SP_DEPOL1 : SP_DEPOL2;
+        for (int i = 0; i < 2 * k; ++i) set_qubit(n, i, bits[i]);
+        if (k == 1) {
+            const ld d = 1.L - q / 2;
+            n.step.par.push_back(make_double2((double)(q / 2 / d), (double)((1.L - q) / d)));
+            scalar(d);
+            S.bits -= (double)std::log2(d);  // d >= 1/3
+        } else if (std::abs(1.L - q) > 0.001L) {
+            n.step.par.push_back(make_double2((double)(q / 4 / (1.L - q)), 0.));
+            scalar(1.L - q);
+            S.bits -= (double)std::log2(std::abs(1.L - q));
+        } else {
+            n.step.form = 1;
+            n.step.par.push_back(make_double2((double)(q / 4), (double)(1.L - q)));
+        }
+        push(n);
+    }
+
+    void schedule(PhaseProgram* P) {
+        const int N = (int)nodes.size();
+        std::vector<std::vector<int>> after(N);
+        for (int j = 0; j < N; ++j)
+            for (int i = 0; i < j; ++i)
+                if (!commute(nodes[i], nodes[j])) {
+                    after[i].push_back(j);
+                    ++nodes[j].waits;
+                }
+        int left = N;
+        auto finish = [&](int i) {
+            nodes[i].done = true;
+            --left;
+            for (int j : after[i]) --nodes[j].waits;
+        };
+        auto others = [&]() {  // every ready step that is no diagonal
+            bool any = false, again = true;
+            while (again) {
+                again = false;
+                for (int i = 0; i < N; ++i)
+                    if (!nodes[i].done && !nodes[i].diag && nodes[i].waits == 0) {
+                        P->steps.push_back(nodes[i].step);
+                        finish(i);
+                        any = again = true;
+                    }
+            }
+            return any;
+        };
+        auto diagonals = [&](bool signs_only) {
+            ProgStep s;
+            bool any = false, sign = true;
+            cl val[16];
+            bool touched[16] = {};
+            for (int j = 0; j < 16; ++j) val[j] = 1.;
+            for (int i = 0; i < N; ++i) {
+                Node& n = nodes[i];
+                if (n.done || !n.diag || n.waits || (signs_only && !n.sign)) continue;
+                for (int j = 0; j < 16; ++j) {
+                    if (n.val[j] != cl(1.) || (n.free && (par4(n.g[0] & j) ^ n.a))) touched[j] = true;
+                    val[j] = mulc(val[j], n.val[j]);
+                }
+                any = true;
+                sign = sign && n.sign;
+                finish(i);
+            }
+            if (!any) return;
+            if (sign) {
+                s.kind = SP_SIGN;
+                for (int j = 0; j < 16; ++j)
+                    if (val[j] != cl(1.)) s.mask |= (uint16_t)(1u << j);
+                if (!s.mask) return;
+            } else {
+                s.kind = SP_DIAG;
+                for (int j = 0; j < 16; ++j) {
+                    s.par.push_back(rounded(val[j]));
+                    s.xpar.push_back(val[j]);
+                    if (touched[j]) s.mask |= (uint16_t)(1u << j);
+                }
+            }
+            P->steps.push_back(s);
+        };
+        while (left) {
+            others();
+            if (!left) break;
+            diagonals(true);  // sign flips cost nothing: first
+            if (others()) continue;
+            diagonals(false);
+        }
+        // register j holds coset index out[j] holds coset index i(j)
+        for (int j = 0; j < 16; ++j) {
+            int i = 0;
+            for (int b = 0; b < 4; ++b) i |= (par4(F[b] & j) ^ A[b]) << b;
+            P->out[j] = (uint8_t)i;
+        }
+    }
+};
+
+}  // namespace
+
+std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count, const StOp* ops, const double2* pool) {
+    std::vector<PhaseProgram> out(count);
+    PassScalar S;
+    for (size_t ph = 0; ph < count; ++ph) {
+        const StOp *begin = ops + phases[ph].op_begin, *end = begin + phases[ph].op_count;
+        bool move = false;
+        for (const StOp* o = begin; o != end; ++o) {
+            const double2* m = pool + o->param;
+            const bool one = o->kind == ST_DENSE1;  // an X or a diagonal is no matrix
+            const bool flip = one && m[0].x == 0. && m[0].y == 0. && m[3].x == 0. && m[3].y == 0.;
+            const bool diag = one && m[1].x == 0. && m[1].y == 0. && m[2].x == 0. && m[2].y == 0.;
+            move = move || o->kind == ST_DENSE2 || o->kind == ST_DEPOL1 || o->kind == ST_DEPOL2 || (one && !flip && !diag);
+        }
+        Builder B(S, move);
+        for (const StOp* op = begin; op != end; ++op) {
+            const StOp& o = *op;
+            const double2* p = pool + o.param;
+            switch (o.kind) {
+                case ST_RX:
+                case ST_RY: B.rot(o.a, (ld)p[0].x + p[1].x, (ld)p[0].y + p[1].y, o.kind == ST_RX); break;
+                case ST_DIAG1: B.diag1(o.a, joined(p[0], p[2]), joined(p[1], p[3]), o.aux != 0); break;
+                case ST_CNOT: B.cnot(o.a, o.b); break;
+                case ST_CZ: B.cz(o.a, o.b); break;
+                case ST_SWAP: B.swap(o.a, o.b); break;
+                case ST_DENSE1: B.dense1(o.a, p); break;
+                case ST_DENSE2: B.dense2(o.a, o.b, p); break;
+                case ST_DEPOL1: {
+                    const int bits[2] = {o.a, o.b};
+                    B.depol(bits, 1, (ld)p[0].x * 4 / 3);
+                    break;
+                }
+                case ST_DEPOL2: {
+                    const int bits[4] = {o.a, o.b, o.aux & 3, (o.aux >> 2) & 3};
+                    B.depol(bits, 2, (ld)p[0].x * 16 / 15);
+                    break;
+                }
+                default: break;
+            }
+        }
+        B.schedule(&out[ph]);
+    }
+    if (S.any) {
+        // the pass's scalar joins the fullest set of diagonal factors, else it is a step of its own
+        ProgStep* best = nullptr;
+        for (PhaseProgram& P : out)
+            for (ProgStep& s : P.steps)
+                if (s.kind == SP_DIAG && (!best || __builtin_popcount(s.mask) > __builtin_popcount(best->mask))) best = &s;
+        if (best) {
+            best->mask = 0xffff;
+            for (int j = 0; j < 16; ++j) best->par[j] = rounded(mulc(S.value, best->xpar[j]));
+        } else {
+            ProgStep s;
+            s.kind = SP_SCALE;
+            s.form = S.complex;
+            s.par.push_back(rounded(S.value));
+            out.back().steps.push_back(s);
+        }
+    }
+    return out;
+}
+
+// Codes: run_step in csrc/staged.cu.
+void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vector<double2>* pool, StPhase* phase) {
+    auto bit = [](uint8_t v) { return __builtin_ctz(v); };
+    phase->step_begin = (uint32_t)steps->size();
+    for (const ProgStep& s : P.steps) {
+        StStep t{};
+        t.param = (uint32_t)pool->size();
+        t.mask = s.mask;
+        const int a = s.nq > 0 ? bit(s.v[0]) : 0, b = s.nq > 1 ? bit(s.v[1]) : 0;
+        switch (s.kind) {
+            case SP_DIAG: t.code = 0; break;
+            case SP_SIGN: t.code = 1; break;
+            case SP_SCALE: t.code = s.form ? 3 : 2; break;
+            case SP_CNOT: t.code = (uint8_t)(16 + a * 4 + b); break;
+            case SP_X: t.code = (uint8_t)(16 + a * 5); break;
+            case SP_SWAP: t.code = (uint8_t)(32 + std::min(a, b) * 4 + std::max(a, b)); break;
+            case SP_DENSE1: t.code = (uint8_t)(32 + a * 5); break;
+            case SP_DEPOL1: t.code = (uint8_t)(32 + std::max(a, b) * 4 + std::min(a, b)); break;
+            case SP_DENSE2: t.code = (uint8_t)(48 + a * 4 + b); break;
+            case SP_DEPOL2: {  // by the partner of register bit 0: 1, 2 or 3
+                const int c = bit(s.v[2]), d = bit(s.v[3]);
+                const int mate = a == 0 ? c : b == 0 ? d : c == 0 ? a : b;
+                t.code = (uint8_t)(48 + (mate - 1) * 5);
+                t.mask = s.form;
+                break;
+            }
+            case SP_ROT: {
+                const bool tan = s.form == RF_Y_TAN || s.form == RF_X_TAN, x = s.form >= RF_X_TAN;
+                t.code = (uint8_t)(64 + 32 * x + 16 * !tan + s.v[0]);
+                const int low = s.v[0] & -s.v[0];
+                for (int j = 0, k = 0; j < 16; ++j)
+                    if (!(j & low)) t.mask |= (uint16_t)(step_bit(s, 0, j) << k++);
+                break;
+            }
+        }
+        if (s.kind == SP_ROT && (s.form == RF_Y_COT || s.form == RF_X_COT))
+            pool->push_back(make_double2(s.par[0].x, 1.));  // c = cot, s = 1: the same products and sums
+        else
+            pool->insert(pool->end(), s.par.begin(), s.par.end());
+        steps->push_back(t);
+    }
+    phase->step_count = (uint32_t)(steps->size() - phase->step_begin);
+    phase->out0 = P.out[0];
+    for (int k = 0; k < 4; ++k) phase->out[k] = P.out[1 << k] ^ P.out[0];
+}
+
+}  // namespace qs

@@ -1,4 +1,4 @@
-// Staged executor: several gates per HBM pass, each gate applied with its own (unfused) arithmetic.
+// Staged executor: many gates per HBM pass.
 //
 // A pass owns a set Q of m "tile qubits" (always including qubits 0..3, so every HBM access is a
 // run of >= 16 contiguous amplitudes = 256 B).  Each CTA loads one tile -- the 2^m amplitudes that
@@ -7,10 +7,18 @@
 // pass instead of one per gate.  Inside the tile, gates are grouped into "phases" of at most 4 tile
 // qubits: each thread gathers the 16 amplitudes of its 4-qubit coset into registers, applies all the
 // phase's gates there, and scatters them back, so shared memory is touched once per phase, not once
-// per gate.  The host scheduler (below) builds passes and phases greedily from the gate list; a gate
-// is only moved past gates on disjoint qubits, so the result equals gate-by-gate application up to
-// rounding order (~1e-16).  Gates the pass kernel does not cover (more than 2 targets, controls,
-// Pauli strings, multi-qubit diagonals) run between passes with the gate-by-gate kernels.
+// per gate.  A phase's gates run as a program of rotations, collected diagonals and register relabellings
+// (phase_program.hpp), which the kernels here interpret step by step; the specialised pass kernels
+// (pass_codegen.cpp) run the same programs as straight-line code.  The host scheduler (below) builds passes
+// and phases greedily from the gate list in rotation form (fusion.cpp); a gate is only moved past gates
+// on disjoint qubits, so the result equals gate-by-gate application up to rounding (~1e-16).  Gates the
+// pass kernel does not cover (more than 2 targets, controls, Pauli strings, multi-qubit diagonals) run
+// between passes with the gate-by-gate kernels.
+//
+// What bounds it on small states is the chain of steps in a CTA: one coset per thread (256 threads for a
+// 2^12-amplitude tile, where 128 threads took two in turn) and rotations in place of matrices halved it: the
+// 16-qubit layered circuit (16 tiles, 454 gates) and
+// its 64-string energy went from 0.495 to 0.287 ms.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -25,6 +33,7 @@
 
 #include "circuit.hpp"
 #include "qs_internal.cuh"
+#include "phase_program.hpp"
 #include "staged.hpp"
 
 namespace qs {
@@ -35,11 +44,82 @@ struct StPassArgs {
     int io;                // bit 0: the first phase gathers from HBM; bit 1: the last phase scatters to HBM
     UINT q[kTileBits];     // global qubit of tile bit j, ascending, q[j] = j for j < kLowFixed
     const StPhase* phases;
-    const StOp* ops;
-    const double2* pool;
+    const StStep* steps;
+    const double2* pool;   // the steps' parameters
 };
 
-// ---------------------------------------------------------------- register ops
+// ---------------------------------------------------------------- register steps
+// The steps of a phase program (phase_program.hpp) on a thread's 16 amplitudes; the arithmetic of each is
+// that of the specialised kernels' (csrc/pass_codegen.cpp), in the same order.
+// A parameter read at its use (volatile: a whole matrix is not held in registers).
+__device__ __forceinline__ double2 ld_par(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double flipped(double t, unsigned odd) {  // -t where odd is 1
+    return __hiloint2double(__double2hiint(t) ^ (int)(odd << 31), __double2loint(t));
+}
+// Rotations: register pairs (lo, lo ^ V), lo without V's lowest bit.  A pair whose lo has the qubit's value 1
+// (bit k of `rev`) runs with the sine's sign reversed.
+template <int V, class F>
+__device__ __forceinline__ void for_pairs(double2 (&r)[16], F f) {
+    constexpr int low = V & -V;
+    int k = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (!(j & low)) f(r[j], r[j ^ V], k++);
+}
+template <int V>
+__device__ __forceinline__ void r_ry_tan(double2 (&r)[16], double t0, unsigned rev) {
+    for_pairs<V>(r, [&](double2& x, double2& y, int k) {
+        const double t = flipped(t0, (rev >> k) & 1u);
+        const double2 X = x;
+        x = make_double2(fma(t, y.x, X.x), fma(t, y.y, X.y));
+        y = make_double2(fma(-t, X.x, y.x), fma(-t, X.y, y.y));
+    });
+}
+template <int V>
+__device__ __forceinline__ void r_ry_full(double2 (&r)[16], double c, double s0, unsigned rev) {
+    for_pairs<V>(r, [&](double2& x, double2& y, int k) {
+        const double s = flipped(s0, (rev >> k) & 1u);
+        const double2 X = x;
+        x = make_double2(fma(c, X.x, s * y.x), fma(c, X.y, s * y.y));
+        y = make_double2(fma(c, y.x, -s * X.x), fma(c, y.y, -s * X.y));
+    });
+}
+template <int V>
+__device__ __forceinline__ void r_rx_tan(double2 (&r)[16], double t) {
+    for_pairs<V>(r, [&](double2& x, double2& y, int) {
+        const double2 X = x;
+        x = make_double2(fma(-t, y.y, X.x), fma(t, y.x, X.y));
+        y = make_double2(fma(-t, X.y, y.x), fma(t, X.x, y.y));
+    });
+}
+template <int V>
+__device__ __forceinline__ void r_rx_full(double2 (&r)[16], double c, double s) {
+    for_pairs<V>(r, [&](double2& x, double2& y, int) {
+        const double2 X = x;
+        x = make_double2(fma(c, X.x, -s * y.y), fma(c, X.y, s * y.x));
+        y = make_double2(fma(c, y.x, -s * X.y), fma(c, y.y, s * X.x));
+    });
+}
+__device__ __forceinline__ void r_diag(double2 (&r)[16], const double2* __restrict__ p, unsigned mask) {
+#pragma unroll
+    for (int h = 0; h < 16; h += 4) {
+        double2 d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] = ld_par(p + h + j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((mask >> (h + j)) & 1u) r[h + j] = cmul(d[j], r[h + j]);
+    }
+}
+__device__ __forceinline__ void r_sign(double2 (&r)[16], unsigned mask) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        r[j] = make_double2(flipped(r[j].x, (mask >> j) & 1u), flipped(r[j].y, (mask >> j) & 1u));
+}
 template <int B>
 __device__ __forceinline__ void r_dense1(double2 (&r)[16], const double2* __restrict__ p) {
     const double2 m0 = p[0], m1 = p[1], m2 = p[2], m3 = p[3];
@@ -49,63 +129,6 @@ __device__ __forceinline__ void r_dense1(double2 (&r)[16], const double2* __rest
             const double2 x = r[j], y = r[j | (1 << B)];
             r[j] = cfma(m1, y, cmul(m0, x));
             r[j | (1 << B)] = cfma(m3, y, cmul(m2, x));
-        }
-}
-template <int B>
-__device__ __forceinline__ void r_diag1(double2 (&r)[16], const double2* __restrict__ p) {
-    const double2 d0 = p[0], d1 = p[1];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = cmul((j & (1 << B)) ? d1 : d0, r[j]);
-}
-// RX: {c, i s; i s, c}
-template <int B>
-__device__ __forceinline__ void r_rx(double2 (&r)[16], const double2* __restrict__ p) {
-    const double c = p[0].x, s = p[0].y;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << B))) {
-            const double2 x = r[j], y = r[j | (1 << B)];
-            r[j] = make_double2(fma(c, x.x, -s * y.y), fma(c, x.y, s * y.x));
-            r[j | (1 << B)] = make_double2(fma(c, y.x, -s * x.y), fma(c, y.y, s * x.x));
-        }
-}
-// RY: {c, s; -s, c}
-template <int B>
-__device__ __forceinline__ void r_ry(double2 (&r)[16], const double2* __restrict__ p) {
-    const double c = p[0].x, s = p[0].y;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << B))) {
-            const double2 x = r[j], y = r[j | (1 << B)];
-            r[j] = make_double2(fma(c, x.x, s * y.x), fma(c, x.y, s * y.y));
-            r[j | (1 << B)] = make_double2(fma(c, y.x, -s * x.x), fma(c, y.y, -s * x.y));
-        }
-}
-template <int C, int T>
-__device__ __forceinline__ void r_cnot(double2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << C)) && !(j & (1 << T))) {
-            const double2 t = r[j];
-            r[j] = r[j | (1 << T)];
-            r[j | (1 << T)] = t;
-        }
-}
-template <int A, int B>
-__device__ __forceinline__ void r_cz(double2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << A)) && (j & (1 << B))) r[j] = make_double2(-r[j].x, -r[j].y);
-}
-template <int A, int B>
-__device__ __forceinline__ void r_swap(double2 (&r)[16]) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((j & (1 << A)) && !(j & (1 << B))) {
-            const int k = j ^ (1 << A) ^ (1 << B);
-            const double2 t = r[j];
-            r[j] = r[k];
-            r[k] = t;
         }
 }
 // matrix-index bit 0 <-> register bit A (first target), bit 1 <-> B
@@ -120,93 +143,109 @@ __device__ __forceinline__ void r_dense2(double2 (&r)[16], const double2* __rest
             for (int x = 0; x < 4; ++x) v[x] = r[o[x]];
 #pragma unroll
             for (int y = 0; y < 4; ++y) {
-                double2 acc = cmul(p[y * 4], v[0]);
+                double2 acc = cmul(ld_par(p + y * 4), v[0]);
 #pragma unroll
-                for (int x = 1; x < 4; ++x) acc = cfma(p[y * 4 + x], v[x], acc);
+                for (int x = 1; x < 4; ++x) acc = cfma(ld_par(p + y * 4 + x), v[x], acc);
                 r[o[y]] = acc;
             }
         }
 }
-
-// Dense 2x2 along register bit A with the matrix chosen by register bit B: p[0..3] where bit B is 0,
-// p[4..7] where it is 1 (a one-qubit gate on the target of a CNOT, with the CNOT folded in).
-template <int A, int B>
-__device__ __forceinline__ void r_csel1(double2 (&r)[16], const double2* __restrict__ p) {
-    const double2 m0 = p[0], m1 = p[1], m2 = p[2], m3 = p[3];
-    const double2 n0 = p[4], n1 = p[5], n2 = p[6], n3 = p[7];
+template <int C, int T>
+__device__ __forceinline__ void r_cnot(double2 (&r)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A))) {
-            const double2 x = r[j], y = r[j | (1 << A)];
-            const bool hi = (j >> B) & 1;
-            r[j] = cfma(hi ? n1 : m1, y, cmul(hi ? n0 : m0, x));
-            r[j | (1 << A)] = cfma(hi ? n3 : m3, y, cmul(hi ? n2 : m2, x));
+        if ((j & (1 << C)) && !(j & (1 << T))) {
+            const double2 t = r[j];
+            r[j] = r[j | (1 << T)];
+            r[j | (1 << T)] = t;
         }
 }
-// A one-qubit dense gate U on the control A of CNOT(A -> B), CNOT first: for j with bits A, B clear
-// and t in {0, B}, out[j^t] = U00 in[j^t] + U01 in[j^t^A^B], out[j^t^A] = U10 in[j^t] + U11 in[j^t^A^B].
-template <int A, int B>
-__device__ __forceinline__ void r_d1_in(double2 (&r)[16], const double2* __restrict__ p) {
-    const double2 m0 = p[0], m1 = p[1], m2 = p[2], m3 = p[3];
-    double2 o[16];
+template <int A>
+__device__ __forceinline__ void r_x(double2 (&r)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
         if (!(j & (1 << A))) {
+            const double2 t = r[j];
+            r[j] = r[j | (1 << A)];
+            r[j | (1 << A)] = t;
+        }
+}
+template <int A, int B>
+__device__ __forceinline__ void r_swap(double2 (&r)[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if ((j & (1 << A)) && !(j & (1 << B))) {
             const int k = j ^ (1 << A) ^ (1 << B);
-            const double2 x = r[j], y = r[k];
-            o[j] = cfma(m1, y, cmul(m0, x));
-            o[j | (1 << A)] = cfma(m3, y, cmul(m2, x));
+            const double2 t = r[j];
+            r[j] = r[k];
+            r[k] = t;
         }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = o[j];
 }
-// The same gate with the CNOT second: out[j^t] = U00 in[j^t] + U01 in[j^t^A],
-// out[j^t^A^B] = U10 in[j^t] + U11 in[j^t^A].
+// One-qubit depolarizing channel, scaled (column and row bit A, B): populations mix, coherences shrink.
 template <int A, int B>
-__device__ __forceinline__ void r_d1_out(double2 (&r)[16], const double2* __restrict__ p) {
-    const double2 m0 = p[0], m1 = p[1], m2 = p[2], m3 = p[3];
-    double2 o[16];
+__device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k) {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
-        if (!(j & (1 << A))) {
-            const double2 x = r[j], y = r[j | (1 << A)];
-            o[j] = cfma(m1, y, cmul(m0, x));
-            o[j ^ (1 << A) ^ (1 << B)] = cfma(m3, y, cmul(m2, x));
+        if (!(j & (1 << A)) && !(j & (1 << B))) {
+            double2 &x = r[j], &y = r[j | (1 << A) | (1 << B)];
+            const double2 X = x;
+            x = make_double2(fma(t, y.x, X.x), fma(t, y.y, X.y));
+            y = make_double2(fma(t, X.x, y.x), fma(t, X.y, y.y));
+            r[j | (1 << A)] = make_double2(k * r[j | (1 << A)].x, k * r[j | (1 << A)].y);
+            r[j | (1 << B)] = make_double2(k * r[j | (1 << B)].x, k * r[j | (1 << B)].y);
         }
+}
+// Two-qubit depolarizing channel on pairs of register bits (0, MATE) and the other two: the four populations
+// have equal bits in each pair.
+template <int MATE>
+__device__ __forceinline__ void r_depol2(double2 (&r)[16], double t, double k, bool full) {
+    constexpr int p = 1 | (1 << MATE), q = 15 ^ p;
+    const double2 S = make_double2((r[0].x + r[p].x) + (r[q].x + r[15].x), (r[0].y + r[p].y) + (r[q].y + r[15].y));
+    if (full) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) r[j] = o[j];
+        for (int j = 0; j < 16; ++j) r[j] = make_double2(k * r[j].x, k * r[j].y);
+    }
+    for (int j : {0, p, q, 15}) r[j] = make_double2(fma(t, S.x, r[j].x), fma(t, S.y, r[j].y));
 }
 
-// One indirect branch per op: the host encodes code = kind * 16 + a * 4 + b (op_code), and every code
-// has its own fully specialised register code (unused codes are empty).  One-qubit kinds use b = a;
-// their b != a codes hold the CNOT-folded ops (DENSE1: ST_CSEL1, DIAG1: ST_D1_IN, RX: ST_D1_OUT), which
-// keeps the switch at 128 codes -- more codes made every pass slower.  Passes without folded ops run
-// the FOLDS = false build, whose switch holds only the plain ops (the folded code placed among the
-// plain one-qubit cases slowed unfused schedules by 12 %).
-template <int CODE, bool FOLDS>
-__device__ __forceinline__ void run_code(double2 (&r)[16], const double2* p) {
-    constexpr int kind = CODE >> 4, A = (CODE >> 2) & 3, B = CODE & 3;
-    if constexpr (kind == ST_DENSE1 && B == A) r_dense1<A>(r, p);
-    else if constexpr (FOLDS && kind == ST_DENSE1) r_csel1<A, B>(r, p);
-    else if constexpr (kind == ST_DIAG1 && B == A) r_diag1<A>(r, p);
-    else if constexpr (FOLDS && kind == ST_DIAG1) r_d1_in<A, B>(r, p);
-    else if constexpr (kind == ST_RX && B == A) r_rx<A>(r, p);
-    else if constexpr (FOLDS && kind == ST_RX) r_d1_out<A, B>(r, p);
-    else if constexpr (kind == ST_RY && B == A) r_ry<A>(r, p);
-    else if constexpr (kind == ST_CNOT && A != B) r_cnot<A, B>(r);
-    else if constexpr (kind == ST_CZ && A != B) r_cz<A, B>(r);
-    else if constexpr (kind == ST_SWAP && A != B) r_swap<A, B>(r);
-    else if constexpr (kind == ST_DENSE2 && A != B) r_dense2<A, B>(r, p);
+// One indirect branch per step: the host's code (encode_program) selects fully specialised register code.
+//   0 diagonal, 1 signs, 2 real and 3 complex scale;  16..31 CNOT a * 4 + b, X at a = b;
+//   32..47 SWAP (a < b), one-qubit matrix (a = b), one-qubit channel (a > b);
+//   48..63 two-qubit matrix, two-qubit channel at a = b (register bit 0's partner a + 1);
+//   64.. RY scaled by the pair vector, 80.. RY with cosine and sine, 96.. RX, 112.. RX with cosine and sine.
+template <int CODE>
+__device__ __forceinline__ void run_step(double2 (&r)[16], const double2* __restrict__ p, unsigned mask) {
+    constexpr int kind = CODE >> 4, V = CODE & 15, A = V >> 2, B = V & 3;
+    if constexpr (CODE == 0) r_diag(r, p, mask);
+    else if constexpr (CODE == 1) r_sign(r, mask);
+    else if constexpr (CODE == 2) {
+        const double k = p[0].x;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = make_double2(k * r[j].x, k * r[j].y);
+    } else if constexpr (CODE == 3) {
+        const double2 z = p[0];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = cmul(z, r[j]);
+    } else if constexpr (kind == 1 && A != B) r_cnot<A, B>(r);
+    else if constexpr (kind == 1) r_x<A>(r);
+    else if constexpr (kind == 2 && A < B) r_swap<A, B>(r);
+    else if constexpr (kind == 2 && A == B) r_dense1<A>(r, p);
+    else if constexpr (kind == 2) r_depol1<A, B>(r, p[0].x, p[0].y);
+    else if constexpr (kind == 3 && A != B) r_dense2<A, B>(r, p);
+    else if constexpr (kind == 3 && A < 3) r_depol2<A + 1>(r, p[0].x, p[0].y, mask != 0);
+    else if constexpr (kind == 4 && V) r_ry_tan<V>(r, p[0].x, mask);
+    else if constexpr (kind == 5 && V) r_ry_full<V>(r, p[0].x, p[0].y, mask);
+    else if constexpr (kind == 6 && V) r_rx_tan<V>(r, p[0].x);
+    else if constexpr (kind == 7 && V) r_rx_full<V>(r, p[0].x, p[0].y);
 }
 #define QS_CODE1(c) \
-    case c: run_code<c, FOLDS>(r, p); break;
+    case c: run_step<c>(r, p, s.mask); break;
 #define QS_CODE4(c) QS_CODE1(c) QS_CODE1(c + 1) QS_CODE1(c + 2) QS_CODE1(c + 3)
 #define QS_CODE16(c) QS_CODE4(c) QS_CODE4(c + 4) QS_CODE4(c + 8) QS_CODE4(c + 12)
-template <bool FOLDS>
-__device__ __forceinline__ void apply_op(const StOp& op, double2 (&r)[16], const double2* pool) {
-    const double2* p = pool + op.param;
-    switch (op.pad) {
-        QS_CODE16(0)
+__device__ __forceinline__ void apply_step(const StStep& s, double2 (&r)[16], const double2* __restrict__ pool) {
+    const double2* p = pool + s.param;
+    switch (s.code) {
+        QS_CODE4(0)
         QS_CODE16(16)
         QS_CODE16(32)
         QS_CODE16(48)
@@ -221,34 +260,35 @@ __device__ __forceinline__ void apply_op(const StOp& op, double2 (&r)[16], const
 #undef QS_CODE4
 #undef QS_CODE1
 
-// XOR swizzle of the tile index for conflict-free 16-byte shared-memory accesses (linear over XOR,
-// so swz(a | b) = swz(a) ^ swz(b) for disjoint bit sets).
-__device__ __forceinline__ UINT swz(UINT u) { return u ^ (((u >> 4) ^ (u >> 7) ^ (u >> 10)) & 7u); }
+__device__ __forceinline__ UINT swz(UINT u) { return QS_SWZ(u); }
 
-// Tile index u = tid + k * kStThreads (k < 2^(m-7)) has global offset base | lo_off | hi_off[k]:
-// lo_off takes tid's bits 0..6 to the tile qubits q[0..6], hi_off[k] takes k's bits to q[7..].
+// Tile index u = tid + k * THREADS has global offset base | lo_off | hi_off[k]: lo_off takes tid's bits to
+// the lowest tile qubits, hi_off[k] takes k's bits to the others.
 
-// Global rows of 16 amplitudes per thread from the swizzled tile to HBM (rows k0 .. k0 + 15).
-template <class T>
+// Global rows of 16 amplitudes per thread from the swizzled tile to HBM.
+template <int THREADS, class T>
 __device__ __forceinline__ void tile_rows_store(T* __restrict__ s, const double2* tile, ITYPE off,
-    const ITYPE* hi_off, UINT tsize, int k0) {
+    const ITYPE* hi_off, UINT tsize) {
     const UINT tid = threadIdx.x;
     double2 v[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-        if (tid + (UINT)(k0 + k) * kStThreads < tsize) v[k] = tile[swz(tid + (UINT)(k0 + k) * kStThreads)];
+        if (tid + (UINT)k * THREADS < tsize) v[k] = tile[swz(tid + (UINT)k * THREADS)];
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-        if (tid + (UINT)(k0 + k) * kStThreads < tsize) st_amp(s + (off | hi_off[k0 + k]), v[k]);
+        if (tid + (UINT)k * THREADS < tsize) st_amp(s + (off | hi_off[k]), v[k]);
 }
 
 // One tile of one pass: load, apply every phase, store.  Shared by the per-pass kernel and the
-// persistent multi-circuit kernel.  `tile` holds 2^m amplitudes (m <= kTileBits) in FP64 whatever the
-// state's type E (complex128, or complex64 widened on load and rounded on store).  Ends with a CTA
-// barrier so the shared buffers can be reused immediately.
-template <int MAX_BITS, bool FOLDS, class E>
+// persistent multi-circuit kernel.  `tile` holds 2^m amplitudes (m <= MAX_BITS) in FP64 whatever the
+// state's type E (complex128, or complex64 widened on load and rounded on store).  THREADS is the largest
+// tile's coset count: one 16-amplitude coset per thread and phase.  Ends with a CTA barrier so the shared
+// buffers can be reused immediately.
+template <int MAX_BITS, int THREADS, class E>
 __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs& a, ITYPE T, double2* tile,
     ITYPE* hi_off) {
+    static_assert(THREADS == 1 << (MAX_BITS - kPhaseBits), "one coset per thread");
+    constexpr int TB = MAX_BITS - kPhaseBits;
     const int m = a.m;
     const UINT tsize = 1u << m;
     // base: insert zeros at the tile qubits into the tile index
@@ -258,13 +298,13 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
     const bool hbm_first = a.io & 1, hbm_last = (a.io >> 1) & 1;
     ITYPE lo_off = 0;
     if (!hbm_first || !hbm_last) {
-        if (tid < (1 << (MAX_BITS - 7))) {
+        if (tid < 16) {
             ITYPE o = 0;
-            for (int j = 7; j < m; ++j)
-                if ((tid >> (j - 7)) & 1) o |= 1ULL << a.q[j];
+            for (int j = TB; j < m; ++j)
+                if ((tid >> (j - TB)) & 1) o |= 1ULL << a.q[j];
             hi_off[tid] = o;
         }
-        for (int j = 0; j < 7 && j < m; ++j)
+        for (int j = 0; j < TB && j < m; ++j)
             if ((tid >> j) & 1) lo_off |= 1ULL << a.q[j];
         __syncthreads();
     }
@@ -274,26 +314,26 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
             // 16-byte cp.async copies straight into the swizzled tile: every copy of a thread in flight at
             // once, without holding registers
 #pragma unroll
-            for (int k = 0; k < (1 << (MAX_BITS - 7)); ++k)
-                if ((UINT)tid + (UINT)k * kStThreads < tsize) {
+            for (int k = 0; k < 16; ++k)
+                if ((UINT)tid + (UINT)k * THREADS < tsize) {
                     const unsigned dst =
-                        (unsigned)__cvta_generic_to_shared(tile + swz((UINT)tid + (UINT)k * kStThreads));
+                        (unsigned)__cvta_generic_to_shared(tile + swz((UINT)tid + (UINT)k * THREADS));
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(s + (off | hi_off[k]))
                                  : "memory");
                 }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
         } else {
-            // complex64: widened in registers, 4 loads in flight per thread before their stores
+            // complex64: widened in registers, 8 loads in flight per thread before their stores
 #pragma unroll
-            for (int k0 = 0; k0 < (1 << (MAX_BITS - 7)); k0 += 4) {
-                double2 v[4];
+            for (int k0 = 0; k0 < 16; k0 += 8) {
+                double2 v[8];
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if ((UINT)tid + (UINT)(k0 + k) * kStThreads < tsize) v[k] = ld_amp(s + (off | hi_off[k0 + k]));
+                for (int k = 0; k < 8; ++k)
+                    if ((UINT)tid + (UINT)(k0 + k) * THREADS < tsize) v[k] = ld_amp(s + (off | hi_off[k0 + k]));
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if ((UINT)tid + (UINT)(k0 + k) * kStThreads < tsize)
-                        tile[swz((UINT)tid + (UINT)(k0 + k) * kStThreads)] = v[k];
+                for (int k = 0; k < 8; ++k)
+                    if ((UINT)tid + (UINT)(k0 + k) * THREADS < tsize)
+                        tile[swz((UINT)tid + (UINT)(k0 + k) * THREADS)] = v[k];
             }
         }
         __syncthreads();
@@ -306,50 +346,64 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
         // HBM (the host sets this when the phase's bits are all >= 4, so that a coset's lanes 0..15 cover
         // 16 consecutive amplitudes): no tile load or store round through shared memory.
         const bool from_hbm = hbm_first && ph == 0, to_hbm = hbm_last && ph == a.nphases - 1;
-        // Byte offset of register amplitude j from the coset's first one: the XOR of sb[p] over the set
-        // bits p of j (the swizzle is XOR-linear); in HBM, the XOR of gb[p].  The 16 amplitudes are
-        // visited in Gray-code order so that each address is the previous one with one offset XORed in.
-        UINT sb[4];
-        ITYPE gb[4];
+        if ((UINT)tid < ncos) {
+            UINT u0 = 0;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            sb[p] = swz(1u << P.bits[p]) << 4;
-            gb[p] = 1ULL << a.q[P.bits[p]];
-        }
-        for (UINT c = tid; c < ncos; c += kStThreads) {
-            UINT u0 = c;
-#pragma unroll
-            for (int p = 0; p < 4; ++p) u0 = (UINT)insert0(u0, P.bits[p]);
+            for (int k = 0; k < TB; ++k) u0 |= ((tid >> k) & 1u) << P.order[k];
             ITYPE g0 = base;  // global index of the coset's first amplitude (only for HBM phases)
             if (from_hbm || to_hbm)
                 for (int j = 0; j < m; ++j)
                     if ((u0 >> j) & 1) g0 |= 1ULL << a.q[j];
             double2 r[16];
-            UINT addr = swz(u0) << 4;
+            // Offset of coset index j from the coset's first amplitude: the XOR of one offset per set bit of
+            // j (the swizzle is XOR-linear).  The 16 amplitudes are visited in Gray-code order, so that each
+            // address is the previous one with one offset XORed in.
             if (from_hbm) {
                 ITYPE gi = g0;
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
-                    if (g) gi ^= gb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
+                    if (g) gi ^= 1ULL << a.q[P.bits[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3]];
                     r[g ^ (g >> 1)] = ld_amp(s + gi);
                 }
             } else {
+                UINT sb[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) sb[p] = swz(1u << P.bits[p]) << 4;
+                UINT addr = swz(u0) << 4;
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
                     if (g) addr ^= sb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     r[g ^ (g >> 1)] = *reinterpret_cast<const double2*>(tile_bytes + addr);
                 }
-                addr = swz(u0) << 4;
             }
-            for (UINT o = 0; o < P.op_count; ++o) apply_op<FOLDS>(a.ops[P.op_begin + o], r, a.pool);
+            for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
+            // register j goes to coset index out0 ^ (XOR of out[k] over the bits k of j)
+            auto tile_index = [&](UINT i) {
+                UINT u = 0;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) u |= ((i >> p) & 1u) << P.bits[p];
+                return u;
+            };
             if (to_hbm) {
-                ITYPE gi = g0;
+                ITYPE gb[4], gi = g0;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    gb[p] = 0;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        if ((P.out[p] >> b) & 1) gb[p] |= 1ULL << a.q[P.bits[b]];
+                    if ((P.out0 >> p) & 1) gi |= 1ULL << a.q[P.bits[p]];
+                }
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
                     if (g) gi ^= gb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     st_amp(s + gi, r[g ^ (g >> 1)]);
                 }
             } else {
+                UINT sb[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) sb[p] = swz(tile_index(P.out[p])) << 4;
+                UINT addr = swz(u0 | tile_index(P.out0)) << 4;
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
                     if (g) addr ^= sb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
@@ -359,20 +413,16 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
         }
         if (!to_hbm) __syncthreads();
     }
-    if (!hbm_last) {
-        tile_rows_store(s, tile, base | lo_off, hi_off, tsize, 0);
-        if constexpr (MAX_BITS > 11)
-            if (tsize > 16 * kStThreads) tile_rows_store(s, tile, base | lo_off, hi_off, tsize, 16);
-    }
+    if (!hbm_last) tile_rows_store<THREADS>(s, tile, base | lo_off, hi_off, tsize);
     __syncthreads();
 }
 
 // One CTA per tile; the tile (2^m x 16 bytes, up to 64 KiB) is dynamic shared memory.
-template <bool FOLDS, class E>
-__global__ void __launch_bounds__(kStThreads, 3) k_staged_pass(E* __restrict__ s, const __grid_constant__ StPassArgs a) {
+template <class E>
+__global__ void __launch_bounds__(kStThreads, 2) k_staged_pass(E* __restrict__ s, const __grid_constant__ StPassArgs a) {
     extern __shared__ double2 st_tile[];
-    __shared__ ITYPE hi_off[1 << (kTileBits - 7)];
-    staged_tile<kTileBits, FOLDS>(s, a, blockIdx.x, st_tile, hi_off);
+    __shared__ ITYPE hi_off[16];
+    staged_tile<kTileBits, kStThreads>(s, a, blockIdx.x, st_tile, hi_off);
 }
 
 // Opt k_staged_pass in to 64 KiB of dynamic shared memory, once per device.
@@ -384,13 +434,9 @@ static int staged_allow_smem() {
     std::lock_guard<std::mutex> lock(mu);
     if ((int)done.size() <= dev) done.resize(dev + 1, 0);
     if (!done[dev]) {
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<false, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
             (int)(sizeof(double2) << kTileBits)));
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<true, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int)(sizeof(double2) << kTileBits)));
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<false, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int)(sizeof(double2) << kTileBits)));
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<true, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
             (int)(sizeof(double2) << kTileBits)));
         done[dev] = 1;
     }
@@ -403,6 +449,7 @@ using cd = std::complex<double>;
 
 static bool stageable(const GateRec& g) {
     if (!g.controls.empty()) return false;
+    if (g.depol) return true;
     switch (g.kind) {
         case QS_GATE_RX:
         case QS_GATE_RY:
@@ -522,7 +569,6 @@ static std::vector<PassPlan> plan_passes(const std::vector<GateRec>& G, UINT n, 
 
 struct DevPass {
     bool single;
-    bool folds;  // the pass has CNOT-folded ops
     int gate;
     StPassArgs args;
     size_t phase_begin = 0;  // the pass's phases in StagedPlan::phases
@@ -533,18 +579,16 @@ struct DevPass {
 template <class E>
 static void launch_pass(E* state, const DevPass& d, ITYPE tiles, cudaStream_t st) {
     const size_t smem = sizeof(double2) << d.args.m;  // the tile is FP64 for either state type
-    if (d.folds) k_staged_pass<true, E><<<(unsigned)tiles, kStThreads, smem, st>>>(state, d.args);
-    else k_staged_pass<false, E><<<(unsigned)tiles, kStThreads, smem, st>>>(state, d.args);
+    k_staged_pass<E><<<(unsigned)tiles, kStThreads, smem, st>>>(state, d.args);
 }
 
 struct StagedPlan {
     ITYPE dim = 0;
     std::vector<DevPass> passes;
-    void* dev = nullptr;  // phases | ops | pool
+    void* dev = nullptr;  // phases | steps | parameters
     // host copies of the schedule (for specialised pass kernels)
     std::vector<StPhase> phases;
-    std::vector<StOp> ops;
-    std::vector<double2> pool;
+    std::vector<PhaseProgram> programs;
     bool specialized = false;  // every pass has its specialised kernel
     double compile_ms = 0.;    // wall time of compiling them
     ~StagedPlan() {
@@ -559,105 +603,47 @@ static int local_bit(const std::vector<UINT>& q, UINT g) {
     return -1;
 }
 
-// Dispatch code of an op (see run_code).
-static uint8_t op_code(const StOp& o) {
-    int kind = o.kind;
-    if (kind == ST_CSEL1) kind = ST_DENSE1;
-    else if (kind == ST_D1_IN) kind = ST_DIAG1;
-    else if (kind == ST_D1_OUT) kind = ST_RX;
-    return (uint8_t)(kind * 16 + o.a * 4 + o.b);
-}
-
-// Fold CNOTs into a neighbouring one-qubit dense op of the same phase (ops [begin, end) of `ops`, in
-// program order), which costs the CNOT's register moves and dispatch nothing: a CNOT whose nearest
-// earlier op on its two register bits is a dense op U (on either bit) runs at U's place, after it;
-// failing that, one whose nearest later op on them is a dense op runs at that op's place, before it.
-// A folded CNOT takes its host op's place in the order, so a CNOT is not moved past an earlier folded
-// CNOT on the same bits.
-// On the target T: CNOT.U_T = U (control 0) / X U (control 1); U_T.CNOT = U / U X (ST_CSEL1).  On the
-// control C: U_C.CNOT pairs (c, t) with (c^1, t^1) on input (ST_D1_IN), CNOT.U_C on output (ST_D1_OUT).
-// A CZ folds the same way into a dense op on either of its qubits: CZ.U = U / Z U, U.CZ = U / U Z.
-static void absorb_cnots(std::vector<StOp>& ops, std::vector<double2>& pool, size_t begin) {
-    auto touches = [](const StOp& o, int bit) {
-        const bool two = o.kind == ST_CNOT || o.kind == ST_CZ || o.kind == ST_SWAP || o.kind == ST_DENSE2 ||
-                         o.kind == ST_CSEL1 || o.kind == ST_D1_IN || o.kind == ST_D1_OUT;
-        return o.a == bit || (two && o.b == bit);
+// The tile bits outside a phase, in the order in which the coset number's bits run over them: three with
+// independent swizzle vectors first (the lowest such triple, for conflict-free accesses), the others ascending.
+static void lane_order(StPhase* P, int m) {
+    std::vector<uint8_t> rest;
+    for (int b = 0; b < m; ++b)
+        if (b != P->bits[0] && b != P->bits[1] && b != P->bits[2] && b != P->bits[3]) rest.push_back((uint8_t)b);
+    const int k = (int)rest.size();
+    auto vec = [](UINT b) { return QS_SWZ(1u << b) & 7u; };
+    auto pick = [&]() {
+        for (int x = 0; x < k; ++x)
+            for (int y = x + 1; y < k; ++y)
+                for (int z = y + 1; z < k; ++z) {
+                    const UINT a = vec(rest[x]), b = vec(rest[y]), c = vec(rest[z]);
+                    if (!a || !b || a == b || !c || c == a || c == b || c == (a ^ b)) continue;
+                    std::vector<uint8_t> out = {rest[x], rest[y], rest[z]};
+                    for (int i = 0; i < k; ++i)
+                        if (i != x && i != y && i != z) out.push_back(rest[i]);
+                    rest.swap(out);
+                    return;
+                }
     };
-    const size_t end = ops.size();
-    std::vector<char> dead(end, 0);
-    std::vector<size_t> at_op(end);  // place of each op in the order (a folded CNOT: its host op)
-    for (size_t i = begin; i < end; ++i) at_op[i] = i;
-    for (size_t i = begin; i < end; ++i) {
-        if (ops[i].kind != ST_CNOT && ops[i].kind != ST_CZ) continue;
-        const bool cz = ops[i].kind == ST_CZ;
-        const int c = ops[i].a, t = ops[i].b;
-        // a folded CNOT on c or t placed strictly between lo and hi forbids the move
-        auto blocked = [&](size_t lo, size_t hi) {
-            for (size_t j = begin; j < end; ++j)
-                if (dead[j] && at_op[j] > lo && at_op[j] < hi && (touches(ops[j], c) || touches(ops[j], t)))
-                    return true;
-            return false;
-        };
-        auto fold = [&](size_t k, bool cnot_first) {
-            StOp& u = ops[k];
-            const double2 m0 = pool[u.param], m1 = pool[u.param + 1], m2 = pool[u.param + 2], m3 = pool[u.param + 3];
-            const uint32_t at = (uint32_t)pool.size();
-            const double2 n0 = make_double2(-m0.x, -m0.y), n1 = make_double2(-m1.x, -m1.y),
-                          n2 = make_double2(-m2.x, -m2.y), n3 = make_double2(-m3.x, -m3.y);
-            if (cz) {  // the other qubit selects U or its sign-flipped form
-                u.kind = ST_CSEL1;
-                u.b = (uint8_t)(u.a == t ? c : t);
-                for (const double2& v : {m0, m1, m2, m3}) pool.push_back(v);
-                if (cnot_first) for (const double2& v : {m0, n1, m2, n3}) pool.push_back(v);  // U Z
-                else for (const double2& v : {m0, m1, n2, n3}) pool.push_back(v);             // Z U
-            } else if (u.a == t) {
-                u.kind = ST_CSEL1;
-                u.b = (uint8_t)c;
-                for (const double2& v : {m0, m1, m2, m3}) pool.push_back(v);
-                if (cnot_first) for (const double2& v : {m1, m0, m3, m2}) pool.push_back(v);  // U X
-                else for (const double2& v : {m2, m3, m0, m1}) pool.push_back(v);             // X U
-            } else {
-                u.kind = cnot_first ? ST_D1_IN : ST_D1_OUT;
-                u.b = (uint8_t)t;
-                for (const double2& v : {m0, m1, m2, m3}) pool.push_back(v);
-            }
-            u.param = at;
-            dead[i] = 1;
-            at_op[i] = k;
-        };
-        for (size_t k = i; k-- > begin;) {
-            if (dead[k] || !(touches(ops[k], c) || touches(ops[k], t))) continue;
-            if (ops[k].kind == ST_DENSE1 && !blocked(k, i)) fold(k, false);
-            break;
-        }
-        if (dead[i]) continue;
-        for (size_t k = i + 1; k < end; ++k) {
-            if (dead[k] || !(touches(ops[k], c) || touches(ops[k], t))) continue;
-            if (ops[k].kind == ST_DENSE1 && !blocked(i, k)) fold(k, true);
-            break;
-        }
-    }
-    size_t w = begin;
-    for (size_t i = begin; i < end; ++i)
-        if (!dead[i]) {
-            ops[i].pad = op_code(ops[i]);
-            ops[w++] = ops[i];
-        }
-    ops.resize(w);
+    pick();
+    for (int i = 0; i < 8; ++i) P->order[i] = i < k ? rest[i] : 0;
 }
 
 struct HostPlan {
     std::vector<PassPlan> passes;
     std::vector<StPhase> phases;
-    std::vector<StOp> ops;
+    std::vector<StOp> ops;      // the phases' gates and their parameters
     std::vector<double2> pool;
+    std::vector<PhaseProgram> programs;  // one per phase
+    std::vector<StStep> steps;  // the programs as the generic kernels read them
+    std::vector<double2> params;
     struct Range {
         size_t phase_begin, nphases;
     };
     std::vector<Range> pp;
 };
 
-// Host-only part of planning: passes, phases and encoded ops (no device calls).
+// Host-only part of planning: passes, phases and their programs (no device calls).  The gates are in
+// rotation form.
 static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits = kTileBits) {
     H->passes = plan_passes(gates, n, tile_bits);
     const std::vector<PassPlan>& passes = H->passes;
@@ -719,7 +705,7 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
                 }
             }
             for (int b = 0; b < m && __builtin_popcountll(bestR) < kPhaseBits; ++b) bestR |= 1ULL << b;
-            StPhase ph;
+            StPhase ph{};
             int nb = 0;
             int regbit[64];
             for (int b = 0; b < m; ++b)
@@ -733,43 +719,41 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
                 StOp op{};
                 auto rb = [&](UINT gq) { return (uint8_t)regbit[local_bit(p.q, gq)]; };
                 op.param = (uint32_t)pool.size();
-                const double ang = g.angle;
+                if (g.depol) {
+                    op.kind = g.depol == 1 ? ST_DEPOL1 : ST_DEPOL2;
+                    op.a = rb(g.targets[0]);
+                    op.b = rb(g.targets[1]);
+                    if (g.depol == 2) op.aux = (uint8_t)(rb(g.targets[2]) | rb(g.targets[3]) << 2);
+                    pool.push_back(make_double2(g.prob, 0.));
+                    ops.push_back(op);
+                    continue;
+                }
+                if (g.extended) {  // parameters as hi + lo
+                    op.a = op.b = rb(g.targets[0]);
+                    auto split = [&](long double x0, long double y0, long double x1, long double y1, int pairs) {
+                        const long double v[2][2] = {{x0, y0}, {x1, y1}};
+                        for (int i = 0; i < pairs; ++i) pool.push_back(make_double2((double)v[i][0], (double)v[i][1]));
+                        for (int i = 0; i < pairs; ++i)
+                            pool.push_back(make_double2((double)(v[i][0] - (double)v[i][0]), (double)(v[i][1] - (double)v[i][1])));
+                    };
+                    if (g.kind == QS_GATE_DIAGONAL) {
+                        op.kind = ST_DIAG1;
+                        op.aux = g.free_phase;
+                        split(g.xd[0].real(), g.xd[0].imag(), g.xd[1].real(), g.xd[1].imag(), 2);
+                    } else {
+                        op.kind = g.kind == QS_GATE_RX ? ST_RX : ST_RY;
+                        split(g.xc, g.xs, 0.L, 0.L, 1);
+                    }
+                    ops.push_back(op);
+                    continue;
+                }
                 switch (g.kind) {
-                    case QS_GATE_RX:
-                        op.kind = ST_RX;
-                        op.a = rb(g.targets[0]);
-                        pool.push_back(make_double2(std::cos(ang / 2), std::sin(ang / 2)));
-                        break;
-                    case QS_GATE_RY:
-                        op.kind = ST_RY;
-                        op.a = rb(g.targets[0]);
-                        pool.push_back(make_double2(std::cos(ang / 2), std::sin(ang / 2)));
-                        break;
-                    case QS_GATE_RZ:
-                        op.kind = ST_DIAG1;
-                        op.a = rb(g.targets[0]);
-                        pool.push_back(make_double2(std::cos(ang / 2), std::sin(ang / 2)));
-                        pool.push_back(make_double2(std::cos(ang / 2), -std::sin(ang / 2)));
-                        break;
                     case QS_GATE_CNOT:
-                        op.kind = ST_CNOT;
-                        op.a = rb(g.targets[0]);
-                        op.b = rb(g.targets[1]);
-                        break;
                     case QS_GATE_CZ:
-                        op.kind = ST_CZ;
-                        op.a = rb(g.targets[0]);
-                        op.b = rb(g.targets[1]);
-                        break;
                     case QS_GATE_SWAP:
-                        op.kind = ST_SWAP;
+                        op.kind = g.kind == QS_GATE_CNOT ? ST_CNOT : g.kind == QS_GATE_CZ ? ST_CZ : ST_SWAP;
                         op.a = rb(g.targets[0]);
                         op.b = rb(g.targets[1]);
-                        break;
-                    case QS_GATE_DIAGONAL:
-                        op.kind = ST_DIAG1;
-                        op.a = rb(g.targets[0]);
-                        for (int i = 0; i < 2; ++i) pool.push_back(make_double2(g.matrix[i].real(), g.matrix[i].imag()));
                         break;
                     default:  // dense 1 or 2 targets
                         if (g.targets.size() == 1) {
@@ -784,13 +768,10 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
                         }
                         break;
                 }
-                if (op.kind == ST_DENSE1 || op.kind == ST_DIAG1 || op.kind == ST_RX || op.kind == ST_RY)
-                    op.b = op.a;  // one-qubit ops: b = a (see run_code)
-                op.pad = op_code(op);
                 ops.push_back(op);
             }
-            absorb_cnots(ops, pool, ph.op_begin);
             ph.op_count = (uint32_t)(ops.size() - ph.op_begin);
+            lane_order(&ph, m);
             phases.push_back(ph);
             std::vector<char> taken(gates.size(), 0);
             for (int gi : best) taken[gi] = 1;
@@ -798,6 +779,11 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
             for (int gi : todo)
                 if (!taken[gi]) rest.push_back(gi);
             todo.swap(rest);
+        }
+        std::vector<PhaseProgram> prog = build_pass_program(phases.data() + ph0, phases.size() - ph0, ops.data(), pool.data());
+        for (size_t i = 0; i < prog.size(); ++i) {
+            encode_program(prog[i], &H->steps, &H->params, &phases[ph0 + i]);
+            H->programs.push_back(std::move(prog[i]));
         }
         pp.push_back({ph0, phases.size() - ph0});
     }
@@ -817,27 +803,24 @@ static int upload_plan(const HostPlan& H, ITYPE dim, std::shared_ptr<StagedPlan>
     auto P = std::make_shared<StagedPlan>();
     P->dim = dim;
     P->phases = H.phases;
-    P->ops = H.ops;
-    P->pool = H.pool;
+    P->programs = H.programs;
     const std::vector<PassPlan>& passes = H.passes;
     const std::vector<StPhase>& phases = H.phases;
-    const std::vector<StOp>& ops = H.ops;
-    const std::vector<double2>& pool = H.pool;
     const std::vector<HostPlan::Range>& pp = H.pp;
     // upload
-    const size_t bph = sizeof(StPhase) * phases.size(), bop = sizeof(StOp) * ops.size(),
-                 bpo = sizeof(double2) * pool.size();
-    const size_t o_ops = (bph + 255) / 256 * 256, o_pool = o_ops + (bop + 255) / 256 * 256;
-    const size_t total = o_pool + bpo + 256;
+    const size_t bph = sizeof(StPhase) * phases.size(), bst = sizeof(StStep) * H.steps.size(),
+                 bpa = sizeof(double2) * H.params.size();
+    const size_t o_steps = (bph + 255) / 256 * 256, o_params = o_steps + (bst + 255) / 256 * 256;
+    const size_t total = o_params + bpa + 256;
     QS_CUDA_CHECK(cudaMalloc(&P->dev, total));
     std::vector<char> host(total, 0);
     if (bph) memcpy(host.data(), phases.data(), bph);
-    if (bop) memcpy(host.data() + o_ops, ops.data(), bop);
-    if (bpo) memcpy(host.data() + o_pool, pool.data(), bpo);
+    if (bst) memcpy(host.data() + o_steps, H.steps.data(), bst);
+    if (bpa) memcpy(host.data() + o_params, H.params.data(), bpa);
     QS_CUDA_CHECK(cudaMemcpy(P->dev, host.data(), total, cudaMemcpyHostToDevice));
     const StPhase* dph = (const StPhase*)P->dev;
-    const StOp* dop = (const StOp*)((char*)P->dev + o_ops);
-    const double2* dpo = (const double2*)((char*)P->dev + o_pool);
+    const StStep* dst = (const StStep*)((char*)P->dev + o_steps);
+    const double2* dpa = (const double2*)((char*)P->dev + o_params);
     for (size_t i = 0; i < passes.size(); ++i) {
         DevPass d{};
         d.single = passes[i].single;
@@ -857,11 +840,8 @@ static int upload_plan(const HostPlan& H, ITYPE dim, std::shared_ptr<StagedPlan>
             }
             d.args.phases = dph + pp[i].phase_begin;
             d.phase_begin = pp[i].phase_begin;
-            for (size_t ph = pp[i].phase_begin; ph < pp[i].phase_begin + pp[i].nphases; ++ph)
-                for (uint32_t o = phases[ph].op_begin; o < phases[ph].op_begin + phases[ph].op_count; ++o)
-                    d.folds = d.folds || ops[o].kind == ST_CSEL1 || ops[o].kind == ST_D1_IN || ops[o].kind == ST_D1_OUT;
-            d.args.ops = dop;
-            d.args.pool = dpo;
+            d.args.steps = dst;
+            d.args.pool = dpa;
         }
         P->passes.push_back(d);
     }
@@ -894,9 +874,9 @@ static PassDesc pass_desc(const StagedPlan& P, const DevPass& d) {
     pd.m = d.args.m;
     pd.io = d.args.io;
     for (int j = 0; j < d.args.m; ++j) pd.q[j] = d.args.q[j];
-    pd.phases.assign(P.phases.begin() + d.phase_begin, P.phases.begin() + d.phase_begin + d.args.nphases);
-    pd.ops = P.ops.data();
-    pd.pool = P.pool.data();
+    pd.nphases = d.args.nphases;
+    pd.phases = P.phases.data() + d.phase_begin;
+    pd.programs = P.programs.data() + d.phase_begin;
     return pd;
 }
 
@@ -945,11 +925,13 @@ static bool want_specialized(const Circuit& c, ITYPE dim) {
 }
 
 static int ensure_plan(Circuit& c, ITYPE dim) {
-    if (!c.plan || c.plan->dim != dim) QS_TRY(build_plan(c.gates, c.n, dim, &c.plan));
+    if (!c.plan || c.plan->dim != dim) {
+        c.rgates = rotation_form(c.gates);
+        QS_TRY(build_plan(c.rgates, c.n, dim, &c.plan));
+    }
     if (want_specialized(c, dim)) QS_TRY(specialize_plan(*c.plan));
     return QS_OK;
 }
-
 
 int run_staged(Circuit& c, void* state, ITYPE dim, cudaStream_t st) {
     if (c.n < kPhaseBits) {  // too small for a 4-qubit register phase
@@ -957,7 +939,7 @@ int run_staged(Circuit& c, void* state, ITYPE dim, cudaStream_t st) {
         return QS_OK;
     }
     QS_TRY(ensure_plan(c, dim));
-    return run_plan(c.gates, *c.plan, state, dim, st);
+    return run_plan(c.rgates, *c.plan, state, dim, st);
 }
 
 // ---- FP64 gate fusion + staged passes, block size and tile shape chosen by measurement.
@@ -1060,7 +1042,7 @@ static int ensure_fused_plan(Circuit& c, ITYPE dim, cudaStream_t st) {
     if (c.fplan && c.fplan->dim == dim) return QS_OK;
     const bool spec = want_specialized(c, dim);
     if (c.fusion_k >= 0) {
-        c.fgates = fuse_gates(c.gates, c.fusion_k);
+        c.fgates = executor_gates(c.gates, c.fusion_k, &c.fused_count);
         c.fused_k = c.fusion_k;
         c.fused_tile_bits = kTileBits;
         QS_TRY(build_plan(c.fgates, c.n, dim, &c.fplan));
@@ -1070,7 +1052,8 @@ static int ensure_fused_plan(Circuit& c, ITYPE dim, cudaStream_t st) {
     c.tune_ms.assign(kTuneSlots, -1.);
     double best = 0.;
     auto consider = [&](int k, int tile_bits, int slot) -> int {
-        std::vector<GateRec> fg = fuse_gates(c.gates, k);
+        size_t count = 0;
+        std::vector<GateRec> fg = executor_gates(c.gates, k, &count);
         std::shared_ptr<StagedPlan> P;
         QS_TRY(build_plan(fg, c.n, dim, &P, tile_bits));
         double ms = 0.;
@@ -1079,6 +1062,7 @@ static int ensure_fused_plan(Circuit& c, ITYPE dim, cudaStream_t st) {
         if (!c.fplan || ms < best) {
             best = ms;
             c.fgates.swap(fg);
+            c.fused_count = count;
             c.fplan = P;
             c.fused_k = k;
             c.fused_tile_bits = tile_bits;
@@ -1111,7 +1095,7 @@ static int c64_block_size(const Circuit& c) { return (c.fusion_k >= 0 && c.fusio
 static int ensure_c64_plan(Circuit& c, ITYPE dim) {
     const int k = c64_block_size(c);
     if (c.cplan && c.cplan->dim == dim && c.ck == k) return QS_OK;
-    c.cgates = fuse_gates(c.gates, k);
+    c.cgates = executor_gates(c.gates, k);
     c.ck = k;
     QS_TRY(build_plan(c.cgates, c.n, dim, &c.cplan));
     for (const DevPass& d : c.cplan->passes)
@@ -1140,7 +1124,7 @@ int staged_pass_count(Circuit& c, ITYPE dim, UINT* out) {
         return QS_OK;
     }
     HostPlan H;
-    make_host_plan(c.gates, c.n, &H);
+    make_host_plan(rotation_form(c.gates), c.n, &H);
     *out = (UINT)H.passes.size();
     return QS_OK;
 }
@@ -1154,7 +1138,7 @@ extern "C" QS_API int qs_circuit_staged_stats(qs_circuit_t circuit, QS_UINT* pas
     qs::Circuit* c = reinterpret_cast<qs::Circuit*>(circuit);
     if (!c || !passes || !phases || !ops || !single_gates) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
     qs::HostPlan H;
-    qs::make_host_plan(c->gates, c->n, &H);
+    qs::make_host_plan(qs::rotation_form(c->gates), c->n, &H);
     UINT single = 0;
     for (const qs::PassPlan& p : H.passes) single += p.single ? 1 : 0;
     *passes = (QS_UINT)H.passes.size();
@@ -1173,7 +1157,7 @@ extern "C" QS_API int qs_circuit_fusion_info(qs_circuit_t circuit, int* k, QS_UI
     qs::Circuit* c = reinterpret_cast<qs::Circuit*>(circuit);
     if (!c || !k || !gate_count || !passes) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
     *k = c->fplan ? c->fused_k : -1;
-    *gate_count = c->fplan ? (QS_UINT)c->fgates.size() : 0;
+    *gate_count = c->fplan ? (QS_UINT)c->fused_count : 0;
     *passes = c->fplan ? (QS_UINT)c->fplan->passes.size() : 0;
     if (estimates_ms)
         for (int i = 0; i < qs::kTuneSlots; ++i)
@@ -1219,13 +1203,12 @@ extern "C" QS_API int qs_circuit_specialized_source(qs_circuit_t circuit, QS_ITY
     if (dim != (1ULL << c->n)) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "dim differs from 2^qubit_count");
     if (c->n < (UINT)qs::kPhaseBits + 3) return qs::set_error(QS_ERR_NOT_SUPPORTED, "fewer than 7 qubits");
     qs::HostPlan H;
-    qs::make_host_plan(c->gates, c->n, &H);
+    qs::make_host_plan(qs::rotation_form(c->gates), c->n, &H);
     if (pass >= H.passes.size() || H.passes[pass].single)
         return qs::set_error(QS_ERR_INVALID_ARGUMENT, "no such staged pass");
     qs::StagedPlan P;
     P.phases = H.phases;
-    P.ops = H.ops;
-    P.pool = H.pool;
+    P.programs = H.programs;
     qs::DevPass d{};
     d.args.m = (int)H.passes[pass].q.size();
     for (int j = 0; j < d.args.m; ++j) d.args.q[j] = H.passes[pass].q[j];
@@ -1299,10 +1282,10 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 }
 
 template <class E>
-__global__ void __launch_bounds__(kStThreads, 3) k_batch_staged(const BatchRec* __restrict__ recs, int nrec,
+__global__ void __launch_bounds__(kBatchThreads, 3) k_batch_staged(const BatchRec* __restrict__ recs, int nrec,
     ITYPE total, unsigned long long* head, unsigned* done, int* err, unsigned long long wait_ns) {
     __shared__ double2 tile[1 << kBatchTileBits];
-    __shared__ ITYPE hi_off[1 << (kBatchTileBits - 7)];
+    __shared__ ITYPE hi_off[16];
     __shared__ ITYPE s_item;
     __shared__ int s_rec, s_abort;
     __shared__ StPassArgs s_args;  // the record's pass, copied so the tile code indexes shared memory
@@ -1342,7 +1325,7 @@ __global__ void __launch_bounds__(kStThreads, 3) k_batch_staged(const BatchRec* 
             s_state = (E*)recs[s_rec].state;
         }
         __syncthreads();
-        staged_tile<kBatchTileBits, true>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
+        staged_tile<kBatchTileBits, kBatchThreads>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
         if (tid == 0) {
             __threadfence();
             atomicAdd(done + s_rec, 1u);
@@ -1358,7 +1341,7 @@ static int batch_block_size(const Circuit& c) { return (c.fusion_k >= 0 && c.fus
 static int ensure_batch_plan(Circuit& c, ITYPE dim) {
     const int k = batch_block_size(c);
     if (c.bplan && c.bplan->dim == dim && c.bk == k) return QS_OK;
-    c.bgates = fuse_gates(c.gates, k);
+    c.bgates = executor_gates(c.gates, k);
     c.bk = k;
     return build_plan(c.bgates, c.n, dim, &c.bplan, kBatchTileBits);
 }
@@ -1388,7 +1371,7 @@ static int batch_records(Circuit* const* cs, void* const* states, UINT count, st
             pool.emplace_back([&] {
                 for (UINT i; (i = next.fetch_add(1)) < count;)
                     if (need[i]) {
-                        fg[i] = fuse_gates(cs[i]->gates, batch_block_size(*cs[i]));
+                        fg[i] = executor_gates(cs[i]->gates, batch_block_size(*cs[i]));
                         make_host_plan(fg[i], cs[i]->n, &hp[i], kBatchTileBits);
                     }
             });
@@ -1455,16 +1438,16 @@ static int batch_kernel(void* buf, const BatchLayout& L, int nrec, ITYPE total, 
     cudaStream_t st) {
     int per_sm = 0;
     if (c64)
-        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<float2>, kStThreads, 0));
+        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<float2>, kBatchThreads, 0));
     else
-        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<double2>, kStThreads, 0));
+        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<double2>, kBatchThreads, 0));
     const ITYPE resident = (ITYPE)std::max(1, per_sm) * sm_count();
     const unsigned grid = (unsigned)std::min<ITYPE>(resident, total);
     const BatchRec* drec = (const BatchRec*)buf;
     if (c64)
-        k_batch_staged<float2><<<grid, kStThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
+        k_batch_staged<float2><<<grid, kBatchThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
     else
-        k_batch_staged<double2><<<grid, kStThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
+        k_batch_staged<double2><<<grid, kBatchThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
     return check_launch("k_batch_staged");
 }
 
@@ -1698,7 +1681,7 @@ extern "C" QS_API int qs_debug_batch_wait_expiry(qs_circuit_t circuit, void* sta
     UINT passes = 0;
     {
         qs::HostPlan H;
-        std::vector<qs::GateRec> fg = qs::fuse_gates(c->gates, qs::batch_block_size(*c));
+        std::vector<qs::GateRec> fg = qs::executor_gates(c->gates, qs::batch_block_size(*c));
         qs::make_host_plan(fg, c->n, &H, qs::kBatchTileBits);
         passes = (UINT)H.passes.size();
     }

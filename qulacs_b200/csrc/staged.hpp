@@ -1,7 +1,7 @@
 // Host-visible description of a staged pass (csrc/staged.cu builds it; csrc/pass_codegen.cpp turns one
 // pass into a specialised kernel).  A pass owns m tile qubits q[0..m-1] (ascending, q[j] = j for
 // j < kLowFixed); its gates run in phases of 4 tile bits, each phase a list of register ops on a
-// thread's 16-amplitude coset.
+// thread's 16-amplitude coset, run as a program of register steps.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,38 +18,59 @@ namespace qs {
 constexpr int kLowFixed = 4;        // qubits 0..3 always belong to a tile
 constexpr int kTileBits = 12;       // pass kernel: 2^12 amplitudes = 64 KiB of shared memory per CTA
 constexpr int kBatchTileBits = 11;  // multi-circuit kernel: 2^11 amplitudes = 32 KiB
-constexpr int kStThreads = 128;     // 16 (m = 11) or 32 (m = 12) amplitudes per thread; 1 or 2 cosets per phase
-constexpr int kPhaseBits = 4;       // 16 amplitudes in registers per thread
+constexpr int kPhaseBits = 4;       // 16 amplitudes (a coset) in registers per thread
+constexpr int kStThreads = 256;     // pass kernel: one coset per thread of a 2^12-amplitude tile
+constexpr int kBatchThreads = 128;  // multi-circuit kernel: one per thread of a 2^11-amplitude tile
 
-// ST_CSEL1, ST_D1_IN and ST_D1_OUT are a one-qubit dense gate with a CNOT (or CZ) folded in.
+// XOR swizzle of the tile index.  A quarter warp's eight 16-byte accesses are conflict-free when the
+// low three bits of swz() differ, that is when the swizzle vectors of the three tile bits that its lanes
+// run over are independent.  With these shifts every set of 4 phase bits out of 11 or 12 tile bits leaves
+// such a triple, which lane_order puts first.  Linear over XOR: swz(a | b) = swz(a) ^ swz(b) for disjoint bits.
+#define QS_SWZ(u) ((u) ^ ((((u) >> 3) ^ ((u) >> 5) ^ ((u) >> 6) ^ ((u) >> 8)) & 7u))
+
+// Gates of a phase, from which its program (phase_program.hpp) is built.
 enum StKind : uint8_t {
-    ST_DENSE1 = 0, ST_DIAG1, ST_RX, ST_RY, ST_CNOT, ST_CZ, ST_SWAP, ST_DENSE2, ST_CSEL1, ST_D1_IN, ST_D1_OUT
+    ST_DENSE1 = 0, ST_DIAG1, ST_RX, ST_RY, ST_CNOT, ST_CZ, ST_SWAP, ST_DENSE2,
+    // depolarizing channels of a density matrix seen as a vector; parameter: the channel's probability.
+    // a, b: column and row bit (one qubit), or the two column bits with the row bits in aux (two qubits)
+    ST_DEPOL1, ST_DEPOL2
 };
 
 struct StOp {
-    uint8_t kind, a, b, pad;  // a, b: register-bit indices 0..3 within the phase; pad: dispatch code
-    uint32_t param;           // index into the parameter pool (double2)
+    uint8_t kind, a, b, aux;  // a, b: register-bit indices 0..3 within the phase; aux: ST_DIAG1 1 = its phase is
+                              // a parameter, ST_DEPOL2 the row bits
+    uint32_t param;           // index into the parameter pool (double2); the parameters of ST_RX, ST_RY and
+                              // ST_DIAG1 are followed by their low parts (hi + lo)
+};
+// A step of a phase's program for the generic kernels.
+struct StStep {
+    uint8_t code, pad;
+    uint16_t mask;   // registers of a diagonal, or the register pairs of a rotation that run reversed
+    uint32_t param;  // index into the steps' parameter pool
 };
 struct StPhase {
     uint8_t bits[4];  // tile-local bit positions, ascending
-    uint32_t op_begin, op_count;
+    uint8_t order[8];  // tile bit of bit k of the coset number
+    uint8_t out0, out[4];  // after the steps register j holds coset index out0 ^ (XOR of out[k] over the bits k of j)
+    uint32_t op_begin, op_count;      // its gates (host)
+    uint32_t step_begin, step_count;  // its program
 };
 
 // One pass as the code generator sees it: tile qubits, the HBM-direct first/last phase flags, and the
-// host copies of its phases, ops and parameters.
+// programs of its phases.
+struct PhaseProgram;
 struct PassDesc {
     int m = 0;
     int io = 0;  // bit 0: the first phase gathers from HBM; bit 1: the last phase scatters to HBM
     UINT q[kTileBits] = {};
-    std::vector<StPhase> phases;  // op_begin indexes `ops`
-    const StOp* ops = nullptr;
-    const double2* pool = nullptr;
+    const StPhase* phases = nullptr;
+    const PhaseProgram* programs = nullptr;
+    int nphases = 0;
 };
 
-// csrc/pass_codegen.cpp: a kernel for one pass with its tile qubits, phase bits and op list compiled
+// csrc/pass_codegen.cpp: a kernel for one pass with its tile qubits, phase bits and programs compiled
 // in (NVRTC, sm_100a), cached by source for the life of the process.  `handle` receives the
-// cache entry (valid until exit), launched over dim >> m CTAs of kStThreads threads with 16 << m bytes
-// of dynamic shared memory.  QS_ERR_NOT_SUPPORTED when NVRTC cannot be loaded.
+// cache entry (valid until exit), launched over dim >> m CTAs with 16 << m bytes of dynamic shared memory.  QS_ERR_NOT_SUPPORTED when NVRTC cannot be loaded.
 // The kernel depends only on the pass's structure: its gate parameters are a kernel-parameter block
 // whose values `params` receives (empty when the pass has too many and they are literals instead), to
 // be passed at every launch.

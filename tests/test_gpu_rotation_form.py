@@ -1,0 +1,119 @@
+"""Specialised passes on circuits whose one-qubit gates sit at the edges of their rotation form: exact
+signs, flips and identities, near-flips (cosine below 2^-20), zero angles, projections and other
+non-unitary matrices, runs of mixed gates, every tile size, and depolarizing channels at the ends of
+their range."""
+import math
+
+import numpy as np
+import pytest
+
+from conftest import AMP_TOL, random_state, random_unitary
+from qulacs_b200 import DensityMatrix, QuantumCircuit, QuantumState, gate as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _one_qubit_gates(q, rng):
+    tiny = 2.0 ** -24
+    return [G.X(q), G.Y(q), G.Z(q), G.H(q), G.S(q), G.Tdag(q), G.sqrtX(q), G.sqrtYdag(q), G.RX(q, math.pi),
+            G.RY(q, math.pi), G.RY(q, math.pi - tiny), G.RX(q, math.pi + tiny), G.RY(q, 0.0), G.RZ(q, 0.0),
+            G.RX(q, 0.0), G.RZ(q, math.pi), G.RY(q, 5.0), G.RX(q, -4.0), G.U3(q, math.pi, 0.3, -1.0),
+            G.U3(q, 0.0, 0.2, 0.1), G.U3(q, 1e-9, 2.0, 1.0), G.DenseMatrix(q, random_unitary(1, rng)),
+            G.DenseMatrix(q, np.array([[1.1, 0.2j], [0.3, 0.8 - 0.1j]])),
+            G.DenseMatrix(q, np.array([[0.0, 0.9], [-1.2j, 0.0]])),
+            G.DenseMatrix(q, np.array([[0.0, 0.9], [1e-3, 0.0]])),
+            G.DiagonalMatrix([q], [0.9j, -1.1])]
+
+
+@pytest.mark.parametrize("n", [7, 11, 12, 14])
+@pytest.mark.parametrize("mode", ["staged", "staged_fused"])
+def test_edge_gates_against_oracle(port, n, mode):
+    rng = np.random.default_rng(70 + n)
+    c = QuantumCircuit(n)
+    c.set_specialized(1)
+    if mode == "staged_fused":
+        c.set_fusion(1)
+    want = random_state(n, rng)
+    s = QuantumState(n)
+    s.load(want)
+
+    def add(g, controls=()):
+        c.add_gate(g)
+        if g.name == "CNOT":
+            port.CNOT_gate(g.targets[0], g.targets[1], want)
+        elif g.name == "CZ":
+            port.CZ_gate(g.targets[0], g.targets[1], want)
+        else:
+            port.multi_qubit_dense_matrix_gate(g.targets, g.get_matrix(), want)
+
+    pool = [g for _ in range(6) for g in _one_qubit_gates(0, rng)]
+    for i in rng.permutation(len(pool)):
+        g = pool[i].copy()
+        g.targets = [int(rng.integers(n))]
+        add(g)
+        r = rng.random()
+        a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+        if r < 0.25:
+            add(G.CNOT(a, b))
+        elif r < 0.5:
+            add(G.CZ(a, b))
+        elif r < 0.6:
+            add(G.SWAP(a, b))
+        elif r < 0.65:
+            add(G.DenseMatrix([a, b], random_unitary(2, rng)))
+    for q in (0, n - 1):
+        add(G.P0(q))
+    c.update_quantum_state(s, mode=mode)
+    assert np.max(np.abs(s.get_vector() - want)) <= AMP_TOL * max(1.0, float(np.max(np.abs(want))))
+
+
+def test_long_runs_of_near_flips_keep_their_scale(port):
+    """200 near-flips on the qubits of one tile: the cosines deferred over a pass (2^-19 each) exceed the
+    bound on a deferred scale, so the later ones must not be deferred."""
+    n = 12
+    rng = np.random.default_rng(8)
+    c = QuantumCircuit(n)
+    c.set_specialized(1)
+    want = random_state(n, rng)
+    s = QuantumState(n)
+    s.load(want)
+    for i in range(200):
+        g = G.RY(i % n, math.pi - 2.0 ** -18) if i % 2 else G.RX(i % n, math.pi - 2.0 ** -18)
+        c.add_gate(g)
+        port.multi_qubit_dense_matrix_gate(g.targets, g.get_matrix(), want)
+        if i % n == n - 1:
+            c.add_gate(G.CNOT(0, n - 1))
+            port.CNOT_gate(0, n - 1, want)
+    c.update_quantum_state(s)
+    assert np.max(np.abs(s.get_vector() - want)) <= AMP_TOL
+
+
+@pytest.mark.parametrize("p1,p2", [(0.01, 0.02), (0.75, 15 / 16), (1.0, 1.0), (0.0, 0.9374)])
+@pytest.mark.parametrize("mode", ["staged", "staged_fused"])
+def test_channels_against_gate_by_gate(mode, p1, p2):
+    """11 qubits: the smallest density matrix whose passes are specialised.  The channel kernels of the
+    gate-by-gate mode are checked against the oracle in test_gpu_dm.py."""
+    n = 11
+    rng = np.random.default_rng(9)
+    c = QuantumCircuit(n)
+    for _ in range(3):
+        for q in range(n):
+            c.add_gate(G.RY(q, float(rng.uniform(0, 6))))
+            c.add_gate(G.DepolarizingNoise(q, p1))
+            c.add_gate(G.U3(q, *(float(x) for x in rng.uniform(0, 6, 3))))
+            c.add_gate(G.DepolarizingNoise(q, 0.03))
+        for _ in range(n):
+            a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+            c.add_gate(G.CZ(a, b) if rng.random() < 0.5 else G.CNOT(a, b))
+            c.add_gate(G.TwoQubitDepolarizingNoise(a, b, p2 if rng.random() < 0.2 else 0.01))
+        c.add_gate(G.DenseMatrix(3, np.array([[1.0, 0.1], [0.0, 0.9]])))  # not unitary: channels stay before it
+    if mode == "staged_fused":
+        c.set_fusion(2)
+    psi = QuantumState(n)
+    psi.set_Haar_random_state(4)
+    a, b = DensityMatrix(n), DensityMatrix(n)
+    a.load(psi)
+    b.load(psi)
+    c.update_quantum_state(a, mode=mode)
+    c.update_quantum_state(b, mode="gate_by_gate")
+    assert np.max(np.abs(a.get_matrix() - b.get_matrix())) <= AMP_TOL
