@@ -204,7 +204,7 @@ static void xmatrix(const GateRec& g, cl* m) {
 // carried forward -- through controls, CZ and diagonals, which commute with it -- into the D2 of the next
 // run on the qubit.  Gates that do not commute with a carried diagonal (CNOT targets, dense blocks, ...)
 // get it just before them.  Phases common to a whole state are multiplied up and emitted once at the end.
-std::vector<GateRec> rotation_form(const std::vector<GateRec>& G) {
+std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
     // A qubit's run of gates not emitted yet is diag(1, d), then a core, then diag(p0, p1).  The core is kept
     // as a rotation while it is one: which factors a run gets must not depend on the signs of its angles.
     enum Core { NONE, REAL, RX, MATRIX };
@@ -275,7 +275,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G) {
         k.post = k.post_free = false;
         k.p0 = k.p1 = 1.L;
         const cl zero(0.L);
-        if (core == RX && k.any) {
+        if (core == RX && (k.any || !spec)) {
             const ld c = k.c, s = k.s;
             k.m[0] = k.m[3] = c;
             k.m[1] = k.m[2] = cl(0.L, s);
@@ -322,22 +322,20 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G) {
             else diagonal(q, p0, p1, false);  // a projection; commutes with the carried diagonal
         }
     };
-    auto add_one = [&](const GateRec& g) {
-        Qubit& k = Q[g.targets[0]];
-        cl m[4];
-        xmatrix(g, m);
+    auto add_matrix = [&](UINT q, int kind, const cl* m) {
+        Qubit& k = Q[q];
         const cl zero(0.L);
         if (m[1] == zero && m[2] == zero) {
             k.p0 = xmul(m[0], k.p0);
             k.p1 = xmul(m[3], k.p1);
             k.post = true;
-            k.post_free = k.post_free || g.kind == QS_GATE_RZ;
-            if (k.core == NONE) end_run(g.targets[0]);
+            k.post_free = k.post_free || kind == QS_GATE_RZ;
+            if (k.core == NONE) end_run(q);
             return;
         }
         // a real rotation, or one after a sign of the |1> row
         bool real = true;
-        for (const cl& z : m) real = real && z.imag() == 0.L;
+        for (int i = 0; i < 4; ++i) real = real && m[i].imag() == 0.L;
         real = real && m[0] != zero && is_unitary2(m);
         if (real && !k.post && (k.core == NONE || k.core == REAL)) {
             const ld c = m[0].real(), s = m[1].real();
@@ -352,7 +350,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G) {
             }
             return;
         }
-        if (g.kind == QS_GATE_RX && !k.post && (k.core == NONE || k.core == RX)) {
+        if (kind == QS_GATE_RX && !k.post && (k.core == NONE || k.core == RX)) {
             const ld c = m[0].real(), s = m[1].imag();
             const ld c0 = k.core == RX ? k.c : 1.L, s0 = k.core == RX ? k.s : 0.L;
             k.core = RX;
@@ -372,9 +370,24 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G) {
         k.post = k.post_free = false;
         k.p0 = k.p1 = 1.L;
     };
+    const ld h = std::sqrt(0.5L);
+    const cl had[4] = {h, h, h, -h};
     for (const GateRec& g : G) {
         if (g.targets.size() == 1 && g.controls.empty() && g.kind != QS_GATE_DEPOLARIZING) {
-            add_one(g);
+            cl m[4];
+            xmatrix(g, m);
+            add_matrix(g.targets[0], g.kind, m);
+            continue;
+        }
+        if (g.kind == QS_GATE_CNOT && !spec) {
+            add_matrix(g.targets[1], QS_GATE_DENSE, had);
+            end_run(g.targets[0]);
+            end_run(g.targets[1]);
+            GateRec z;
+            z.kind = QS_GATE_CZ;
+            z.targets = g.targets;
+            out.push_back(z);
+            add_matrix(g.targets[1], QS_GATE_DENSE, had);
             continue;
         }
         for (UINT q : g.qubits()) end_run(q);
@@ -431,8 +444,8 @@ static bool dense_pays(const std::vector<GateRec>& G, ITYPE mask, const std::vec
     return cost > 16;
 }
 
-std::vector<GateRec> executor_gates(const std::vector<GateRec>& G, int k, size_t* blocks) {
-    return rotation_form(fuse_blocks(G, k, dense_pays, blocks));
+std::vector<GateRec> executor_gates(const std::vector<GateRec>& G, int k, bool spec, size_t* blocks) {
+    return rotation_form(fuse_blocks(G, k, dense_pays, blocks), spec);
 }
 
 // A one-qubit depolarizing channel commutes with every unitary on its qubit, and channels of strengths

@@ -26,10 +26,10 @@ struct Node {
     // diagonal factors: functionals of the register index (1 or 2 of them) and the 16 values
     int nf = 0;
     uint8_t g[2] = {};
-    uint8_t a = 0;      // affine part of g[0]
     bool sign = false;  // values +-1
     bool free = false;  // one functional, free phase: counts as a factor whatever its value
-    cl val[16];
+    cl lo = 1., hi = 1.;  // value where the factor's bits (its mask) are 0 and 1
+    uint16_t on = 0;
     ProgStep step;      // other nodes: in the algebra of X^v (v in vs) and Z^f (f in fs)
     int nv = 0, ns = 0;
     uint8_t vs[4], fs[4];
@@ -74,7 +74,7 @@ struct Builder {
     std::vector<Node> nodes;
     PassScalar& S;
     const bool move;  // CNOT, SWAP and X are steps; the map stays the identity
-    Builder(PassScalar& s, bool m) : S(s), move(m) {}
+    Builder(PassScalar& s, bool m, size_t gates) : S(s), move(m) { nodes.reserve(gates); }
 
     // qubit i of the node's step is register bit b; x, z: whether the node moves and reads it
     void set_qubit(Node& n, int i, int b, bool x = true, bool z = true) {
@@ -94,7 +94,6 @@ struct Builder {
         n.diag = true;
         n.nf = 1;
         n.g[0] = F[b];
-        n.a = A[b];
         const double m0 = (double)std::norm(d0), m1 = (double)std::norm(d1);
         const bool ok = m0 > 0.25 && m0 < 4. && m1 > 0.25 && m1 < 4.;
         n.free = free;
@@ -106,11 +105,13 @@ struct Builder {
             if (d0 != cl(1.)) scalar(d0, free);
             const cl r = d1 == -d0 ? cl(-1.) : d0 == cl(1.) ? d1 : d1 / d0;
             n.sign = !free && r == cl(-1.);
-            for (int j = 0; j < 16; ++j) n.val[j] = (par4(F[b] & j) ^ A[b]) ? r : cl(1.);
+            n.hi = r;
         } else {  // projections and the like
-            for (int j = 0; j < 16; ++j) n.val[j] = (par4(F[b] & j) ^ A[b]) ? d1 : d0;
+            n.lo = d0;
+            n.hi = d1;
         }
-        push(n);
+        for (int j = 0; j < 16; ++j) n.on |= (uint16_t)((par4(F[b] & j) ^ A[b]) << j);
+        push(std::move(n));
     }
     void scalar(cl z, bool free = false) {
         S.any = true;
@@ -123,9 +124,9 @@ struct Builder {
         n.nf = 2;
         n.g[0] = F[a];
         n.g[1] = F[b];
-        for (int j = 0; j < 16; ++j)
-            n.val[j] = ((par4(F[a] & j) ^ A[a]) && (par4(F[b] & j) ^ A[b])) ? cl(-1.) : cl(1.);
-        push(n);
+        n.hi = -1.;
+        for (int j = 0; j < 16; ++j) n.on |= (uint16_t)(((par4(F[a] & j) ^ A[a]) & (par4(F[b] & j) ^ A[b])) << j);
+        push(std::move(n));
     }
     // csim's RY {c, s; -s, c} (x = false) or RX {c, i s; i s, c}
     void rot(int b, ld c, ld s, bool x) {
@@ -149,7 +150,7 @@ struct Builder {
             n.step.form = base + 2;
             n.step.par.push_back(make_double2((double)c, (double)s));
         }
-        push(n);
+        push(std::move(n));
     }
     void flip(int b) {
         if (move) return perm(SP_X, b, -1);
@@ -160,7 +161,7 @@ struct Builder {
         n.step.kind = kind;
         set_qubit(n, 0, a, kind != SP_CNOT, kind != SP_X);
         if (b >= 0) set_qubit(n, 1, b, true, kind == SP_SWAP);
-        push(n);
+        push(std::move(n));
     }
     void cnot(int c, int t) {
         if (move) return perm(SP_CNOT, c, t);
@@ -186,7 +187,7 @@ struct Builder {
         n.step.kind = SP_DENSE1;
         set_qubit(n, 0, b);
         n.step.par.assign(m, m + 4);
-        push(n);
+        push(std::move(n));
     }
     void dense2(int a, int b, const double2* m) {
         Node n;
@@ -194,7 +195,7 @@ struct Builder {
         set_qubit(n, 0, a);
         set_qubit(n, 1, b);
         n.step.par.assign(m, m + 16);
-        push(n);
+        push(std::move(n));
     }
     // depolarizing channel of strength q (rho -> (1 - q) rho + q I / 2^k tr): column bits, then row bits
     void depol(const int* bits, int k, ld q) {
@@ -214,7 +215,7 @@ struct Builder {
             n.step.form = 1;
             n.step.par.push_back(make_double2((double)(q / 4), (double)(1.L - q)));
         }
-        push(n);
+        push(std::move(n));
     }
 
     void schedule(PhaseProgram* P) {
@@ -232,18 +233,22 @@ struct Builder {
             --left;
             for (int j : after[i]) --nodes[j].waits;
         };
-        auto others = [&]() {  // every ready step that is no diagonal
-            bool any = false, again = true;
-            while (again) {
-                again = false;
+        std::vector<int> ready;
+        auto others = [&]() {  // every ready step that is no diagonal, rotations by register bit
+            bool any = false;
+            while (true) {
+                ready.clear();
                 for (int i = 0; i < N; ++i)
-                    if (!nodes[i].done && !nodes[i].diag && nodes[i].waits == 0) {
-                        P->steps.push_back(nodes[i].step);
-                        finish(i);
-                        any = again = true;
-                    }
+                    if (!nodes[i].done && !nodes[i].diag && nodes[i].waits == 0) ready.push_back(i);
+                if (ready.empty()) return any;
+                std::stable_sort(ready.begin(), ready.end(),
+                    [&](int x, int y) { return (nodes[x].rot ? nodes[x].step.v[0] : 0) < (nodes[y].rot ? nodes[y].step.v[0] : 0); });
+                for (int i : ready) {
+                    P->steps.push_back(std::move(nodes[i].step));
+                    finish(i);
+                }
+                any = true;
             }
-            return any;
         };
         auto diagonals = [&](bool signs_only) {
             ProgStep s;
@@ -254,9 +259,12 @@ struct Builder {
             for (int i = 0; i < N; ++i) {
                 Node& n = nodes[i];
                 if (n.done || !n.diag || n.waits || (signs_only && !n.sign)) continue;
+                const bool lo = n.lo != cl(1.), hi = n.hi != cl(1.) || n.free;
                 for (int j = 0; j < 16; ++j) {
-                    if (n.val[j] != cl(1.) || (n.free && (par4(n.g[0] & j) ^ n.a))) touched[j] = true;
-                    val[j] = mulc(val[j], n.val[j]);
+                    const bool on = (n.on >> j) & 1;
+                    if (!(on ? hi : lo)) continue;
+                    touched[j] = true;
+                    val[j] = mulc(val[j], on ? n.hi : n.lo);
                 }
                 any = true;
                 sign = sign && n.sign;
@@ -276,7 +284,7 @@ struct Builder {
                     if (touched[j]) s.mask |= (uint16_t)(1u << j);
                 }
             }
-            P->steps.push_back(s);
+            P->steps.push_back(std::move(s));
         };
         while (left) {
             others();
@@ -309,7 +317,7 @@ std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count
             const bool diag = one && m[1].x == 0. && m[1].y == 0. && m[2].x == 0. && m[2].y == 0.;
             move = move || o->kind == ST_DENSE2 || o->kind == ST_DEPOL1 || o->kind == ST_DEPOL2 || (one && !flip && !diag);
         }
-        Builder B(S, move);
+        Builder B(S, move, (size_t)(end - begin));
         for (const StOp* op = begin; op != end; ++op) {
             const StOp& o = *op;
             const double2* p = pool + o.param;
@@ -357,10 +365,67 @@ std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count
     return out;
 }
 
+// The program as rounds, if it holds nothing else than signs, diagonals and scaled RY on register bits.
+static bool encode_rounds(const PhaseProgram& P, StPhase* phase, std::vector<double2>* pool) {
+    for (const ProgStep& s : P.steps) {
+        const bool ry = s.kind == SP_ROT && s.form == RF_Y_TAN && !(s.v[0] & (s.v[0] - 1)) && s.f[0] == s.v[0];
+        if (!ry && s.kind != SP_DIAG && s.kind != SP_SIGN && s.kind != SP_SCALE) return false;
+    }
+    const double2 one = make_double2(1., 0.);
+    double2 d[16];
+    double t[4];
+    int used;    // register bits with a rotation in this round
+    bool diag;
+    auto clear = [&]() {
+        for (double2& v : d) v = one;
+        for (double& v : t) v = 0.;
+        used = 0;
+        diag = false;
+    };
+    auto close = [&]() {
+        pool->insert(pool->end(), d, d + 16);
+        pool->push_back(make_double2(t[0], t[1]));
+        pool->push_back(make_double2(t[2], t[3]));
+        ++phase->rounds;
+        clear();
+    };
+    clear();
+    phase->param = (uint32_t)pool->size();
+    phase->rounds = phase->tail = 0;
+    for (const ProgStep& s : P.steps) {
+        if (s.kind == SP_ROT) {
+            const int b = __builtin_ctz(s.v[0]);
+            if (used >> b) close();  // ascending: the order in which a round runs them
+            used |= 1 << b;
+            t[b] = s.a[0] ? -s.par[0].x : s.par[0].x;
+            continue;
+        }
+        if (used) close();
+        diag = true;
+        for (int j = 0; j < 16; ++j) {
+            if (s.kind != SP_SCALE && !((s.mask >> j) & 1)) continue;
+            const double2 z = s.kind == SP_SIGN ? make_double2(-1., 0.) : s.par[s.kind == SP_SCALE ? 0 : j];
+            // signs next to factors stay exact
+            d[j] = make_double2(z.x * d[j].x - z.y * d[j].y, z.x * d[j].y + z.y * d[j].x);
+        }
+    }
+    if (used) close();
+    else if (diag) {
+        pool->insert(pool->end(), d, d + 16);
+        phase->tail = 1;
+    }
+    return true;
+}
+
 // Codes: run_step in csrc/staged.cu.
 void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vector<double2>* pool, StPhase* phase) {
     auto bit = [](uint8_t v) { return __builtin_ctz(v); };
     phase->step_begin = (uint32_t)steps->size();
+    phase->out0 = P.out[0];
+    for (int k = 0; k < 4; ++k) phase->out[k] = P.out[1 << k] ^ P.out[0];
+    phase->step_count = 0;
+    if (encode_rounds(P, phase, pool)) return;
+    phase->rounds = phase->tail = 0;
     for (const ProgStep& s : P.steps) {
         StStep t{};
         t.param = (uint32_t)pool->size();
@@ -399,8 +464,6 @@ void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vect
         steps->push_back(t);
     }
     phase->step_count = (uint32_t)(steps->size() - phase->step_begin);
-    phase->out0 = P.out[0];
-    for (int k = 0; k < 4; ++k) phase->out[k] = P.out[1 << k] ^ P.out[0];
 }
 
 }  // namespace qs

@@ -52,8 +52,8 @@ constexpr double kMaxDeferredBits = 400.;
 // The programs of a pass's phases, from its ops.
 std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count, const StOp* ops, const double2* pool);
 
-// A phase's program as the generic kernels read it: steps and parameters appended, and the phase's map from
-// register bits to tile bits after the steps filled in.
+// A phase's program as the generic kernels read it: rounds or steps and their parameters appended, and the
+// phase's map from register bits to tile bits after them filled in.
 void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vector<double2>* pool, StPhase* phase);
 
 // Value of a step's qubit i in register j.

@@ -15,10 +15,10 @@
 // pass kernel does not cover (more than 2 targets, controls, Pauli strings, multi-qubit diagonals) run
 // between passes with the gate-by-gate kernels.
 //
-// What bounds it on small states is the chain of steps in a CTA: one coset per thread (256 threads for a
-// 2^12-amplitude tile, where 128 threads took two in turn) and rotations in place of matrices halved it: the
-// 16-qubit layered circuit (16 tiles, 454 gates) and
-// its 64-string energy went from 0.495 to 0.287 ms.
+// What bounds the generic kernel on small states is the chain of steps in a CTA: one coset per thread (256
+// threads for a 2^12-amplitude tile, where 128 threads took two in turn) and rotations in place of matrices
+// brought the 16-qubit layered circuit (16 tiles, 454 gates) from 0.43 to 0.23 ms, rounds (run_rounds) to 0.21;
+// 20 layers of U3 + CZ on 26 qubits took 46.9 ms step by step and 29.2 in rounds (specialised: 16.0).
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -260,6 +260,24 @@ __device__ __forceinline__ void apply_step(const StStep& s, double2 (&r)[16], co
 #undef QS_CODE4
 #undef QS_CODE1
 
+// Rounds of 16 diagonal factors and a scaled rotation on each register bit (factor 1, tangent 0 where there is
+// none): straight-line code on fixed registers.  Conditions around the parts, or the switch over step kinds,
+// cost moves of the whole coset at every join: the FP64 pipe was 15 % busy at 63 % issue with the switch, 20 %
+// with conditions, 35 % (46 % in the fullest passes) with rounds.  Reading factors ahead across rounds gained
+// 3 % at 14 qubits and lost 3 % at 26, and was not kept.
+__device__ __forceinline__ void run_rounds(const StPhase& P, double2 (&r)[16], const double2* __restrict__ p) {
+#pragma unroll 1
+    for (UINT o = 0; o < P.rounds; ++o, p += 18) {
+        r_diag(r, p, 0xffffu);
+        const double2 t01 = ld_par(p + 16), t23 = ld_par(p + 17);
+        r_ry_tan<1>(r, t01.x, 0);
+        r_ry_tan<2>(r, t01.y, 0);
+        r_ry_tan<4>(r, t23.x, 0);
+        r_ry_tan<8>(r, t23.y, 0);
+    }
+    if (P.tail) r_diag(r, p, 0xffffu);
+}
+
 __device__ __forceinline__ UINT swz(UINT u) { return QS_SWZ(u); }
 
 // Tile index u = tid + k * THREADS has global offset base | lo_off | hi_off[k]: lo_off takes tid's bits to
@@ -376,7 +394,9 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
                     r[g ^ (g >> 1)] = *reinterpret_cast<const double2*>(tile_bytes + addr);
                 }
             }
-            for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
+            if (P.step_count == 0) run_rounds(P, r, a.pool + P.param);
+            else
+                for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
             // register j goes to coset index out0 ^ (XOR of out[k] over the bits k of j)
             auto tile_index = [&](UINT i) {
                 UINT u = 0;
@@ -463,11 +483,11 @@ static bool stageable(const GateRec& g) {
     }
 }
 
-static ITYPE qmask(const std::vector<UINT>& qs) {
-    ITYPE m = 0;
-    for (UINT q : qs) m |= 1ULL << q;
-    return m;
-}
+// A gate as the scheduler sees it.
+struct GateMask {
+    ITYPE q;    // its qubits
+    bool stage;  // runs inside passes
+};
 
 struct PassPlan {
     bool single = false;  // a gate run by the gate-by-gate kernels
@@ -477,28 +497,29 @@ struct PassPlan {
 };
 
 // Absorb greedily in program order with a fixed tile set; returns the absorbed gate indices.
-static std::vector<int> absorb(const std::vector<GateRec>& G, const std::vector<int>& pending, ITYPE Q, UINT n) {
-    std::vector<int> out;
+static void absorb(const std::vector<GateMask>& G, const std::vector<int>& pending, ITYPE Q, UINT n,
+    std::vector<int>* got) {
+    std::vector<int>& out = *got;
+    out.clear();
     ITYPE blocked = 0;
     const ITYPE all = (n >= 64) ? ~0ULL : ((1ULL << n) - 1);
     for (int gi : pending) {
-        const ITYPE gm = qmask(G[gi].qubits());
-        if ((gm & blocked) || !stageable(G[gi]) || (gm & ~Q)) {
+        const ITYPE gm = G[gi].q;
+        if ((gm & blocked) || !G[gi].stage || (gm & ~Q)) {
             blocked |= gm;
             if ((blocked & all) == all) break;
             continue;
         }
         out.push_back(gi);
     }
-    return out;
 }
 
 // Grow Q greedily in program order (capacity m), absorbing as we go.
-static ITYPE greedy_q(const std::vector<GateRec>& G, const std::vector<int>& pending, ITYPE Q, int m) {
+static ITYPE greedy_q(const std::vector<GateMask>& G, const std::vector<int>& pending, ITYPE Q, int m) {
     ITYPE blocked = 0;
     for (int gi : pending) {
-        const ITYPE gm = qmask(G[gi].qubits());
-        if ((gm & blocked) || !stageable(G[gi])) {
+        const ITYPE gm = G[gi].q;
+        if ((gm & blocked) || !G[gi].stage) {
             blocked |= gm;
             continue;
         }
@@ -509,15 +530,23 @@ static ITYPE greedy_q(const std::vector<GateRec>& G, const std::vector<int>& pen
     return Q;
 }
 
-static std::vector<PassPlan> plan_passes(const std::vector<GateRec>& G, UINT n, int tile_bits) {
+static std::vector<PassPlan> plan_passes(const std::vector<GateRec>& gates, UINT n, int tile_bits) {
     std::vector<PassPlan> plan;
+    std::vector<GateMask> G(gates.size());
+    for (size_t i = 0; i < G.size(); ++i) {
+        G[i] = {0, stageable(gates[i])};
+        for (UINT q : gates[i].targets) G[i].q |= 1ULL << q;
+        for (UINT q : gates[i].controls) G[i].q |= 1ULL << q;
+    }
+    std::vector<char> taken(G.size(), 0);
+    std::vector<int> got, best;
     std::vector<int> pending(G.size());
     for (size_t i = 0; i < G.size(); ++i) pending[i] = (int)i;
     const int m = (int)std::min<UINT>((UINT)tile_bits, n);
     const int low = std::min(kLowFixed, m);
     const ITYPE lowmask = (1ULL << low) - 1;
     while (!pending.empty()) {
-        if (!stageable(G[pending[0]])) {
+        if (!G[pending[0]].stage) {
             PassPlan p;
             p.single = true;
             p.gate = pending[0];
@@ -533,12 +562,12 @@ static std::vector<PassPlan> plan_passes(const std::vector<GateRec>& G, UINT n, 
             for (int j = 0; j < m - low; ++j) Q |= 1ULL << (a + j);
             cands.push_back(Q);
         }
-        std::vector<int> best;
+        best.clear();
         ITYPE bestQ = 0;
         for (ITYPE Q : cands) {
-            std::vector<int> got = absorb(G, pending, Q, n);
+            absorb(G, pending, Q, n, &got);
             if (got.size() > best.size()) {
-                best = got;
+                best.swap(got);
                 bestQ = Q;
             }
         }
@@ -557,12 +586,8 @@ static std::vector<PassPlan> plan_passes(const std::vector<GateRec>& G, UINT n, 
             if (bestQ >> q & 1ULL) p.q.push_back(q);
         p.gates = best;
         plan.push_back(p);
-        std::vector<char> taken(G.size(), 0);
         for (int gi : best) taken[gi] = 1;
-        std::vector<int> rest;
-        for (int gi : pending)
-            if (!taken[gi]) rest.push_back(gi);
-        pending.swap(rest);
+        pending.erase(std::remove_if(pending.begin(), pending.end(), [&](int gi) { return taken[gi] != 0; }), pending.end());
     }
     return plan;
 }
@@ -595,13 +620,6 @@ struct StagedPlan {
         if (dev) cudaFree(dev);
     }
 };
-
-// Tile-local bit of a global qubit.
-static int local_bit(const std::vector<UINT>& q, UINT g) {
-    for (size_t j = 0; j < q.size(); ++j)
-        if (q[j] == g) return (int)j;
-    return -1;
-}
 
 // The tile bits outside a phase, in the order in which the coset number's bits run over them: three with
 // independent swizzle vectors first (the lowest such triple, for conflict-free accesses), the others ascending.
@@ -644,7 +662,9 @@ struct HostPlan {
 
 // Host-only part of planning: passes, phases and their programs (no device calls).  The gates are in
 // rotation form.
-static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits = kTileBits) {
+// `spec`: the passes will run specialised kernels.
+static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits = kTileBits,
+    bool spec = false) {
     H->passes = plan_passes(gates, n, tile_bits);
     const std::vector<PassPlan>& passes = H->passes;
     std::vector<StPhase>& phases = H->phases;
@@ -658,58 +678,64 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
         }
         const size_t ph0 = phases.size();
         // phases: greedy over the pass's gates (program order) with 4 register bits each
-        std::vector<int> todo = p.gates;
+        struct Todo {
+            int gate;
+            UINT bits;  // its tile-local bits
+        };
+        std::vector<Todo> todo;
+        int local[64];
+        for (size_t j = 0; j < p.q.size(); ++j) local[p.q[j]] = (int)j;
+        for (int gi : p.gates) {
+            UINT bm = 0;
+            for (UINT g : gates[gi].targets) bm |= 1u << local[g];
+            todo.push_back({gi, bm});
+        }
+        std::vector<int> got, best;
         const int m = (int)p.q.size();
         while (!todo.empty()) {
-            std::vector<int> lb;  // per gate: its tile-local bits
             // candidates: greedy in order, and windows of 4 consecutive tile bits
-            auto bits_of = [&](int gi) {
-                ITYPE bm = 0;
-                for (UINT g : gates[gi].qubits()) bm |= 1ULL << local_bit(p.q, g);
-                return bm;
-            };
-            auto take = [&](ITYPE R, std::vector<int>* got) {
-                ITYPE blocked = 0;
-                for (int gi : todo) {
-                    const ITYPE bm = bits_of(gi);
+            auto take = [&](UINT R) {
+                got.clear();
+                UINT blocked = 0;
+                for (const Todo& t : todo) {
+                    const UINT bm = t.bits;
                     if ((bm & blocked) || (bm & ~R)) {
                         blocked |= bm;
                         continue;
                     }
-                    got->push_back(gi);
+                    got.push_back(t.gate);
                 }
             };
-            std::vector<ITYPE> cands;
+            std::vector<UINT> cands;
             {
-                ITYPE R = 0, blocked = 0;
-                for (int gi : todo) {
-                    const ITYPE bm = bits_of(gi);
+                UINT R = 0, blocked = 0;
+                for (const Todo& t : todo) {
+                    const UINT bm = t.bits;
                     if (bm & blocked) {
                         blocked |= bm;
                         continue;
                     }
-                    if (__builtin_popcountll(R | bm) <= kPhaseBits) R |= bm;
+                    if (__builtin_popcount(R | bm) <= kPhaseBits) R |= bm;
                     else blocked |= bm;
                 }
                 cands.push_back(R);
             }
-            for (int a0 = 0; a0 + kPhaseBits <= m; ++a0) cands.push_back(((1ULL << kPhaseBits) - 1) << a0);
-            std::vector<int> best;
-            ITYPE bestR = 0;
-            for (ITYPE R : cands) {
-                std::vector<int> got;
-                take(R, &got);
+            for (int a0 = 0; a0 + kPhaseBits <= m; ++a0) cands.push_back(((1u << kPhaseBits) - 1) << a0);
+            best.clear();
+            UINT bestR = 0;
+            for (UINT R : cands) {
+                take(R);
                 if (got.size() > best.size()) {
-                    best = got;
+                    best.swap(got);
                     bestR = R;
                 }
             }
-            for (int b = 0; b < m && __builtin_popcountll(bestR) < kPhaseBits; ++b) bestR |= 1ULL << b;
+            for (int b = 0; b < m && __builtin_popcount(bestR) < kPhaseBits; ++b) bestR |= 1u << b;
             StPhase ph{};
             int nb = 0;
             int regbit[64];
             for (int b = 0; b < m; ++b)
-                if (bestR >> b & 1ULL) {
+                if (bestR >> b & 1u) {
                     regbit[b] = nb;
                     ph.bits[nb++] = (uint8_t)b;
                 }
@@ -717,7 +743,7 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
             for (int gi : best) {
                 const GateRec& g = gates[gi];
                 StOp op{};
-                auto rb = [&](UINT gq) { return (uint8_t)regbit[local_bit(p.q, gq)]; };
+                auto rb = [&](UINT gq) { return (uint8_t)regbit[local[gq]]; };
                 op.param = (uint32_t)pool.size();
                 if (g.depol) {
                     op.kind = g.depol == 1 ? ST_DEPOL1 : ST_DEPOL2;
@@ -773,17 +799,15 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
             ph.op_count = (uint32_t)(ops.size() - ph.op_begin);
             lane_order(&ph, m);
             phases.push_back(ph);
-            std::vector<char> taken(gates.size(), 0);
-            for (int gi : best) taken[gi] = 1;
-            std::vector<int> rest;
-            for (int gi : todo)
-                if (!taken[gi]) rest.push_back(gi);
-            todo.swap(rest);
+            size_t at = 0;  // best lists todo's gates in order
+            todo.erase(std::remove_if(todo.begin(), todo.end(),
+                           [&](const Todo& t) { return at < best.size() && best[at] == t.gate && (++at, true); }),
+                todo.end());
         }
         std::vector<PhaseProgram> prog = build_pass_program(phases.data() + ph0, phases.size() - ph0, ops.data(), pool.data());
         for (size_t i = 0; i < prog.size(); ++i) {
-            encode_program(prog[i], &H->steps, &H->params, &phases[ph0 + i]);
-            H->programs.push_back(std::move(prog[i]));
+            if (!spec) encode_program(prog[i], &H->steps, &H->params, &phases[ph0 + i]);
+            else H->programs.push_back(std::move(prog[i]));
         }
         pp.push_back({ph0, phases.size() - ph0});
     }
@@ -792,9 +816,9 @@ static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* 
 static int upload_plan(const HostPlan& H, ITYPE dim, std::shared_ptr<StagedPlan>* out);
 
 static int build_plan(const std::vector<GateRec>& gates, UINT n, ITYPE dim, std::shared_ptr<StagedPlan>* out,
-    int tile_bits = kTileBits) {
+    int tile_bits = kTileBits, bool spec = false) {
     HostPlan H;
-    make_host_plan(gates, n, &H, tile_bits);
+    make_host_plan(gates, n, &H, tile_bits, spec);
     return upload_plan(H, dim, out);
 }
 
@@ -925,11 +949,14 @@ static bool want_specialized(const Circuit& c, ITYPE dim) {
 }
 
 static int ensure_plan(Circuit& c, ITYPE dim) {
-    if (!c.plan || c.plan->dim != dim) {
-        c.rgates = rotation_form(c.gates);
-        QS_TRY(build_plan(c.rgates, c.n, dim, &c.plan));
-    }
-    if (want_specialized(c, dim)) QS_TRY(specialize_plan(*c.plan));
+    if (c.plan && c.plan->dim == dim) return QS_OK;
+    const bool spec = want_specialized(c, dim);
+    std::shared_ptr<StagedPlan> P;
+    std::vector<GateRec> g = rotation_form(c.gates, spec);
+    QS_TRY(build_plan(g, c.n, dim, &P, kTileBits, spec));
+    if (spec) QS_TRY(specialize_plan(*P));
+    c.rgates.swap(g);
+    c.plan = P;
     return QS_OK;
 }
 
@@ -1042,20 +1069,22 @@ static int ensure_fused_plan(Circuit& c, ITYPE dim, cudaStream_t st) {
     if (c.fplan && c.fplan->dim == dim) return QS_OK;
     const bool spec = want_specialized(c, dim);
     if (c.fusion_k >= 0) {
-        c.fgates = executor_gates(c.gates, c.fusion_k, &c.fused_count);
+        c.fgates = executor_gates(c.gates, c.fusion_k, spec, &c.fused_count);
         c.fused_k = c.fusion_k;
         c.fused_tile_bits = kTileBits;
-        QS_TRY(build_plan(c.fgates, c.n, dim, &c.fplan));
-        if (spec) QS_TRY(specialize_plan(*c.fplan));
+        std::shared_ptr<StagedPlan> P;
+        QS_TRY(build_plan(c.fgates, c.n, dim, &P, kTileBits, spec));
+        if (spec) QS_TRY(specialize_plan(*P));
+        c.fplan = P;
         return QS_OK;
     }
     c.tune_ms.assign(kTuneSlots, -1.);
     double best = 0.;
     auto consider = [&](int k, int tile_bits, int slot) -> int {
         size_t count = 0;
-        std::vector<GateRec> fg = executor_gates(c.gates, k, &count);
+        std::vector<GateRec> fg = executor_gates(c.gates, k, spec, &count);
         std::shared_ptr<StagedPlan> P;
-        QS_TRY(build_plan(fg, c.n, dim, &P, tile_bits));
+        QS_TRY(build_plan(fg, c.n, dim, &P, tile_bits, spec));
         double ms = 0.;
         QS_TRY(estimate_plan_ms(fg, *P, dim, st, spec, &ms));
         c.tune_ms[slot] = ms;
@@ -1095,7 +1124,7 @@ static int c64_block_size(const Circuit& c) { return (c.fusion_k >= 0 && c.fusio
 static int ensure_c64_plan(Circuit& c, ITYPE dim) {
     const int k = c64_block_size(c);
     if (c.cplan && c.cplan->dim == dim && c.ck == k) return QS_OK;
-    c.cgates = executor_gates(c.gates, k);
+    c.cgates = executor_gates(c.gates, k, false);
     c.ck = k;
     QS_TRY(build_plan(c.cgates, c.n, dim, &c.cplan));
     for (const DevPass& d : c.cplan->passes)
@@ -1124,7 +1153,7 @@ int staged_pass_count(Circuit& c, ITYPE dim, UINT* out) {
         return QS_OK;
     }
     HostPlan H;
-    make_host_plan(rotation_form(c.gates), c.n, &H);
+    make_host_plan(rotation_form(c.gates, true), c.n, &H, kTileBits, true);
     *out = (UINT)H.passes.size();
     return QS_OK;
 }
@@ -1138,7 +1167,7 @@ extern "C" QS_API int qs_circuit_staged_stats(qs_circuit_t circuit, QS_UINT* pas
     qs::Circuit* c = reinterpret_cast<qs::Circuit*>(circuit);
     if (!c || !passes || !phases || !ops || !single_gates) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
     qs::HostPlan H;
-    qs::make_host_plan(qs::rotation_form(c->gates), c->n, &H);
+    qs::make_host_plan(qs::rotation_form(c->gates, true), c->n, &H, qs::kTileBits, true);
     UINT single = 0;
     for (const qs::PassPlan& p : H.passes) single += p.single ? 1 : 0;
     *passes = (QS_UINT)H.passes.size();
@@ -1203,7 +1232,7 @@ extern "C" QS_API int qs_circuit_specialized_source(qs_circuit_t circuit, QS_ITY
     if (dim != (1ULL << c->n)) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "dim differs from 2^qubit_count");
     if (c->n < (UINT)qs::kPhaseBits + 3) return qs::set_error(QS_ERR_NOT_SUPPORTED, "fewer than 7 qubits");
     qs::HostPlan H;
-    qs::make_host_plan(qs::rotation_form(c->gates), c->n, &H);
+    qs::make_host_plan(qs::rotation_form(c->gates, true), c->n, &H, qs::kTileBits, true);
     if (pass >= H.passes.size() || H.passes[pass].single)
         return qs::set_error(QS_ERR_INVALID_ARGUMENT, "no such staged pass");
     qs::StagedPlan P;
@@ -1341,7 +1370,7 @@ static int batch_block_size(const Circuit& c) { return (c.fusion_k >= 0 && c.fus
 static int ensure_batch_plan(Circuit& c, ITYPE dim) {
     const int k = batch_block_size(c);
     if (c.bplan && c.bplan->dim == dim && c.bk == k) return QS_OK;
-    c.bgates = executor_gates(c.gates, k);
+    c.bgates = executor_gates(c.gates, k, false);
     c.bk = k;
     return build_plan(c.bgates, c.n, dim, &c.bplan, kBatchTileBits);
 }
@@ -1371,7 +1400,7 @@ static int batch_records(Circuit* const* cs, void* const* states, UINT count, st
             pool.emplace_back([&] {
                 for (UINT i; (i = next.fetch_add(1)) < count;)
                     if (need[i]) {
-                        fg[i] = executor_gates(cs[i]->gates, batch_block_size(*cs[i]));
+                        fg[i] = executor_gates(cs[i]->gates, batch_block_size(*cs[i]), false);
                         make_host_plan(fg[i], cs[i]->n, &hp[i], kBatchTileBits);
                     }
             });
@@ -1681,7 +1710,7 @@ extern "C" QS_API int qs_debug_batch_wait_expiry(qs_circuit_t circuit, void* sta
     UINT passes = 0;
     {
         qs::HostPlan H;
-        std::vector<qs::GateRec> fg = qs::executor_gates(c->gates, qs::batch_block_size(*c));
+        std::vector<qs::GateRec> fg = qs::executor_gates(c->gates, qs::batch_block_size(*c), false);
         qs::make_host_plan(fg, c->n, &H, qs::kBatchTileBits);
         passes = (UINT)H.passes.size();
     }

@@ -45,7 +45,7 @@ struct StOp {
 // A step of a phase's program for the generic kernels.
 struct StStep {
     uint8_t code, pad;
-    uint16_t mask;   // registers of a diagonal, or the register pairs of a rotation that run reversed
+    uint16_t mask;   // registers of a diagonal or of signs, or the register pairs of a rotation that run reversed
     uint32_t param;  // index into the steps' parameter pool
 };
 struct StPhase {
@@ -53,7 +53,10 @@ struct StPhase {
     uint8_t order[8];  // tile bit of bit k of the coset number
     uint8_t out0, out[4];  // after the steps register j holds coset index out0 ^ (XOR of out[k] over the bits k of j)
     uint32_t op_begin, op_count;      // its gates (host)
-    uint32_t step_begin, step_count;  // its program
+    // Its program for the generic kernels: `rounds` of 16 diagonal factors and 4 tangents (16 + 2 entries of the
+    // parameter pool from `param`), then 16 more factors if `tail`; or, where it needs other steps, those.
+    uint32_t rounds, tail, param;
+    uint32_t step_begin, step_count;
 };
 
 // One pass as the code generator sees it: tile qubits, the HBM-direct first/last phase flags, and the
