@@ -283,6 +283,12 @@ template <class T>
 int ev_tiled(const PauliTerm* terms, const std::vector<int>& xidx, UINT n, const T* s, ITYPE dim, cudaStream_t st,
     double* values, std::vector<int>* rest, std::vector<int>* zidx);
 
+constexpr UINT kBatchEvSingleQubits = 18;  // states at least this large are evaluated by passes of their own
+// values[k] of the listed terms of one state, in one launch (one job per bit-flip string).
+template <class T>
+int ev_listed(const PauliTerm* terms, const std::vector<int>& zidx, const std::vector<int>& xidx, const T* s, ITYPE dim,
+    cudaStream_t st, double* values);
+
 template <class T>
 int ev_batch(const PauliTerm* terms, UINT count, const T* s, ITYPE dim, cudaStream_t st, double* values) {
     std::vector<int> zidx, xidx;
@@ -307,6 +313,11 @@ int ev_batch(const PauliTerm* terms, UINT count, const T* s, ITYPE dim, cudaStre
         part = (double*)buf;
         dz = (ITYPE*)((char*)buf + sizeof(double) * part_doubles);
     }
+    // What is left of a small state's terms goes out as one launch: it is in the L2 cache, and a launch, a
+    // fold and a synchronisation per string cost ~20 us (30 strings at 10 qubits: 600 us, in one launch 30).  A
+    // large state is read from HBM once per string either way, and its strings come 16 to a pass or alone.
+    if (n < kBatchEvSingleQubits && zidx.size() + xidx.size() > 1)
+        return ev_listed<T>(terms, zidx, xidx, s, dim, st, values);
     // Z-only terms left: kZChunk per pass.
     for (size_t c0 = 0; c0 < zidx.size(); c0 += kZChunk) {
         const int nz = (int)std::min<size_t>(kZChunk, zidx.size() - c0);
@@ -921,17 +932,108 @@ extern "C" QS_API int qs_batch_expectation_values_c64(void* const* states, const
         (cudaStream_t)stream);
 }
 namespace qs {
-constexpr UINT kBatchEvSingleQubits = 18;  // states at least this large are evaluated on their own
+// Work of k_batch_ev: jobs, and the masks and outputs of the Z-only ones.
+struct EvJobs {
+    std::vector<EvJob> jobs;
+    std::vector<ITYPE> zm;
+    std::vector<UINT> zout;
+    ITYPE total = 0;
+
+    void add(EvJob J) {
+        J.prefix = total;
+        total += (J.items + kEvChunk - 1) / kEvChunk;
+        jobs.push_back(J);
+    }
+    void flip(const void* s, int c64, ITYPE dim, const PauliTerm& t, UINT out) {
+        EvJob J{};
+        J.s = s;
+        J.c64 = c64;
+        J.items = dim / 2;
+        J.x = t.x;
+        J.z = t.z;
+        J.nrot = t.nrot;
+        J.pivot = t.pivot;
+        J.kind = 1;
+        J.out = out;
+        add(J);
+    }
+    // up to kEvZ Z-only terms (mask, output)
+    void z_only(const void* s, int c64, ITYPE dim, const ITYPE* masks, const UINT* outs, int count) {
+        EvJob J{};
+        J.s = s;
+        J.c64 = c64;
+        J.items = dim;
+        J.kind = 0;
+        J.nz = count;
+        J.zoff = (UINT)zm.size();
+        zm.insert(zm.end(), masks, masks + count);
+        zout.insert(zout.end(), outs, outs + count);
+        add(J);
+    }
+    // values[0 .. nvals): one upload, the jobs, their folds, one copy back
+    int run(UINT nvals, cudaStream_t st, double* values) const {
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t bj = up(sizeof(EvJob) * jobs.size()), bz = up(sizeof(ITYPE) * (zm.size() + 1)),
+                     bo = up(sizeof(UINT) * (zout.size() + 1)), bp = up(sizeof(double) * kEvZ * total);
+        void* buf;
+        QS_TRY(scratch(st, bj + bz + bo + bp + sizeof(double) * nvals, &buf));
+        char* p = (char*)buf;
+        std::vector<char> host(bj + bz + bo);
+        memcpy(host.data(), jobs.data(), sizeof(EvJob) * jobs.size());
+        if (!zm.empty()) {
+            memcpy(host.data() + bj, zm.data(), sizeof(ITYPE) * zm.size());
+            memcpy(host.data() + bj + bz, zout.data(), sizeof(UINT) * zout.size());
+        }
+        const EvJob* dj = (const EvJob*)p;
+        double* dpart = (double*)(p + bj + bz + bo);
+        double* dval = (double*)(p + bj + bz + bo + bp);
+        QS_CUDA_CHECK(cudaMemcpyAsync(p, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+        const unsigned grid = (unsigned)std::min<ITYPE>(total, (ITYPE)sm_count() * 8);
+        k_batch_ev<<<grid, 256, 0, st>>>(dj, (int)jobs.size(), total, (const ITYPE*)(p + bj), dpart);
+        QS_TRY(check_launch("k_batch_ev"));
+        k_batch_ev_fold<<<(unsigned)jobs.size(), 256, 0, st>>>(dj, dpart, (const UINT*)(p + bj + bz), dval);
+        QS_TRY(check_launch("k_batch_ev_fold"));
+        QS_CUDA_CHECK(cudaMemcpyAsync(values, dval, sizeof(double) * nvals, cudaMemcpyDeviceToHost, st));
+        QS_CUDA_CHECK(cudaStreamSynchronize(st));
+        return QS_OK;
+    }
+};
+
+template <class T>
+int ev_listed(const PauliTerm* terms, const std::vector<int>& zidx, const std::vector<int>& xidx, const T* s, ITYPE dim,
+    cudaStream_t st, double* values) {
+    constexpr int c64 = sizeof(T) == sizeof(float2);
+    EvJobs W;
+    UINT at = 0;  // values in the order of zidx, then xidx
+    for (size_t z0 = 0; z0 < zidx.size(); z0 += kEvZ) {
+        ITYPE m[kEvZ];
+        UINT o[kEvZ];
+        int c = 0;
+        for (; c < kEvZ && z0 + c < zidx.size(); ++c) {
+            m[c] = terms[zidx[z0 + c]].z;
+            o[c] = at++;
+        }
+        W.z_only(s, c64, dim, m, o, c);
+    }
+    for (int k : xidx) W.flip(s, c64, dim, terms[k], at++);
+    std::vector<double> v(at);
+    QS_TRY(W.run(at, st, v.data()));
+    at = 0;
+    for (int k : zidx) values[k] = v[at++];
+    for (int k : xidx) values[k] = v[at++];
+    return QS_OK;
+}
+template int ev_listed<double2>(const PauliTerm*, const std::vector<int>&, const std::vector<int>&, const double2*, ITYPE,
+    cudaStream_t, double*);
+template int ev_listed<float2>(const PauliTerm*, const std::vector<int>&, const std::vector<int>&, const float2*, ITYPE,
+    cudaStream_t, double*);
 
 // `skip_large`: leave the terms of states of >= kBatchEvSingleQubits qubits to the caller.
 static int batch_ev_impl(void* const* states, const QS_UINT* qubit_counts, QS_UINT count, const QS_UINT* term_offsets,
     const QS_ITYPE* x_masks, const QS_ITYPE* z_masks, const QS_UINT* y_counts, double* values, int c64,
     cudaStream_t st, bool skip_large) {
     if (!states || !qubit_counts || !term_offsets || !values) return set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
-    std::vector<EvJob> jobs;
-    std::vector<ITYPE> zm;
-    std::vector<UINT> zout;
-    ITYPE total = 0;
+    EvJobs W;
     const UINT nterms = term_offsets[count];
     for (UINT i = 0; i < count; ++i) {
         const UINT n = qubit_counts[i];
@@ -958,73 +1060,34 @@ static int batch_ev_impl(void* const* states, const QS_UINT* qubit_counts, QS_UI
             }
             continue;
         }
-        std::vector<UINT> zlist;
+        ITYPE zmask[kEvZ];
+        UINT zidx[kEvZ];
+        int nz = 0;
         for (UINT k = term_offsets[i]; k < term_offsets[i + 1]; ++k) {
             if ((x_masks[k] | z_masks[k]) >> n)
                 return set_error(QS_ERR_INVALID_ARGUMENT, "batch expectation: mask beyond qubit count");
             if (x_masks[k] == 0) {
-                zlist.push_back(k);
+                zmask[nz] = z_masks[k];
+                zidx[nz++] = k;
+                if (nz == kEvZ) {
+                    W.z_only(states[i], c64, dim, zmask, zidx, nz);
+                    nz = 0;
+                }
                 continue;
             }
-            EvJob J{};
-            J.s = states[i];
-            J.c64 = c64;
-            J.items = dim / 2;
-            J.prefix = total;
-            J.x = x_masks[k];
-            J.z = z_masks[k];
-            J.nrot = y_counts[k];
-            J.pivot = (UINT)(63 - __builtin_clzll(x_masks[k]));
-            J.kind = 1;
-            J.out = k;
-            total += (J.items + kEvChunk - 1) / kEvChunk;
-            jobs.push_back(J);
+            PauliTerm t;
+            t.x = x_masks[k];
+            t.z = z_masks[k];
+            t.nrot = y_counts[k];
+            t.pivot = (UINT)(63 - __builtin_clzll(x_masks[k]));
+            W.flip(states[i], c64, dim, t, k);
         }
-        for (size_t z0 = 0; z0 < zlist.size(); z0 += kEvZ) {
-            EvJob J{};
-            J.s = states[i];
-            J.c64 = c64;
-            J.items = dim;
-            J.prefix = total;
-            J.kind = 0;
-            J.nz = (int)std::min<size_t>(kEvZ, zlist.size() - z0);
-            J.zoff = (UINT)zm.size();
-            for (int w = 0; w < J.nz; ++w) {
-                zm.push_back(z_masks[zlist[z0 + w]]);
-                zout.push_back(zlist[z0 + w]);
-            }
-            total += (J.items + kEvChunk - 1) / kEvChunk;
-            jobs.push_back(J);
-        }
+        if (nz) W.z_only(states[i], c64, dim, zmask, zidx, nz);
     }
-    if (jobs.empty()) return QS_OK;
-    const size_t bj = sizeof(EvJob) * jobs.size(), bz = sizeof(ITYPE) * (zm.size() + 1),
-                 bo = sizeof(UINT) * (zout.size() + 1), bp = sizeof(double) * kEvZ * total,
-                 bv = sizeof(double) * nterms;
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    void* buf;
-    QS_TRY(scratch(st, up(bj) + up(bz) + up(bo) + up(bp) + up(bv), &buf));
-    char* p = (char*)buf;
-    EvJob* dj = (EvJob*)p;
-    ITYPE* dz = (ITYPE*)(p + up(bj));
-    UINT* dzo = (UINT*)(p + up(bj) + up(bz));
-    double* dpart = (double*)(p + up(bj) + up(bz) + up(bo));
-    double* dval = (double*)(p + up(bj) + up(bz) + up(bo) + up(bp));
-    QS_CUDA_CHECK(cudaMemcpyAsync(dj, jobs.data(), bj, cudaMemcpyHostToDevice, st));
-    if (!zm.empty()) {
-        QS_CUDA_CHECK(cudaMemcpyAsync(dz, zm.data(), sizeof(ITYPE) * zm.size(), cudaMemcpyHostToDevice, st));
-        QS_CUDA_CHECK(cudaMemcpyAsync(dzo, zout.data(), sizeof(UINT) * zout.size(), cudaMemcpyHostToDevice, st));
-    }
-    QS_CUDA_CHECK(cudaMemsetAsync(dval, 0, bv, st));
-    const unsigned grid = (unsigned)std::min<ITYPE>(total, (ITYPE)sm_count() * 8);
-    k_batch_ev<<<grid, 256, 0, st>>>(dj, (int)jobs.size(), total, dz, dpart);
-    QS_TRY(check_launch("k_batch_ev"));
-    k_batch_ev_fold<<<(unsigned)jobs.size(), 256, 0, st>>>(dj, dpart, dzo, dval);
-    QS_TRY(check_launch("k_batch_ev_fold"));
+    if (W.jobs.empty()) return QS_OK;
     // only the entries of the states evaluated here (large states' values are already in `values`)
     std::vector<double> hv(nterms);
-    QS_CUDA_CHECK(cudaMemcpyAsync(hv.data(), dval, bv, cudaMemcpyDeviceToHost, st));
-    QS_CUDA_CHECK(cudaStreamSynchronize(st));
+    QS_TRY(W.run(nterms, st, hv.data()));
     for (UINT i = 0; i < count; ++i)
         if (qubit_counts[i] < kBatchEvSingleQubits)
             for (UINT k = term_offsets[i]; k < term_offsets[i + 1]; ++k) values[k] = hv[k];

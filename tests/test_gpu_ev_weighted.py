@@ -162,3 +162,22 @@ def test_weighted_identity_repeated_and_zero_terms(port, kernels):
     obs = observable(n, terms, coefs)
     want = oracle_sum(port, a, terms, coefs).real
     assert abs(obs.get_expectation_value(s) - want) <= EV_TOL * float(np.sum(np.abs(coefs)))
+
+
+@pytest.mark.parametrize("c64", [False, True])
+@pytest.mark.parametrize("n,terms", [(1, 2), (2, 3), (5, 17), (10, 40), (11, 3), (17, 3)])
+def test_small_state_strings_in_one_launch(port, n, terms, c64):
+    """States below the pass evaluator (or with too few strings for it): every string of the call in one
+    launch, Z-only strings 16 to a job, against the oracle."""
+    rng = np.random.default_rng(300 + n)
+    v = random_state(n, rng)
+    if c64:
+        v = v.astype(np.complex64).astype(np.complex128)
+    s = QuantumStateC64(n) if c64 else QuantumState(n)
+    s.load(v)
+    ts = W.random_pauli_terms(n, terms, 1, min(4, n), seed=n)
+    ts += [(0.5, [q], [3]) for q in range(n)]
+    obs = W.to_observable(ts, n)
+    want = np.array([port.expectation_value(tl, ids, v) for _, tl, ids in ts])
+    assert np.max(np.abs(obs.term_values(s) - want)) <= EV_TOL
+    assert abs(obs.get_expectation_value(s) - float(np.dot([t[0] for t in ts], want))) <= EV_TOL * len(ts)
