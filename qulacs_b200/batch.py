@@ -20,7 +20,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import call
-from .observable import masks
+from .observable import masks_of
 from .state import QuantumState
 
 ALIGN = 256
@@ -108,23 +108,12 @@ class BatchRunner:
             else:  # every circuit in one persistent launch
                 call("qs_batch_update_quantum_states", circs, states, k, self.stream)
             # all terms of all observables in one launch
-            xm, zm, ny, offs, coefs, nq = [], [], [], [0], [], []
-            for i in wave:
-                obs = jobs[i][1]
-                for t in obs.terms:
-                    x, z, y = masks(t.targets, t.ids)
-                    xm.append(x)
-                    zm.append(z)
-                    ny.append(y)
-                    coefs.append(t.coef)
-                offs.append(len(xm))
-                nq.append(jobs[i][0].qubit_count)
-            xa = np.ascontiguousarray(np.array(xm, dtype=np.uint64))
-            za = np.ascontiguousarray(np.array(zm, dtype=np.uint64))
-            ya = np.ascontiguousarray(np.array(ny, dtype=np.uint32))
-            oa = np.ascontiguousarray(np.array(offs, dtype=np.uint32))
-            qa = np.ascontiguousarray(np.array(nq, dtype=np.uint32))
-            ca = np.ascontiguousarray(np.array(coefs, dtype=np.complex128)).view(np.float64)
+            terms = [t for i in wave for t in jobs[i][1].terms]
+            xa, za, ya = masks_of(terms)
+            oa = np.zeros(k + 1, dtype=np.uint32)
+            np.cumsum([len(jobs[i][1].terms) for i in wave], out=oa[1:])
+            qa = np.array([jobs[i][0].qubit_count for i in wave], dtype=np.uint32)
+            ca = np.array([t.coef for t in terms], dtype=np.complex128).view(np.float64)
             energies = np.zeros(2 * k)
             vp = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
             call("qs_batch_expectation_weighted", states, vp(qa), k, vp(oa), vp(xa), vp(za), vp(ya), vp(ca),

@@ -223,7 +223,7 @@ class QuantumState:
         out = np.empty(sampling_count, dtype=np.uint64)
         call("qs_state_sampling", self._ptr, self.dim, int(sampling_count), int(random_seed) & 0xFFFFFFFF,
              _ptr(out), self.stream)
-        return [int(x) for x in out]
+        return out.tolist()
 
     def sampling_with_uniforms(self, uniforms) -> np.ndarray:
         u = np.ascontiguousarray(np.asarray(uniforms, dtype=np.float64))
@@ -492,7 +492,7 @@ class DensityMatrix:
             random_seed = _random_seed()
         u = np.empty(int(sampling_count), dtype=np.float64)
         call("qs_reference_uniforms", int(random_seed) & 0xFFFFFFFF, u.size, _ptr(u))
-        return [int(x) for x in self.sampling_with_uniforms(u)]
+        return self.sampling_with_uniforms(u).tolist()
 
     def sampling_with_uniforms(self, uniforms) -> np.ndarray:
         u = np.ascontiguousarray(np.asarray(uniforms, dtype=np.float64))

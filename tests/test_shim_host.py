@@ -221,3 +221,34 @@ def test_observable_copy_hermitian_and_matrix():
     c2 = QuantumCircuit(8)
     c2.add_FusedSWAP_gate(0, 4, 2)
     assert c2.gate_list[0].get_name() == "FusedSWAP" and c2.gate_list[0].get_target_index_list() == [0, 1, 4, 5]
+
+
+def test_masks_of_many_terms_equal_the_one_by_one_masks():
+    """Array masks against masks() per operator, at the sizes on both sides of the switch: empty operators,
+    identity factors, repeated qubits, Y counts, unequal lists and the highest qubit."""
+    import numpy as np
+
+    from qulacs_b200 import PauliOperator
+    from qulacs_b200.observable import masks, masks_of
+    rng = np.random.default_rng(5)
+    for count in (0, 1, 47, 48, 300):
+        ops = []
+        for _ in range(count):
+            n = int(rng.integers(0, 7))
+            op = PauliOperator(coef=1.0, targets=[int(q) for q in rng.choice(64, size=n, replace=False)],
+                               pauli_ids=[int(p) for p in rng.integers(0, 4, size=n)])
+            if n and rng.random() < 0.1:
+                op.targets.append(op.targets[0])  # lists are public: a repeated qubit, and one id more or less
+                op.ids.append(2)
+            if n and rng.random() < 0.1:
+                op.ids.pop()
+            ops.append(op)
+        x, z, y = masks_of(ops)
+        assert (x.dtype, z.dtype, y.dtype) == (np.uint64, np.uint64, np.uint32) and x.size == count
+        for i, op in enumerate(ops):
+            assert (int(x[i]), int(z[i]), int(y[i])) == masks(op.targets, op.ids)
+    for bad in (4, -1):
+        ops = [PauliOperator(coef=1.0, targets=[0], pauli_ids=[1]) for _ in range(60)]
+        ops[7].ids[0] = bad
+        with pytest.raises(ValueError):
+            masks_of(ops)
