@@ -369,25 +369,37 @@ __global__ void __launch_bounds__(256) k_chunk_sums(const T* __restrict__ s, ITY
     if (threadIdx.x == 0) sums[blockIdx.x] = acc;
 }
 
-// Inclusive scan of n values by one CTA of 1024 threads: thread t owns a contiguous range.
+// Inclusive scan of n values by one CTA of 1024 threads: thread t owns a contiguous range.  The threads' offsets
+// come from two rounds of warp shuffles: one thread adding 1024 totals in turn was a third of what 1024 shots
+// from 26 qubits take beside reading the state (0.375 -> 0.316 ms with the indices' list made in one call).
 __global__ void __launch_bounds__(1024) k_scan_sums(const double* __restrict__ sums, ITYPE n, double* __restrict__ incl) {
-    __shared__ double part[1024];
+    __shared__ double part[32];
     const ITYPE per = (n + 1023) / 1024;
     const ITYPE lo = (ITYPE)threadIdx.x * per, hi = min(n, lo + per);
     double acc = 0.;
     for (ITYPE i = lo; i < hi; ++i) acc += sums[i];
-    part[threadIdx.x] = acc;
+    // exclusive offset of each thread: shuffles within a warp, then over the 32 warps' totals
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double incl_w = acc;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const double v = __shfl_up_sync(0xffffffffu, incl_w, d);
+        if (lane >= d) incl_w += v;
+    }
+    if (lane == 31) part[warp] = incl_w;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double run = 0.;
-        for (int t = 0; t < 1024; ++t) {
-            const double v = part[t];
-            part[t] = run;  // exclusive offset of thread t
-            run += v;
+    if (warp == 0) {
+        double t = part[lane];
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const double v = __shfl_up_sync(0xffffffffu, t, d);
+            if (lane >= d) t += v;
         }
+        part[lane] = t;
     }
     __syncthreads();
-    double run = part[threadIdx.x];
+    const double before = __shfl_up_sync(0xffffffffu, incl_w, 1);
+    double run = (warp ? part[warp - 1] : 0.) + (lane ? before : 0.);
     for (ITYPE i = lo; i < hi; ++i) {
         run += sums[i];
         incl[i] = run;
