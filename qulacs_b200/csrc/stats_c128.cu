@@ -283,6 +283,7 @@ template <class T>
 int ev_tiled(const PauliTerm* terms, const std::vector<int>& xidx, UINT n, const T* s, ITYPE dim, cudaStream_t st,
     double* values, std::vector<int>* rest, std::vector<int>* zidx);
 
+constexpr UINT kEvOneLaunchQubits = 12;    // whole Hamiltonians of states up to this size go out as one launch
 constexpr UINT kBatchEvSingleQubits = 18;  // states at least this large are evaluated by passes of their own
 // values[k] of the listed terms of one state, in one launch (one job per bit-flip string).
 template <class T>
@@ -2024,6 +2025,23 @@ int ev_weighted(const PauliTerm* terms, const double2* coefs, UINT count, const 
     constexpr bool c64 = sizeof(T) == sizeof(float2);
     bool imag = false;
     for (UINT k = 0; k < count; ++k) imag |= coefs[k].y != 0.;
+    // A small state's terms in one launch, one job per bit-flip string: they read it from the L2 cache, and a pass
+    // of the weighted kernel over one or two tiles is a chain of strings in one or two CTAs.  8, 32, 64 and 200
+    // strings in us, by passes and so: 11 qubits 61 78 127 210, 58 74 114 183; 12 qubits 53 74 119 217, 52 68 115
+    // 167; 13 qubits 52 76 118 204, 64 78 128 188; 15 qubits 52 74 130 216, 77 92 143 214.  (Forced modes keep the
+    // passes at every size.)
+    if (n <= kEvOneLaunchQubits && g_ev_spec_mode.load() == 1) {
+        std::vector<int> zidx, xidx;
+        for (UINT k = 0; k < count; ++k) (terms[k].x == 0 ? zidx : xidx).push_back((int)k);
+        std::vector<double> v(count);
+        QS_TRY(ev_listed<T>(terms, zidx, xidx, s, dim, st, v.data()));
+        out[0] = out[1] = 0.;
+        for (UINT k = 0; k < count; ++k) {
+            out[0] += coefs[k].x * v[k];
+            out[1] += coefs[k].y * v[k];
+        }
+        return QS_OK;
+    }
     std::shared_ptr<EwPlan> P = ew_plan(terms, count, n, c64, imag);
     double sr = 0., si = 0.;
     if (!P->passes.empty()) {
