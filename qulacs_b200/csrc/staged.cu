@@ -948,12 +948,19 @@ static bool want_specialized(const Circuit& c, ITYPE dim) {
     return dim >= (1ULL << kSpecializeMinQubits);
 }
 
+// Tile size of the generic kernel for a circuit alone.  From 13 to 18 qubits there are at most 64 tiles of 2^12
+// amplitudes for 148 SMs: 2^11 spreads each pass over twice the SMs, at about a third more passes.  U3 + CZ (20
+// layers), HEA (8), layered (10), in us: 16 qubits 215 144 197 against 247 189 214; 18 qubits 267 177 229
+// against 314 215 236.  Up to 12 qubits one tile of the whole state needs one pass (12: 119 72 140 against 127 114
+// 129), from 19 on there are tiles enough (19: 308 206 255 against 305 218 269; 21: 1118 652 952, 818 586 743).
+static int generic_tile_bits(UINT n) { return n >= 13 && n <= 18 ? kTileBits - 1 : kTileBits; }
+
 static int ensure_plan(Circuit& c, ITYPE dim) {
     if (c.plan && c.plan->dim == dim) return QS_OK;
     const bool spec = want_specialized(c, dim);
     std::shared_ptr<StagedPlan> P;
     std::vector<GateRec> g = rotation_form(c.gates, spec);
-    QS_TRY(build_plan(g, c.n, dim, &P, kTileBits, spec));
+    QS_TRY(build_plan(g, c.n, dim, &P, spec ? kTileBits : generic_tile_bits(c.n), spec));
     if (spec) QS_TRY(specialize_plan(*P));
     c.rgates.swap(g);
     c.plan = P;
