@@ -154,19 +154,25 @@ using cl = std::complex<long double>;
 static cl xmul(const cl& x, const cl& y) {
     return cl(x.real() * y.real() - x.imag() * y.imag(), x.real() * y.imag() + x.imag() * y.real());
 }
-static ld xabs(const cl& z) { return std::hypot(z.real(), z.imag()); }
+static ld xnorm(const cl& z) { return z.real() * z.real() + z.imag() * z.imag(); }
+static ld xabs(const cl& z) { return std::sqrt(xnorm(z)); }  // entries of unitaries: no overflow
+static cl xdiv(const cl& x, const cl& y) {  // |y| near 1
+    const ld n = xnorm(y);
+    const cl z = xmul(x, std::conj(y));
+    return cl(z.real() / n, z.imag() / n);
+}
 
 static bool is_unitary2(const cl* u) {
     const cl d = xmul(std::conj(u[0]), u[1]) + xmul(std::conj(u[2]), u[3]);
     constexpr ld tol = 1e-13L;
-    return std::abs(std::norm(u[0]) + std::norm(u[2]) - 1.L) <= tol &&
-           std::abs(std::norm(u[1]) + std::norm(u[3]) - 1.L) <= tol && xabs(d) <= tol;
+    return std::abs(xnorm(u[0]) + xnorm(u[2]) - 1.L) <= tol && std::abs(xnorm(u[1]) + xnorm(u[3]) - 1.L) <= tol &&
+           xnorm(d) <= tol * tol;
 }
 
 // U = diag(1, q1) [[c, -s], [s, c]] diag(p0, p1), c, s >= 0, unit p0, p1, q1, of a unitary U.  Phases are
 // quotients of entries (no angles), each taken where the entries are largest.
 static void zyz(const cl* u, ld* c, ld* s, cl* q1, cl* p0, cl* p1) {
-    const ld c0 = xabs(u[0]), c1 = xabs(u[3]), s0 = xabs(u[2]), s1 = xabs(u[1]), r = std::hypot(c0, s0);
+    const ld c0 = xabs(u[0]), c1 = xabs(u[3]), s0 = xabs(u[2]), s1 = xabs(u[1]), r = std::sqrt(c0 * c0 + s0 * s0);
     *c = c0 / r;
     *s = s0 / r;
     // e0, e1, f0, f1: phases of U00, U11, U10, -U01, with e0 e1 = f0 f1
@@ -187,7 +193,8 @@ static void zyz(const cl* u, ld* c, ld* s, cl* q1, cl* p0, cl* p1) {
 
 // A one-qubit gate's matrix in extended precision (rotations from their angle).
 static void xmatrix(const GateRec& g, cl* m) {
-    const ld c = std::cos((ld)g.angle / 2), s = std::sin((ld)g.angle / 2);
+    ld c = 1.L, s = 0.L;
+    if (g.kind == QS_GATE_RX || g.kind == QS_GATE_RY || g.kind == QS_GATE_RZ) sincosl((ld)g.angle / 2, &s, &c);
     switch (g.kind) {
         case QS_GATE_RX: m[0] = m[3] = c; m[1] = m[2] = cl(0.L, s); return;
         case QS_GATE_RY: m[0] = m[3] = c; m[1] = s; m[2] = -s; return;
@@ -222,6 +229,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         for (UINT q : g.qubits()) n = std::max(n, q + 1);
     std::vector<Qubit> Q(n);
     std::vector<GateRec> out;
+    out.reserve(2 * G.size() + 4);
     bool any_scalar = false;
     cl scalar = 1.L;
     auto diagonal = [&](UINT q, const cl& d0, const cl& d1, bool free_phase) {
@@ -242,7 +250,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         if (free_phase || d0 != cl(1.L)) any_scalar = true;
         scalar = xmul(scalar, d0);
         // an exact sign or identity stays one
-        k.d = xmul(k.d, d1 == d0 ? cl(1.L) : d1 == -d0 ? cl(-1.L) : d1 / d0);
+        k.d = xmul(k.d, d1 == d0 ? cl(1.L) : d1 == -d0 ? cl(-1.L) : xdiv(d1, d0));
     };
     auto flush = [&](UINT q) {  // the carried diagonal as a gate
         Qubit& k = Q[q];
@@ -292,7 +300,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
                 if (k.any) {  // X diag(1, d) = d diag(1, 1 / d) X
                     any_scalar = true;
                     scalar = xmul(scalar, k.d);
-                    k.d = k.d == cl(-1.L) ? k.d : cl(1.L) / k.d;
+                    k.d = k.d == cl(-1.L) ? k.d : xdiv(cl(1.L), k.d);
                 }
                 GateRec x;
                 x.kind = QS_GATE_DENSE;

@@ -40,26 +40,38 @@ struct Node {
 
 int par4(unsigned x) { return __builtin_popcount(x & 15u) & 1; }
 
-// X^v Z^f strings of a rotation: RY is Y = X^v Z^f, RX is X^v.
-bool commute(const Node& a, const Node& b) {
-    if (a.diag && b.diag) return true;
-    if (a.diag || b.diag) {
-        const Node& d = a.diag ? a : b;
-        const Node& o = a.diag ? b : a;
-        for (int i = 0; i < d.nf; ++i)
-            for (int k = 0; k < o.nv; ++k)
-                if (par4(d.g[i] & o.vs[k])) return false;
-        return true;
+// Sets of functionals (or of vectors) as bits of a 16-bit word: odd[v] holds the functionals that are 1 at v.
+struct Odd {
+    uint16_t at[16];
+    Odd() {
+        for (int v = 0; v < 16; ++v) {
+            at[v] = 0;
+            for (int f = 0; f < 16; ++f) at[v] |= (uint16_t)(par4(f & v) << f);
+        }
     }
-    if (a.rot && b.rot)  // two strings
-        return par4((a.ns ? a.fs[0] : 0) & b.vs[0]) == par4((b.ns ? b.fs[0] : 0) & a.vs[0]);
-    for (int i = 0; i < a.ns; ++i)
-        for (int k = 0; k < b.nv; ++k)
-            if (par4(a.fs[i] & b.vs[k])) return false;
-    for (int i = 0; i < b.ns; ++i)
-        for (int k = 0; k < a.nv; ++k)
-            if (par4(b.fs[i] & a.vs[k])) return false;
-    return true;
+};
+const Odd kOdd;
+
+// A node as the commutation test sees it: its functionals (a diagonal's, or a step's Z^f), and those that are 1
+// at one of its vectors (a step's X^v).
+struct Sets {
+    uint16_t f = 0, odd = 0;
+    bool diag = false, rot = false;
+    explicit Sets(const Node& n) : diag(n.diag), rot(n.rot) {
+        if (diag) {
+            for (int i = 0; i < n.nf; ++i) f |= (uint16_t)(1u << n.g[i]);
+            return;
+        }
+        for (int i = 0; i < n.ns; ++i) f |= (uint16_t)(1u << n.fs[i]);
+        for (int i = 0; i < n.nv; ++i) odd |= kOdd.at[n.vs[i]];
+    }
+};
+
+bool commute(const Sets& a, const Sets& b) {
+    if (a.diag && b.diag) return true;
+    const bool ab = a.f & b.odd, ba = b.f & a.odd;
+    if (a.rot && b.rot) return ab == ba;  // two strings X^v Z^f: RY is X^v Z^f, RX is X^v
+    return !ab && !ba;
 }
 
 struct PassScalar {
@@ -103,7 +115,7 @@ struct Builder {
         }
         if (ok) {  // the factor of bit value 0 joins the pass's scalar
             if (d0 != cl(1.)) scalar(d0, free);
-            const cl r = d1 == -d0 ? cl(-1.) : d0 == cl(1.) ? d1 : d1 / d0;
+            const cl r = d1 == -d0 ? cl(-1.) : d0 == cl(1.) ? d1 : mulc(d1, std::conj(d0)) / std::norm(d0);
             n.sign = !free && r == cl(-1.);
             n.hi = r;
         } else {  // projections and the like
@@ -220,10 +232,13 @@ struct Builder {
 
     void schedule(PhaseProgram* P) {
         const int N = (int)nodes.size();
+        std::vector<Sets> sets;
+        sets.reserve(N);
+        for (const Node& n : nodes) sets.emplace_back(n);
         std::vector<std::vector<int>> after(N);
         for (int j = 0; j < N; ++j)
             for (int i = 0; i < j; ++i)
-                if (!commute(nodes[i], nodes[j])) {
+                if (!commute(sets[i], sets[j])) {
                     after[i].push_back(j);
                     ++nodes[j].waits;
                 }
