@@ -19,6 +19,7 @@ from __future__ import annotations
 import argparse
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -573,21 +574,18 @@ def timed_region(step, steps: int, warmup: int, dist=None, sync=None, make_timer
     return ms
 
 
-def fp64_per_amplitude(qubits, m) -> int:
-    """FP64 instructions per amplitude of a gate in the staged register code: a rotation, or any 1-qubit
-    matrix whose entries are each real or imaginary, and a 1-qubit diagonal cost 4; a general 1-qubit
-    matrix 8; a k-qubit permutation or +-1 diagonal (CNOT, CZ, SWAP) 0; any other k-qubit matrix
-    4 x 2^k (2^k complex multiply-adds)."""
-    e = m.ravel()
-    if len(qubits) == 1:
-        if m[0, 1] == 0 and m[1, 0] == 0:
-            return 4
-        if all(x.real == 0 or x.imag == 0 for x in e):
-            return 4
-        return 8
-    if np.all((e == 0) | (e == 1) | (e == -1)):
-        return 0
-    return 4 * (1 << len(qubits))
+def fp64_per_amplitude(circ) -> float:
+    """FP64 instructions per amplitude of the circuit's staged schedule, counted from the generated pass
+    kernels: per 16-amplitude coset, 4 per diagonal factor or scaled rotation pair, 8 per unscaled one, 16 per
+    pair of a 2 x 2 matrix, 64 per quadruple of a 4 x 4 matrix, 2 per real scale."""
+    cost = {"cmul": 4, "ry_tan": 4, "ry_cot": 4, "rx_tan": 4, "rx_cot": 4, "ry_full": 8, "rx_full": 8,
+            "dense1": 16, "dense2": 64, "rscale": 2}
+    total = 0
+    for p in range(circ.pass_count()):
+        src = circ.specialized_source(p)
+        body = src[src.index("__launch_bounds__"):]
+        total += sum(c * len(re.findall(rf"\b{name}\(", body)) for name, c in cost.items())
+    return total / 16.0
 
 
 def serving_latency(requests: int, rate: float, budget_gb: float, workers: int, seed: int = 5005,
@@ -771,13 +769,10 @@ def main():
     per_launch_ms = ms / max(1, passes)
     hbm_peak, peak_kind = peaks()
     achieved = bytes_per_gate(n) / 1e9 / (per_launch_ms / 1e3)
-    # FP64 view of the same work: specialised RX/RY/RZ code issues 4 FP64 instructions per amplitude
-    # per rotation gate (CNOTs move data only); B200 FP64 CUDA-core peak = 148 SMs x 64 FMA/clk.
+    # FP64 view of the same work: the instructions of the generated pass kernels (unscaled rotations gate by
+    # gate: 4 per amplitude); B200 FP64 CUDA-core peak = 148 SMs x 64 FMA/clk.
     rot = sum(1 for g in gates if g[0] in ("RX", "RY", "RZ"))
-    fp64_instr = 4.0 * rot * (1 << n)
-    if fusion is not None and fusion["k"] > 0:
-        fl = circ.fuse(fusion["k"])
-        fp64_instr = float(sum(fp64_per_amplitude(*fl[i]) for i in range(len(fl)))) * (1 << n)
+    fp64_instr = (fp64_per_amplitude(circ) if staged_kernel and n >= 7 else 4.0 * rot) * (1 << n)
     fp64_peak = 148 * 64 * 1.965e9
     kernels = kernel_table(state, n, stream) if not args.no_kernel_table else None
 
@@ -897,8 +892,8 @@ def main():
             "roofline_fp64": {"achieved_tinstr_s": fp64_instr / (ms / 1e3) / 1e12,
                               "peak_tinstr_s": fp64_peak / 1e12,
                               "frac": fp64_instr / (ms / 1e3) / fp64_peak,
-                              "note": "FP64 instr/amplitude: rotation or 1q diagonal 4, 1q dense 8, k-qubit dense "
-                                      "4 x 2^k, CNOT/CZ/SWAP 0; nominal 64 FP64 FMA/clk/SM at 1965 MHz"},
+                              "note": "FP64 instructions of the generated pass kernels (scaled rotation 2 per "
+                                      "amplitude, collected diagonals up to 4); nominal 64 FP64 FMA/clk/SM at 1965 MHz"},
             "kernels": kernels,
             "e2e": {"value": world * len(gates) / (e2e_ms / 1e3), "unit": "gates/s", "ms_per_step": e2e_ms,
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
