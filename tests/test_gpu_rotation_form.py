@@ -1,4 +1,4 @@
-"""Specialised passes on circuits whose one-qubit gates sit at the edges of their rotation form: exact
+"""Specialised and generic passes on circuits whose one-qubit gates sit at the edges of their rotation form: exact
 signs, flips and identities, near-flips (cosine below 2^-20), zero angles, projections and other
 non-unitary matrices, runs of mixed gates, every tile size, and depolarizing channels at the ends of
 their range."""
@@ -7,7 +7,7 @@ import math
 import numpy as np
 import pytest
 
-from conftest import AMP_TOL, random_state, random_unitary
+from conftest import AMP_TOL, random_density_matrix, random_state, random_unitary
 from qulacs_b200 import DensityMatrix, QuantumCircuit, QuantumState, gate as G
 
 pytestmark = pytest.mark.gpu
@@ -25,12 +25,13 @@ def _one_qubit_gates(q, rng):
             G.DiagonalMatrix([q], [0.9j, -1.1])]
 
 
-@pytest.mark.parametrize("n", [7, 11, 12, 14])
+@pytest.mark.parametrize("n", [7, 11, 12, 14, 19])
 @pytest.mark.parametrize("mode", ["staged", "staged_fused"])
-def test_edge_gates_against_oracle(port, n, mode):
+@pytest.mark.parametrize("spec", [1, 0])
+def test_edge_gates_against_oracle(port, n, mode, spec):
     rng = np.random.default_rng(70 + n)
     c = QuantumCircuit(n)
-    c.set_specialized(1)
+    c.set_specialized(spec)
     if mode == "staged_fused":
         c.set_fusion(1)
     want = random_state(n, rng)
@@ -67,13 +68,14 @@ def test_edge_gates_against_oracle(port, n, mode):
     assert np.max(np.abs(s.get_vector() - want)) <= AMP_TOL * max(1.0, float(np.max(np.abs(want))))
 
 
-def test_long_runs_of_near_flips_keep_their_scale(port):
+@pytest.mark.parametrize("spec", [1, 0])
+def test_long_runs_of_near_flips_keep_their_scale(port, spec):
     """200 near-flips on the qubits of one tile: the cosines deferred over a pass (2^-19 each) exceed the
     bound on a deferred scale, so the later ones must not be deferred."""
     n = 12
     rng = np.random.default_rng(8)
     c = QuantumCircuit(n)
-    c.set_specialized(1)
+    c.set_specialized(spec)
     want = random_state(n, rng)
     s = QuantumState(n)
     s.load(want)
@@ -86,6 +88,35 @@ def test_long_runs_of_near_flips_keep_their_scale(port):
             port.CNOT_gate(0, n - 1, want)
     c.update_quantum_state(s)
     assert np.max(np.abs(s.get_vector() - want)) <= AMP_TOL
+
+
+def test_channels_of_a_small_density_matrix(port):
+    """5 qubits: the generic kernel's channel steps, channels merged past unitaries, against the oracle."""
+    n = 5
+    rng = np.random.default_rng(10)
+    c = QuantumCircuit(n)
+    rho = random_density_matrix(n, rng)
+    d = DensityMatrix(n)
+    d.load(rho)
+    want = rho.copy()
+    for _ in range(4):
+        for q in range(n):
+            g = G.RY(q, float(rng.uniform(0, 6)))
+            c.add_gate(g)
+            port.dm_single_qubit_dense_matrix_gate(q, g.get_matrix(), want)
+            c.add_gate(G.DepolarizingNoise(q, 0.1))
+            port.dm_depolarizing_noise(q, 0.1, want)
+            u = random_unitary(1, rng)
+            c.add_gate(G.DenseMatrix(q, u))
+            port.dm_single_qubit_dense_matrix_gate(q, u, want)
+        for a in range(n):
+            b, p = (a + 2) % n, float(rng.choice([0.02, 15 / 16, 1.0]))
+            c.add_gate(G.CZ(a, b) if a % 2 else G.CNOT(a, b))
+            (port.dm_CZ_gate if a % 2 else port.dm_CNOT_gate)(a, b, want)
+            c.add_gate(G.TwoQubitDepolarizingNoise(a, b, p))
+            port.dm_two_qubit_depolarizing_noise(a, b, p, want)
+    c.update_quantum_state(d, mode="staged")
+    assert np.max(np.abs(d.get_matrix() - want)) <= AMP_TOL
 
 
 @pytest.mark.parametrize("p1,p2", [(0.01, 0.02), (0.75, 15 / 16), (1.0, 1.0), (0.0, 0.9374)])
