@@ -549,6 +549,13 @@ QS_API int qs_debug_batch_wait_expiry(qs_circuit_t circuit, void* state, QS_UINT
  * pass waits on its own counter, bounded by wait_limit_us; returns QS_ERR_TIMEOUT, context usable. */
 QS_API int qs_debug_batch_wait_expiry_fused_c64(qs_circuit_t circuit, void* state_c64, QS_UINT wait_limit_us,
     void* stream);
+/* Check of the staged planner without a GPU (no reference counterpart): `circuit` on the HOST state vector
+ * state[2^n], or with density_matrix != 0 on the row-major host matrix state[2^n * 2^n], by the passes, phases
+ * and programs that the staged modes would run at block size k (0..6; 0 = no fusion) with tiles of
+ * 2^tile_bits amplitudes (4..12): the specialised kernels' (specialized != 0) or the generic kernels'.
+ * 4 to 20 qubits of the vector (density matrix: 2 to 10 qubits).  Host only. */
+QS_API int qs_debug_staged_replay(qs_circuit_t circuit, int density_matrix, int k, int specialized, QS_UINT tile_bits,
+    double* state, QS_ITYPE dim);
 /* The same on the fused complex64 tensor-core path: states_c64[i] holds circuits[i]'s 2^n complex64
  * amplitudes (n >= 10).  Missing plans are built on host threads in parallel; then every circuit's
  * passes run in ONE persistent launch (work items: tile pairs of (circuit, pass), a circuit's pass

@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "circuit.hpp"
+#include "host_plan.hpp"
 #include "qs_internal.cuh"
 #include "phase_program.hpp"
 #include "staged.hpp"
@@ -489,13 +490,6 @@ struct GateMask {
     bool stage;  // runs inside passes
 };
 
-struct PassPlan {
-    bool single = false;  // a gate run by the gate-by-gate kernels
-    int gate = -1;
-    std::vector<UINT> q;  // tile qubits (ascending)
-    std::vector<int> gates;
-};
-
 // Absorb greedily in program order with a fixed tile set; returns the absorbed gate indices.
 static void absorb(const std::vector<GateMask>& G, const std::vector<int>& pending, ITYPE Q, UINT n,
     std::vector<int>* got) {
@@ -646,25 +640,7 @@ static void lane_order(StPhase* P, int m) {
     for (int i = 0; i < 8; ++i) P->order[i] = i < k ? rest[i] : 0;
 }
 
-struct HostPlan {
-    std::vector<PassPlan> passes;
-    std::vector<StPhase> phases;
-    std::vector<StOp> ops;      // the phases' gates and their parameters
-    std::vector<double2> pool;
-    std::vector<PhaseProgram> programs;  // one per phase
-    std::vector<StStep> steps;  // the programs as the generic kernels read them
-    std::vector<double2> params;
-    struct Range {
-        size_t phase_begin, nphases;
-    };
-    std::vector<Range> pp;
-};
-
-// Host-only part of planning: passes, phases and their programs (no device calls).  The gates are in
-// rotation form.
-// `spec`: the passes will run specialised kernels.
-static void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits = kTileBits,
-    bool spec = false) {
+void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits, bool spec) {
     H->passes = plan_passes(gates, n, tile_bits);
     const std::vector<PassPlan>& passes = H->passes;
     std::vector<StPhase>& phases = H->phases;

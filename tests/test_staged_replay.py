@@ -1,0 +1,104 @@
+"""The staged planner without a GPU: random circuits through the passes, phases and programs of the staged modes,
+replayed on the host (qs_debug_staged_replay), against plain gate-by-gate application with the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import random_density_matrix, random_state, random_unitary
+from qulacs_b200 import QuantumCircuit
+from qulacs_b200 import gate as G
+from qulacs_b200._lib import call
+
+TOL = 1e-13  # a few hundred gates of rounding (2e-16 each) on normalised states
+
+
+def replay(circ, state, k=0, spec=True, tile_bits=12, dm=False):
+    out = np.ascontiguousarray(state, dtype=np.complex128).copy()
+    call("qs_debug_staged_replay", circ._h, int(dm), k, int(spec), tile_bits, out.ctypes.data_as(C.c_void_p),
+         1 << circ.qubit_count)
+    return out
+
+
+def apply_vector(port, gates, v):
+    """Each gate as a dense matrix over its qubits (controls expanded)."""
+    c = QuantumCircuit(int(np.log2(v.size)))
+    for g in gates:
+        c.add_gate(g)
+    flat = c.fuse(0)
+    for i in range(len(flat)):
+        qubits, m = flat[i]
+        port.multi_qubit_dense_matrix_gate(qubits, m, v)
+    return c
+
+
+def apply_matrix(port, gates, rho):
+    n = int(np.log2(rho.shape[0]))
+    c = QuantumCircuit(n)
+    for g in gates:
+        c.add_gate(g)
+    for g in gates:
+        t = g.get_target_index_list()
+        if g.kind == "DEPOLARIZING":
+            if len(t) == 1:
+                port.dm_depolarizing_noise(t[0], float(g.params[0]), rho)
+            else:
+                port.dm_two_qubit_depolarizing_noise(t[0], t[1], float(g.params[0]), rho)
+            continue
+        one = QuantumCircuit(n)
+        one.add_gate(g)
+        qubits, m = one.fuse(0)[0]
+        port.dm_multi_qubit_dense_matrix_gate(qubits, m, rho)
+    return c
+
+
+def random_gate(n, rng, unitary=True, channels=False):
+    q = int(rng.integers(n))
+    a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+    ang = float(rng.uniform(0, 6.3))
+    r = rng.random()
+    if channels and r < 0.3:
+        p = float(rng.choice([0.02, 0.3, 0.75, 1.0]))
+        return G.DepolarizingNoise(q, p) if rng.random() < 0.6 else G.TwoQubitDepolarizingNoise(a, b, p)
+    if not unitary and rng.random() < 0.25:
+        return [G.DiagonalMatrix([q], [1.0, 0.8]), G.DiagonalMatrix([q], [0.9j, -1.1]), G.P0(q),
+                G.DenseMatrix(q, np.array([[1.1, 0.2j], [0.3, 0.8 - 0.1j]])),
+                G.DenseMatrix(q, np.array([[0.0, 0.9], [-1.2j, 0.0]]))][int(rng.integers(5))]
+    kinds = [lambda: G.RX(q, ang), lambda: G.RY(q, ang), lambda: G.RZ(q, ang), lambda: G.H(q), lambda: G.X(q),
+             lambda: G.Y(q), lambda: G.Z(q), lambda: G.S(q), lambda: G.T(q), lambda: G.sqrtX(q),
+             lambda: G.U3(q, ang, 0.3, -ang), lambda: G.DenseMatrix(q, random_unitary(1, rng)),
+             lambda: G.CNOT(a, b), lambda: G.CNOT(a, b), lambda: G.CZ(a, b), lambda: G.SWAP(a, b),
+             lambda: G.DenseMatrix([a, b], random_unitary(2, rng)), lambda: G.PauliRotation([a, b], [1, 2], ang),
+             lambda: controlled(a, b, rng)]
+    return kinds[int(rng.integers(len(kinds)))]()
+
+
+def controlled(a, b, rng):
+    g = G.DenseMatrix(a, random_unitary(1, rng))
+    g.add_control_qubit(b, int(rng.integers(2)))
+    return g
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("k,tile_bits", [(0, 12), (0, 5), (1, 12), (2, 11)])
+def test_random_state_circuits(port, spec, k, tile_bits):
+    rng = np.random.default_rng(100 * k + tile_bits)
+    for trial in range(12):
+        n = 4 + trial % 4
+        v = random_state(n, rng)
+        want = v.copy()
+        c = apply_vector(port, [random_gate(n, rng, unitary=trial % 2 == 0) for _ in range(60)], want)
+        got = replay(c, v, k, spec, tile_bits)
+        assert np.max(np.abs(got - want)) <= TOL * max(1.0, float(np.max(np.abs(want))))
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("k,tile_bits", [(0, 12), (0, 5), (2, 11)])
+def test_random_noisy_matrix_circuits(port, spec, k, tile_bits):
+    rng = np.random.default_rng(200 * k + tile_bits)
+    for trial in range(8):
+        n = 2 + trial % 3
+        rho = random_density_matrix(n, rng)
+        want = rho.copy()
+        c = apply_matrix(port, [random_gate(n, rng, channels=True) for _ in range(60)], want)
+        assert np.max(np.abs(replay(c, rho, k, spec, tile_bits, dm=True) - want)) <= TOL
