@@ -162,6 +162,9 @@ static cl xdiv(const cl& x, const cl& y) {  // |y| near 1
     return cl(z.real() / n, z.imag() / n);
 }
 
+// Whether |z| is 1 up to the rounding of a few double-precision operations.
+static bool is_unit(const cl& z) { return std::abs(xnorm(z) - 1.L) <= 0x1p-49L; }
+
 static bool is_unitary2(const cl* u) {
     const cl d = xmul(std::conj(u[0]), u[1]) + xmul(std::conj(u[2]), u[3]);
     constexpr ld tol = 1e-13L;
@@ -209,8 +212,9 @@ static void xmatrix(const GateRec& g, cl* m) {
 // matrix in 8, and collect diagonals (phase_program.hpp).  So each run of one-qubit gates is multiplied
 // out and written D1 R D2: R is emitted as RY with its (cosine, sine), D2 as a diagonal before it, and D1 is
 // carried forward -- through controls, CZ and diagonals, which commute with it -- into the D2 of the next
-// run on the qubit.  Gates that do not commute with a carried diagonal (CNOT targets, dense blocks, ...)
-// get it just before them.  Phases common to a whole state are multiplied up and emitted once at the end.
+// run on the qubit.  Only unitary diagonals are carried: a depolarizing channel does not commute with others,
+// and their products have no bound.  Gates that do not commute with a carried diagonal (CNOT targets, dense
+// blocks, ...) get it just before them.  Phases common to a whole state are multiplied up and emitted once at the end.
 std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
     // A qubit's run of gates not emitted yet is diag(1, d), then a core, then diag(p0, p1).  The core is kept
     // as a rotation while it is one: which factors a run gets must not depend on the signs of its angles.
@@ -219,10 +223,10 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         Core core = NONE;
         ld c = 1.L, s = 0.L;  // REAL: {c, s; -s, c}; RX: {c, i s; i s, c}
         cl m[4];              // MATRIX
-        bool post = false, post_free = false;
+        bool post = false, post_free = false, post_unit = true;
         cl p0 = 1.L, p1 = 1.L;
         bool any = false, any_free = false;
-        cl d = 1.L;           // carried
+        cl d = 1.L;           // carried; a product of quotients of unit entries
     };
     UINT n = 0;
     for (const GateRec& g : G)
@@ -267,7 +271,6 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         r.xs = s;
         out.push_back(r);
     };
-    auto fair = [](const cl& z) { return std::norm(z) > 0.25L && std::norm(z) < 4.L; };
     auto core_matrix = [](const Qubit& k, cl* m) {
         if (k.core == MATRIX) std::copy(k.m, k.m + 4, m);
         else if (k.core == REAL) m[0] = m[3] = k.c, m[1] = k.s, m[2] = -k.s;
@@ -276,11 +279,12 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
     };
     auto end_run = [&](UINT q) {  // emits the run's core; what may be carried further stays carried
         Qubit& k = Q[q];
-        const bool post = k.post, post_free = k.post_free;
+        const bool post = k.post, post_free = k.post_free, post_unit = k.post_unit;
         const cl p0 = k.p0, p1 = k.p1;
         Core core = k.core;
         k.core = NONE;
         k.post = k.post_free = false;
+        k.post_unit = true;
         k.p0 = k.p1 = 1.L;
         const cl zero(0.L);
         if (core == RX && (k.any || !spec)) {
@@ -296,7 +300,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         } else if (core == RX) {
             rotation(q, QS_GATE_RX, k.c, k.s);
         } else if (core == MATRIX) {
-            if (u[0] == zero && u[3] == zero && fair(u[1]) && fair(u[2])) {  // diag(u1, u2) X
+            if (u[0] == zero && u[3] == zero) {  // diag(u1, u2) X
                 if (k.any) {  // X diag(1, d) = d diag(1, 1 / d) X
                     any_scalar = true;
                     scalar = xmul(scalar, k.d);
@@ -307,7 +311,8 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
                 x.targets = {q};
                 x.matrix = {0., 1., 1., 0.};
                 out.push_back(x);
-                carry(q, u[1], u[2], false);
+                if (is_unit(u[1]) && is_unit(u[2])) carry(q, u[1], u[2], false);
+                else diagonal(q, u[1], u[2], false);
             } else if (is_unitary2(u)) {
                 ld c, s;
                 cl q1, e0, e1;
@@ -326,8 +331,8 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
             }
         }
         if (post) {
-            if (fair(p0) && fair(p1)) carry(q, p0, p1, post_free);
-            else diagonal(q, p0, p1, false);  // a projection; commutes with the carried diagonal
+            if (post_unit) carry(q, p0, p1, post_free);
+            else diagonal(q, p0, p1, false);  // commutes with the carried diagonal
         }
     };
     auto add_matrix = [&](UINT q, int kind, const cl* m) {
@@ -337,6 +342,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
             k.p0 = xmul(m[0], k.p0);
             k.p1 = xmul(m[3], k.p1);
             k.post = true;
+            k.post_unit = k.post_unit && is_unit(m[0]) && is_unit(m[3]);
             k.post_free = k.post_free || kind == QS_GATE_RZ;
             if (k.core == NONE) end_run(q);
             return;
@@ -376,6 +382,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
             for (int x = 0; x < 2; ++x) k.m[y * 2 + x] = xmul(m[y * 2], a[x]) + xmul(m[y * 2 + 1], a[2 + x]);
         k.core = MATRIX;
         k.post = k.post_free = false;
+        k.post_unit = true;
         k.p0 = k.p1 = 1.L;
     };
     const ld h = std::sqrt(0.5L);
@@ -412,7 +419,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
             }
             default:
                 if (g.depol == 1) {
-                    // a channel commutes with U on the row bit and conj(U) on the column bit together
+                    // a channel commutes with a unitary U on the row bit and conj(U) on the column bit together
                     const Qubit &c = Q[g.targets[0]], &r = Q[g.targets[1]];
                     if (c.any && r.any && c.d == std::conj(r.d)) break;
                 }

@@ -148,3 +148,31 @@ def test_channels_against_gate_by_gate(mode, p1, p2):
     c.update_quantum_state(a, mode=mode)
     c.update_quantum_state(b, mode="gate_by_gate")
     assert np.max(np.abs(a.get_matrix() - b.get_matrix())) <= AMP_TOL
+
+
+@pytest.mark.parametrize("n", [5, 11])
+@pytest.mark.parametrize("mode", ["staged", "staged_fused"])
+def test_channels_after_non_unitary_diagonals(n, mode):
+    """Diagonals that are not unitary before channels, in the generic (5 qubits) and the specialised kernels (11)."""
+    rng = np.random.default_rng(12)
+    c = QuantumCircuit(n)
+    for q in range(n):
+        c.add_gate(G.RY(q, float(rng.uniform(0, 6))))
+        c.add_gate(G.DiagonalMatrix([q], [1.0, 0.8] if q % 2 else [0.9j, -1.1]))
+        c.add_gate(G.DepolarizingNoise(q, 0.3))
+    for q in range(n - 1):
+        c.add_gate(G.CNOT(q, q + 1))
+        c.add_gate(G.DiagonalMatrix([q], [0.8, 1.2]))
+        c.add_gate(G.TwoQubitDepolarizingNoise(q, q + 1, 0.1))
+        c.add_gate(G.DepolarizingNoise(q, 0.1))
+    if mode == "staged_fused":
+        c.set_fusion(1)
+    psi = QuantumState(n)
+    psi.set_Haar_random_state(5)
+    a, b = DensityMatrix(n), DensityMatrix(n)
+    a.load(psi)
+    b.load(psi)
+    c.update_quantum_state(a, mode=mode)
+    c.update_quantum_state(b, mode="gate_by_gate")
+    want = b.get_matrix()
+    assert np.max(np.abs(a.get_matrix() - want)) <= AMP_TOL * max(1.0, float(np.max(np.abs(want))))

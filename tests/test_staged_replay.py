@@ -102,3 +102,30 @@ def test_random_noisy_matrix_circuits(port, spec, k, tile_bits):
         want = rho.copy()
         c = apply_matrix(port, [random_gate(n, rng, channels=True) for _ in range(60)], want)
         assert np.max(np.abs(replay(c, rho, k, spec, tile_bits, dm=True) - want)) <= TOL
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("d", [[1.0, 0.8], [0.9j, -1.1], [0.6, 0.6], [1.0, 1.0 + 2.0 ** -30]])
+def test_channels_after_non_unitary_diagonals(port, d, spec):
+    """A depolarizing channel commutes with unitary diagonals only: one whose entries are not of modulus 1 is
+    applied before the channel that follows it."""
+    gates = [G.RY(0, 1.0), G.DiagonalMatrix([0], d), G.DepolarizingNoise(0, 0.3), G.RY(1, 0.4), G.RZ(0, 0.5),
+             G.DiagonalMatrix([1], d), G.H(1), G.RX(1, 0.3), G.DiagonalMatrix([1], d), G.DepolarizingNoise(1, 0.1),
+             G.TwoQubitDepolarizingNoise(0, 1, 0.2)]
+    rng = np.random.default_rng(3)
+    rho = random_density_matrix(2, rng)
+    want = rho.copy()
+    c = apply_matrix(port, gates, want)
+    assert np.max(np.abs(replay(c, rho, spec=spec, dm=True) - want)) <= TOL
+
+
+@pytest.mark.parametrize("spec", [True, False])
+def test_random_noisy_matrix_circuits_with_non_unitary_gates(port, spec):
+    rng = np.random.default_rng(17)
+    for trial in range(60):
+        n = 2 + trial % 3
+        rho = random_density_matrix(n, rng)
+        want = rho.copy()
+        c = apply_matrix(port, [random_gate(n, rng, unitary=False, channels=True) for _ in range(30)], want)
+        got = replay(c, rho, trial % 3, spec, dm=True)
+        assert np.max(np.abs(got - want)) <= TOL * max(1.0, float(np.max(np.abs(want))))
