@@ -178,7 +178,7 @@ __device__ __forceinline__ void dense2(D2& a, D2& b, D2& c, D2& d, const D2* p) 
     d = row4(p + 12, a, b, c, d);
     a = A; b = B; c = C;
 }
-// One-qubit depolarizing channel, scaled by 1 / (1 - q / 2): populations (x, y) mix, coherences shrink.
+// Populations (x, y) of a one-qubit depolarizing channel mix.
 __device__ __forceinline__ void mix2(D2& x, D2& y, double t) {
     const D2 X = x;
     x = mk(fma(t, y.x, X.x), fma(t, y.y, X.y));
@@ -310,10 +310,12 @@ void emit_step(std::ostringstream& o, const ProgStep& s, ParamSink& ps) {
             break;
         }
         case SP_DEPOL1: {  // qubits: column, row
-            const std::string t = ps.d1(s.par[0].x), k = ps.d1(s.par[0].y);
-            for (int j : bases())
+            const std::string t = ps.d1(s.par[0].x), k = ps.d1(s.par[0].y), d = s.form ? ps.d1(s.par[1].x) : std::string();
+            for (int j : bases()) {
+                if (s.form) o << "      rscale(" << reg(j) << ", " << d << "); rscale(" << reg(coset(j, 3)) << ", " << d << ");\n";
                 o << "      mix2(" << reg(j) << ", " << reg(coset(j, 3)) << ", " << t << "); rscale(" << reg(coset(j, 1))
                   << ", " << k << "); rscale(" << reg(coset(j, 2)) << ", " << k << ");\n";
+            }
             break;
         }
         case SP_DEPOL2: {  // qubits: columns 0, 1, rows 0, 1; populations: equal column and row

@@ -106,19 +106,19 @@ struct Builder {
         n.diag = true;
         n.nf = 1;
         n.g[0] = F[b];
-        const double m0 = (double)std::norm(d0), m1 = (double)std::norm(d1);
-        const bool ok = m0 > 0.25 && m0 < 4. && m1 > 0.25 && m1 < 4.;
         n.free = free;
+        // the factor of bit value 0 joins the pass's scalar if it is 1 in modulus (others have no bound)
+        const bool ok = free || std::abs(std::norm(d0) - 1.L) <= 0x1p-49L;
         if (d0 == d1 && ok && (!free || d0 != cl(1.))) {  // a scalar
             if (d0 != cl(1.)) scalar(d0, free);
             return;
         }
-        if (ok) {  // the factor of bit value 0 joins the pass's scalar
+        if (ok) {
             if (d0 != cl(1.)) scalar(d0, free);
             const cl r = d1 == -d0 ? cl(-1.) : d0 == cl(1.) ? d1 : mulc(d1, std::conj(d0)) / std::norm(d0);
             n.sign = !free && r == cl(-1.);
             n.hi = r;
-        } else {  // projections and the like
+        } else {
             n.lo = d0;
             n.hi = d1;
         }
@@ -214,18 +214,19 @@ struct Builder {
         Node n;
         n.step.kind = k == 1 ? SP_DEPOL1 : SP_DEPOL2;
         for (int i = 0; i < 2 * k; ++i) set_qubit(n, i, bits[i]);
-        if (k == 1) {
-            const ld d = 1.L - q / 2;
-            n.step.par.push_back(make_double2((double)(q / 2 / d), (double)((1.L - q) / d)));
+        const ld d = k == 1 ? 1.L - q / 2 : 1.L - q;  // what the scaled form leaves out
+        const double grow = -std::log2(std::max((double)std::abs(d), 1e-300));
+        const bool scaled = grow <= 10. && S.bits + grow <= kMaxDeferredBits;  // one qubit: d >= 1/3
+        if (scaled) {
             scalar(d);
-            S.bits -= (double)std::log2(d);  // d >= 1/3
-        } else if (std::abs(1.L - q) > 0.001L) {
-            n.step.par.push_back(make_double2((double)(q / 4 / (1.L - q)), 0.));
-            scalar(1.L - q);
-            S.bits -= (double)std::log2(std::abs(1.L - q));
+            S.bits += grow;
+        }
+        n.step.form = !scaled;
+        if (k == 1) {
+            n.step.par.push_back(make_double2((double)(q / 2 / d), (double)((1.L - q) / (scaled ? d : 1.L))));
+            if (!scaled) n.step.par.push_back(make_double2((double)d, 0.));
         } else {
-            n.step.form = 1;
-            n.step.par.push_back(make_double2((double)(q / 4), (double)(1.L - q)));
+            n.step.par.push_back(scaled ? make_double2((double)(q / 4 / d), 0.) : make_double2((double)(q / 4), (double)d));
         }
         push(std::move(n));
     }
@@ -454,7 +455,10 @@ void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vect
             case SP_X: t.code = (uint8_t)(16 + a * 5); break;
             case SP_SWAP: t.code = (uint8_t)(32 + std::min(a, b) * 4 + std::max(a, b)); break;
             case SP_DENSE1: t.code = (uint8_t)(32 + a * 5); break;
-            case SP_DEPOL1: t.code = (uint8_t)(32 + std::max(a, b) * 4 + std::min(a, b)); break;
+            case SP_DEPOL1:
+                t.code = (uint8_t)(32 + std::max(a, b) * 4 + std::min(a, b));
+                t.mask = s.form;
+                break;
             case SP_DENSE2: t.code = (uint8_t)(48 + a * 4 + b); break;
             case SP_DEPOL2: {  // by the partner of register bit 0: 1, 2 or 3
                 const int c = bit(s.v[2]), d = bit(s.v[3]);

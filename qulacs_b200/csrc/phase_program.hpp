@@ -33,7 +33,7 @@ enum RotForm : uint8_t { RF_Y_TAN, RF_Y_COT, RF_Y_FULL, RF_X_TAN, RF_X_COT, RF_X
 // parity(f[i] & j) ^ a[i].
 struct ProgStep {
     StepKind kind = SP_DIAG;
-    uint8_t form = 0;       // SP_ROT: RotForm; SP_DEPOL2: 0 scaled, 1 full
+    uint8_t form = 0;       // SP_ROT: RotForm; SP_DEPOL1, SP_DEPOL2: 0 scaled, 1 full; SP_SCALE: 1 complex
     uint8_t nq = 0;
     uint8_t v[4] = {}, f[4] = {}, a[4] = {};
     uint16_t mask = 0;      // SP_DIAG: registers with a factor; SP_SIGN: registers negated

@@ -182,9 +182,16 @@ __device__ __forceinline__ void r_swap(double2 (&r)[16]) {
             r[k] = t;
         }
 }
-// One-qubit depolarizing channel, scaled (column and row bit A, B): populations mix, coherences shrink.
+// One-qubit depolarizing channel (column and row bit A, B): populations mix, coherences shrink.  `full` (the
+// channel itself, not scaled): the factor by which the populations shrink first.
 template <int A, int B>
-__device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k) {
+__device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k, const double2* __restrict__ full) {
+    if (full) {
+        const double d = full->x;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (!(j & (1 << A)) == !(j & (1 << B))) r[j] = make_double2(d * r[j].x, d * r[j].y);
+    }
 #pragma unroll
     for (int j = 0; j < 16; ++j)
         if (!(j & (1 << A)) && !(j & (1 << B))) {
@@ -231,7 +238,7 @@ __device__ __forceinline__ void run_step(double2 (&r)[16], const double2* __rest
     else if constexpr (kind == 1) r_x<A>(r);
     else if constexpr (kind == 2 && A < B) r_swap<A, B>(r);
     else if constexpr (kind == 2 && A == B) r_dense1<A>(r, p);
-    else if constexpr (kind == 2) r_depol1<A, B>(r, p[0].x, p[0].y);
+    else if constexpr (kind == 2) r_depol1<A, B>(r, p[0].x, p[0].y, mask ? p + 1 : nullptr);
     else if constexpr (kind == 3 && A != B) r_dense2<A, B>(r, p);
     else if constexpr (kind == 3 && A < 3) r_depol2<A + 1>(r, p[0].x, p[0].y, mask != 0);
     else if constexpr (kind == 4 && V) r_ry_tan<V>(r, p[0].x, mask);

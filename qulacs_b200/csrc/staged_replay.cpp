@@ -54,7 +54,11 @@ void dense(cd* r, const int* idx, int k, const double2* m) {
     }
     for (int y = 0; y < k; ++y) r[idx[y]] = o[y];
 }
-void channel1(cd& x, cd& y, cd& a, cd& b, double t, double k) {
+void channel1(cd& x, cd& y, cd& a, cd& b, double t, double k, const double2* full) {
+    if (full) {
+        x *= full->x;
+        y *= full->x;
+    }
     const cd X = x;
     x = axpy(t, y, X);
     y = axpy(t, X, y);
@@ -101,7 +105,7 @@ void run_spec(const ProgStep& s, cd* r) {
             }
             case SP_DENSE1: dense(r, o, 2, s.par.data()); break;
             case SP_DENSE2: dense(r, o, 4, s.par.data()); break;
-            case SP_DEPOL1: channel1(r[j], r[o[3]], r[o[1]], r[o[2]], s.par[0].x, s.par[0].y); break;
+            case SP_DEPOL1: channel1(r[j], r[o[3]], r[o[1]], r[o[2]], s.par[0].x, s.par[0].y, s.form ? &s.par[1] : nullptr); break;
             case SP_DEPOL2: {
                 const int pop[4] = {j, coset(j, 5), coset(j, 10), coset(j, 15)};
                 channel2(r, pop, s.par[0].x, s.form ? s.par[0].y : 1., s.form != 0);
@@ -133,7 +137,7 @@ void run_code(const StStep& s, const double2* p, cd* r) {
         } else if (kind == 2 && A == B) {
             if (base1) dense(r, o, 2, p);
         } else if (kind == 2) {
-            if (base2) channel1(r[j], r[o[3]], r[o[1]], r[o[2]], p[0].x, p[0].y);
+            if (base2) channel1(r[j], r[o[3]], r[o[1]], r[o[2]], p[0].x, p[0].y, s.mask ? p + 1 : nullptr);
         } else if (kind == 3 && A != B) {
             if (base2) dense(r, o, 4, p);
         } else if (kind == 3) {

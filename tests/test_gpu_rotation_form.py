@@ -176,3 +176,25 @@ def test_channels_after_non_unitary_diagonals(n, mode):
     c.update_quantum_state(b, mode="gate_by_gate")
     want = b.get_matrix()
     assert np.max(np.abs(a.get_matrix() - want)) <= AMP_TOL * max(1.0, float(np.max(np.abs(want))))
+
+
+@pytest.mark.parametrize("n", [2, 5, 11])
+def test_hundreds_of_channels_in_one_pass(n):
+    """Channels whose deferred scales exceed the bound of a pass run unscaled, in the generic and the specialised
+    (11 qubits) kernels."""
+    c = QuantumCircuit(n)
+    for i in range(300):
+        c.add_gate(G.DepolarizingNoise(0, 1.0))
+        c.add_gate(G.RY(0, 0.1 * i))
+        c.add_gate(G.CZ(0, 1))
+        if i % 3 == 0:
+            c.add_gate(G.TwoQubitDepolarizingNoise(0, 1, 0.9))
+    psi = QuantumState(n)
+    psi.set_Haar_random_state(6)
+    a, b = DensityMatrix(n), DensityMatrix(n)
+    a.load(psi)
+    b.load(psi)
+    c.update_quantum_state(a, mode="staged")
+    c.update_quantum_state(b, mode="gate_by_gate")
+    got = a.get_matrix()
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got - b.get_matrix())) <= AMP_TOL

@@ -129,3 +129,37 @@ def test_random_noisy_matrix_circuits_with_non_unitary_gates(port, spec):
         c = apply_matrix(port, [random_gate(n, rng, unitary=False, channels=True) for _ in range(30)], want)
         got = replay(c, rho, trial % 3, spec, dm=True)
         assert np.max(np.abs(got - want)) <= TOL * max(1.0, float(np.max(np.abs(want))))
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("p,two", [(0.5, False), (1.0, False), (0.1, True), (0.9, True), (1.0, True), (15 / 16, True)])
+def test_thousands_of_channels_in_one_pass(port, p, two, spec):
+    """The scales that channels defer over a pass are bounded: 2000 of them on one tile."""
+    gates = []
+    for i in range(1000):
+        gates.append(G.TwoQubitDepolarizingNoise(0, 1, p) if two else G.DepolarizingNoise(i % 2, p))
+        gates.append(G.U3(i % 2, 0.7, 0.1 * (i % 50), 0.4))
+        gates.append(G.CZ(0, 1) if i % 3 else G.TwoQubitDepolarizingNoise(1, 0, p))
+    rng = np.random.default_rng(3)
+    rho = random_density_matrix(2, rng)
+    want = rho.copy()
+    c = apply_matrix(port, gates, want)
+    got = replay(c, rho, spec=spec, dm=True)
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got - want)) <= 10 * TOL
+
+
+@pytest.mark.parametrize("spec", [True, False])
+def test_long_products_of_non_unitary_diagonals_in_one_pass(port, spec):
+    """Non-unitary diagonals that shrink the state by 2^-650 over a pass, beside rotations that defer 2^400: the
+    result keeps its precision."""
+    n = 4
+    gates = []
+    for i in range(750):
+        gates += [G.DiagonalMatrix([i % n], [0.55, 0.52]), G.RY(i % n, 2.5), G.CNOT(i % n, (i + 1) % n)]
+    rng = np.random.default_rng(4)
+    v = random_state(n, rng)
+    want = v.copy()
+    c = apply_vector(port, gates, want)
+    got = replay(c, v, spec=spec)
+    assert 0 < np.max(np.abs(want)) < 1e-180
+    assert np.max(np.abs(got - want)) <= 10 * TOL * float(np.max(np.abs(want)))
