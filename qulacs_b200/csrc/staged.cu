@@ -615,6 +615,7 @@ struct StagedPlan {
     // host copies of the schedule (for specialised pass kernels)
     std::vector<StPhase> phases;
     std::vector<PhaseProgram> programs;
+    bool generic = true;       // the generic kernels' programs are on the device
     bool specialized = false;  // every pass has its specialised kernel
     double compile_ms = 0.;    // wall time of compiling them
     ~StagedPlan() {
@@ -805,12 +806,13 @@ static int build_plan(const std::vector<GateRec>& gates, UINT n, ITYPE dim, std:
     return upload_plan(H, dim, out);
 }
 
-// Device copy of a host plan (phases | ops | parameter pool in one allocation) and its launch args.
+// Device copy of a host plan (phases | steps | parameters in one allocation) and its launch args.
 static int upload_plan(const HostPlan& H, ITYPE dim, std::shared_ptr<StagedPlan>* out) {
     auto P = std::make_shared<StagedPlan>();
     P->dim = dim;
     P->phases = H.phases;
     P->programs = H.programs;
+    P->generic = H.programs.empty();
     const std::vector<PassPlan>& passes = H.passes;
     const std::vector<StPhase>& phases = H.phases;
     const std::vector<HostPlan::Range>& pp = H.pp;
@@ -869,6 +871,7 @@ static int run_plan(const std::vector<GateRec>& gates, const StagedPlan& P, void
                 tiles, d.args.m, st));
             continue;
         }
+        if (!P.generic) return set_error(QS_ERR_CUDA, "staged schedule without its specialised kernels");
         launch_pass((double2*)state, d, tiles, st);
         QS_TRY(check_launch("k_staged_pass"));
     }
@@ -888,7 +891,7 @@ static PassDesc pass_desc(const StagedPlan& P, const DevPass& d) {
 }
 
 // Specialised kernels for every pass of a plan, compiled on host threads in parallel.  On failure the
-// plan keeps the generic pass kernel for every pass and the error is returned.
+// error is returned and the plan cannot run: it holds no programs for the generic kernel.
 static int specialize_plan(StagedPlan& P) {
     if (P.specialized) return QS_OK;
     std::vector<size_t> todo;
@@ -1058,39 +1061,46 @@ static int estimate_plan_ms(const std::vector<GateRec>& gates, const StagedPlan&
 static int ensure_fused_plan(Circuit& c, ITYPE dim, cudaStream_t st) {
     if (c.fplan && c.fplan->dim == dim) return QS_OK;
     const bool spec = want_specialized(c, dim);
-    if (c.fusion_k >= 0) {
-        c.fgates = executor_gates(c.gates, c.fusion_k, spec, &c.fused_count);
-        c.fused_k = c.fusion_k;
-        c.fused_tile_bits = kTileBits;
-        std::shared_ptr<StagedPlan> P;
-        QS_TRY(build_plan(c.fgates, c.n, dim, &P, kTileBits, spec));
-        if (spec) QS_TRY(specialize_plan(*P));
-        c.fplan = P;
-        return QS_OK;
-    }
-    c.tune_ms.assign(kTuneSlots, -1.);
-    double best = 0.;
-    auto consider = [&](int k, int tile_bits, int slot) -> int {
+    // the circuit gets a schedule once it can run: a failing candidate leaves none behind
+    struct Candidate {
+        std::vector<GateRec> gates;
         size_t count = 0;
-        std::vector<GateRec> fg = executor_gates(c.gates, k, spec, &count);
-        std::shared_ptr<StagedPlan> P;
-        QS_TRY(build_plan(fg, c.n, dim, &P, tile_bits, spec));
-        double ms = 0.;
-        QS_TRY(estimate_plan_ms(fg, *P, dim, st, spec, &ms));
-        c.tune_ms[slot] = ms;
-        if (!c.fplan || ms < best) {
-            best = ms;
-            c.fgates.swap(fg);
-            c.fused_count = count;
-            c.fplan = P;
-            c.fused_k = k;
-            c.fused_tile_bits = tile_bits;
-        }
-        return QS_OK;
+        std::shared_ptr<StagedPlan> plan;
+        int k = -1, tile_bits = kTileBits;
     };
-    for (int k = 0; k <= kTuneMaxK; ++k) QS_TRY(consider(k, kTileBits, k));
-    if (c.n > (UINT)kTileBits - 1) QS_TRY(consider(c.fused_k, kTileBits - 1, kTuneMaxK + 1));
-    if (spec) QS_TRY(specialize_plan(*c.fplan));
+    auto make = [&](int k, int tile_bits, Candidate* F) -> int {
+        F->k = k;
+        F->tile_bits = tile_bits;
+        F->gates = executor_gates(c.gates, k, spec, &F->count);
+        return build_plan(F->gates, c.n, dim, &F->plan, tile_bits, spec);
+    };
+    Candidate chosen;
+    std::vector<double> ms;
+    if (c.fusion_k >= 0) {
+        QS_TRY(make(c.fusion_k, kTileBits, &chosen));
+    } else {
+        ms.assign(kTuneSlots, -1.);
+        double best = 0.;
+        auto consider = [&](int k, int tile_bits, int slot) -> int {
+            Candidate F;
+            QS_TRY(make(k, tile_bits, &F));
+            QS_TRY(estimate_plan_ms(F.gates, *F.plan, dim, st, spec, &ms[slot]));
+            if (!chosen.plan || ms[slot] < best) {
+                best = ms[slot];
+                chosen = std::move(F);
+            }
+            return QS_OK;
+        };
+        for (int k = 0; k <= kTuneMaxK; ++k) QS_TRY(consider(k, kTileBits, k));
+        if (c.n > (UINT)kTileBits - 1) QS_TRY(consider(chosen.k, kTileBits - 1, kTuneMaxK + 1));
+    }
+    if (spec) QS_TRY(specialize_plan(*chosen.plan));
+    c.tune_ms.swap(ms);
+    c.fgates.swap(chosen.gates);
+    c.fused_count = chosen.count;
+    c.fused_k = chosen.k;
+    c.fused_tile_bits = chosen.tile_bits;
+    c.fplan = chosen.plan;
     return QS_OK;
 }
 

@@ -198,3 +198,28 @@ def test_hundreds_of_channels_in_one_pass(n):
     c.update_quantum_state(b, mode="gate_by_gate")
     got = a.get_matrix()
     assert np.all(np.isfinite(got)) and np.max(np.abs(got - b.get_matrix())) <= AMP_TOL
+
+
+def test_failed_fused_planning_leaves_no_schedule():
+    """A block size whose kernels cannot be compiled (a NaN among parameters that are too many for a parameter
+    block) fails the call; the next call must not find a half-built schedule."""
+    n = 12
+    rng = np.random.default_rng(2)
+    c = QuantumCircuit(n)
+    c.set_specialized(1)
+    c.add_gate(G.DenseMatrix(0, np.full((2, 2), np.nan)))
+    for layer in range(22):  # k = 2: 132 blocks with a 4 x 4 matrix each; k = 0, 1: one angle per gate
+        for a in range(layer % 2, n, 2):
+            b = (a + 1) % n
+            for _ in range(3):
+                c.add_gate(G.RY(a, float(rng.uniform(0.1, 0.5))))
+                c.add_gate(G.RY(b, float(rng.uniform(0.1, 0.5))))
+                c.add_gate(G.CNOT(a, b))
+    s = QuantumState(n)
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="NVRTC compile failed"):
+            c.update_quantum_state(s, mode="staged_fused")
+        assert c.fusion_info()[0] == -1
+    c.set_fusion(0)
+    c.update_quantum_state(s, mode="staged_fused")
+    assert c.fusion_info()[0] == 0
