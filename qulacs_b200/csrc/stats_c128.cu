@@ -985,6 +985,7 @@ struct EvJobs {
     }
     // values[0 .. nvals): one upload, the jobs, their folds, one copy back
     int run(UINT nvals, cudaStream_t st, double* values) const {
+        if (jobs.empty()) return QS_OK;  // a launch of no blocks is an error
         auto up = [](size_t b) { return (b + 255) / 256 * 256; };
         const size_t bj = up(sizeof(EvJob) * jobs.size()), bz = up(sizeof(ITYPE) * (zm.size() + 1)),
                      bo = up(sizeof(UINT) * (zout.size() + 1)), bp = up(sizeof(double) * kEvZ * total);
@@ -1097,7 +1098,6 @@ static int batch_ev_impl(void* const* states, const QS_UINT* qubit_counts, QS_UI
         }
         if (nz) W.z_only(states[i], c64, dim, zmask, zidx, nz);
     }
-    if (W.jobs.empty()) return QS_OK;
     // only the entries of the states evaluated here (large states' values are already in `values`)
     std::vector<double> hv(nterms);
     QS_TRY(W.run(nterms, st, hv.data()));

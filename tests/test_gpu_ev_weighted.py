@@ -181,3 +181,17 @@ def test_small_state_strings_in_one_launch(port, n, terms, c64):
     want = np.array([port.expectation_value(tl, ids, v) for _, tl, ids in ts])
     assert np.max(np.abs(obs.term_values(s) - want)) <= EV_TOL
     assert abs(obs.get_expectation_value(s) - float(np.dot([t[0] for t in ts], want))) <= EV_TOL * len(ts)
+
+
+@pytest.mark.parametrize("n", [1, 5, 12, 14])
+@pytest.mark.parametrize("c64", [False, True])
+def test_empty_sum_is_zero(lib, n, c64):
+    """No terms at all, through the C entry points: 0, at every size."""
+    import ctypes as C
+    s = QuantumStateC64(n) if c64 else QuantumState(n)
+    fn = lib.qs_expectation_value_pauli_weighted_c64 if c64 else lib.qs_expectation_value_pauli_weighted
+    x, y, cf, out = (np.zeros(1, dtype=t) for t in (np.uint64, np.uint32, np.complex128, np.complex128))
+    out[0] = 7.0
+    p = [a.ctypes.data_as(C.c_void_p) for a in (x, y, cf, out)]
+    assert fn(p[0], p[0], p[1], p[2], 0, s.data_ptr(), s.dim, None, p[3]) == 0
+    assert out[0] == 0
