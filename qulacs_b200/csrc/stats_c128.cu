@@ -285,6 +285,12 @@ int ev_tiled(const PauliTerm* terms, const std::vector<int>& xidx, UINT n, const
 
 constexpr UINT kEvOneLaunchQubits = 12;    // whole Hamiltonians of states up to this size go out as one launch
 constexpr UINT kBatchEvSingleQubits = 18;  // states at least this large are evaluated by passes of their own
+// Whether a small state's terms go out as jobs of one launch (ev_listed).  Their own kernels are faster for one
+// bit-flip string alone (at 10 qubits 33 us against 38; two strings 54 against 40) and for up to 16 Z-only strings
+// alone, which share a kernel (2, 8, 16 and 64 strings at 12 qubits: 41 49 55 176 us by their kernels, 47 61 73
+// 113 as jobs of 16 strings, 64 in jobs of 4: 92).  Z-only strings beside bit flips join the launch: one of each
+// at 14 qubits 47 us against 57.
+static bool ev_one_launch(size_t z_only, size_t flips) { return z_only ? flips > 0 || z_only > 16 : flips > 1; }
 // values[k] of the listed terms of one state, in one launch (one job per bit-flip string).
 template <class T>
 int ev_listed(const PauliTerm* terms, const std::vector<int>& zidx, const std::vector<int>& xidx, const T* s, ITYPE dim,
@@ -317,7 +323,7 @@ int ev_batch(const PauliTerm* terms, UINT count, const T* s, ITYPE dim, cudaStre
     // What is left of a small state's terms goes out as one launch: it is in the L2 cache, and a launch, a
     // fold and a synchronisation per string cost ~20 us (30 strings at 10 qubits: 600 us, in one launch 30).  A
     // large state is read from HBM once per string either way, and its strings come 16 to a pass or alone.
-    if (n < kBatchEvSingleQubits && zidx.size() + xidx.size() > 1)
+    if (n < kBatchEvSingleQubits && ev_one_launch(zidx.size(), xidx.size()))
         return ev_listed<T>(terms, zidx, xidx, s, dim, st, values);
     // Z-only terms left: kZChunk per pass.
     for (size_t c0 = 0; c0 < zidx.size(); c0 += kZChunk) {
@@ -828,11 +834,15 @@ QS_API int qs_reference_uniforms(QS_UINT seed, QS_UINT count, double* out) {
 // ---------------------------------------------------------------- batched expectation values
 // <P_k> for the terms of MANY states in one persistent launch.  A job is either up to 16 Z-only terms
 // of one state (one pass over its amplitudes) or one term with a bit flip (one pass over its pairs);
-// jobs are cut into chunks of kEvChunk items, one CTA per chunk at a time; every chunk writes FP64
+// jobs are cut into chunks of `chunk` items, one CTA per chunk at a time; every chunk writes FP64
 // partial sums, which a second kernel folds per job in chunk order (deterministic).
 namespace qs {
 
-constexpr ITYPE kEvChunk = 1 << 14;
+constexpr ITYPE kEvChunk = 1 << 14;  // many states
+// One state: chunks and Z-only jobs small enough that a call is not one CTA's loop.  One bit-flip and one Z-only
+// string at 14 qubits: 70 us with the sizes for many states, 47 with these; two bit flips at 17 qubits 57 and 45.
+constexpr ITYPE kEvListedChunk = 1 << 11;
+constexpr int kEvListedZ = 4;
 constexpr int kEvZ = 16;
 
 struct EvJob {
@@ -849,7 +859,7 @@ struct EvJob {
 };
 
 __global__ void __launch_bounds__(256) k_batch_ev(const EvJob* __restrict__ jobs, int njobs, ITYPE total,
-    const ITYPE* __restrict__ zmasks, double* __restrict__ partials) {
+    ITYPE chunk, const ITYPE* __restrict__ zmasks, double* __restrict__ partials) {
     __shared__ double sm[32];
     __shared__ int s_job;
     for (ITYPE item = blockIdx.x; item < total; item += gridDim.x) {
@@ -864,8 +874,8 @@ __global__ void __launch_bounds__(256) k_batch_ev(const EvJob* __restrict__ jobs
         }
         __syncthreads();
         const EvJob& J = jobs[s_job];
-        const ITYPE c0 = (item - J.prefix) * kEvChunk;
-        const ITYPE c1 = min(J.items, c0 + kEvChunk);
+        const ITYPE c0 = (item - J.prefix) * chunk;
+        const ITYPE c1 = min(J.items, c0 + chunk);
         if (J.kind == 1) {
             double acc = 0.;
             for (ITYPE p = c0 + threadIdx.x; p < c1; p += blockDim.x) {
@@ -904,11 +914,11 @@ __global__ void __launch_bounds__(256) k_batch_ev(const EvJob* __restrict__ jobs
     }
 }
 
-__global__ void k_batch_ev_fold(const EvJob* __restrict__ jobs, const double* __restrict__ partials,
+__global__ void k_batch_ev_fold(const EvJob* __restrict__ jobs, ITYPE chunk, const double* __restrict__ partials,
     const UINT* __restrict__ zout, double* __restrict__ values) {
     __shared__ double sm[32];
     const EvJob& J = jobs[blockIdx.x];
-    const ITYPE nchunks = (J.items + kEvChunk - 1) / kEvChunk;
+    const ITYPE nchunks = (J.items + chunk - 1) / chunk;
     const int width = J.kind == 1 ? 1 : J.nz;
     for (int w = 0; w < width; ++w) {
         double v = 0.;
@@ -951,10 +961,12 @@ struct EvJobs {
     std::vector<ITYPE> zm;
     std::vector<UINT> zout;
     ITYPE total = 0;
+    const ITYPE chunk;
+    explicit EvJobs(ITYPE chunk_items) : chunk(chunk_items) {}
 
     void add(EvJob J) {
         J.prefix = total;
-        total += (J.items + kEvChunk - 1) / kEvChunk;
+        total += (J.items + chunk - 1) / chunk;
         jobs.push_back(J);
     }
     void flip(const void* s, int c64, ITYPE dim, const PauliTerm& t, UINT out) {
@@ -1003,9 +1015,9 @@ struct EvJobs {
         double* dval = (double*)(p + bj + bz + bo + bp);
         QS_CUDA_CHECK(cudaMemcpyAsync(p, host.data(), host.size(), cudaMemcpyHostToDevice, st));
         const unsigned grid = (unsigned)std::min<ITYPE>(total, (ITYPE)sm_count() * 8);
-        k_batch_ev<<<grid, 256, 0, st>>>(dj, (int)jobs.size(), total, (const ITYPE*)(p + bj), dpart);
+        k_batch_ev<<<grid, 256, 0, st>>>(dj, (int)jobs.size(), total, chunk, (const ITYPE*)(p + bj), dpart);
         QS_TRY(check_launch("k_batch_ev"));
-        k_batch_ev_fold<<<(unsigned)jobs.size(), 256, 0, st>>>(dj, dpart, (const UINT*)(p + bj + bz), dval);
+        k_batch_ev_fold<<<(unsigned)jobs.size(), 256, 0, st>>>(dj, chunk, dpart, (const UINT*)(p + bj + bz), dval);
         QS_TRY(check_launch("k_batch_ev_fold"));
         QS_CUDA_CHECK(cudaMemcpyAsync(values, dval, sizeof(double) * nvals, cudaMemcpyDeviceToHost, st));
         QS_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -1017,13 +1029,13 @@ template <class T>
 int ev_listed(const PauliTerm* terms, const std::vector<int>& zidx, const std::vector<int>& xidx, const T* s, ITYPE dim,
     cudaStream_t st, double* values) {
     constexpr int c64 = sizeof(T) == sizeof(float2);
-    EvJobs W;
+    EvJobs W(kEvListedChunk);
     UINT at = 0;  // values in the order of zidx, then xidx
-    for (size_t z0 = 0; z0 < zidx.size(); z0 += kEvZ) {
-        ITYPE m[kEvZ];
-        UINT o[kEvZ];
+    for (size_t z0 = 0; z0 < zidx.size(); z0 += kEvListedZ) {
+        ITYPE m[kEvListedZ];
+        UINT o[kEvListedZ];
         int c = 0;
-        for (; c < kEvZ && z0 + c < zidx.size(); ++c) {
+        for (; c < kEvListedZ && z0 + c < zidx.size(); ++c) {
             m[c] = terms[zidx[z0 + c]].z;
             o[c] = at++;
         }
@@ -1047,7 +1059,7 @@ static int batch_ev_impl(void* const* states, const QS_UINT* qubit_counts, QS_UI
     const QS_ITYPE* x_masks, const QS_ITYPE* z_masks, const QS_UINT* y_counts, double* values, int c64,
     cudaStream_t st, bool skip_large) {
     if (!states || !qubit_counts || !term_offsets || !values) return set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
-    EvJobs W;
+    EvJobs W(kEvChunk);
     const UINT nterms = term_offsets[count];
     for (UINT i = 0; i < count; ++i) {
         const UINT n = qubit_counts[i];
@@ -2030,9 +2042,10 @@ int ev_weighted(const PauliTerm* terms, const double2* coefs, UINT count, const 
     // strings in us, by passes and so: 11 qubits 61 78 127 210, 58 74 114 183; 12 qubits 53 74 119 217, 52 68 115
     // 167; 13 qubits 52 76 118 204, 64 78 128 188; 15 qubits 52 74 130 216, 77 92 143 214.  (Forced modes keep the
     // passes at every size.)
-    if (n <= kEvOneLaunchQubits && g_ev_spec_mode.load() == 1) {
-        std::vector<int> zidx, xidx;
+    std::vector<int> zidx, xidx;
+    if (n <= kEvOneLaunchQubits && g_ev_spec_mode.load() == 1)
         for (UINT k = 0; k < count; ++k) (terms[k].x == 0 ? zidx : xidx).push_back((int)k);
+    if (ev_one_launch(zidx.size(), xidx.size())) {
         std::vector<double> v(count);
         QS_TRY(ev_listed<T>(terms, zidx, xidx, s, dim, st, v.data()));
         out[0] = out[1] = 0.;

@@ -195,3 +195,22 @@ def test_empty_sum_is_zero(lib, n, c64):
     p = [a.ctypes.data_as(C.c_void_p) for a in (x, y, cf, out)]
     assert fn(p[0], p[0], p[1], p[2], 0, s.data_ptr(), s.dim, None, p[3]) == 0
     assert out[0] == 0
+
+
+@pytest.mark.parametrize("c64", [False, True])
+@pytest.mark.parametrize("n", [1, 8, 12, 14, 17])
+@pytest.mark.parametrize("flips,z_only", [(1, 0), (2, 0), (0, 1), (0, 16), (0, 17), (1, 1), (3, 5)])
+def test_small_states_at_the_edges_of_one_launch(port, n, flips, z_only, c64):
+    """Lists on both sides of the rule that sends a small state's strings out as one launch."""
+    rng = np.random.default_rng(17 * n + flips + 3 * z_only)
+    v = random_state(n, rng)
+    if c64:
+        v = v.astype(np.complex64).astype(np.complex128)
+    s = QuantumStateC64(n) if c64 else QuantumState(n)
+    s.load(v)
+    ts = [(float(rng.normal()), [int(rng.integers(n))], [1 + i % 2]) for i in range(flips)]
+    ts += [(float(rng.normal()), [int(rng.integers(n))], [3]) for _ in range(z_only)]
+    obs = W.to_observable(ts, n)
+    want = np.array([port.expectation_value(tl, ids, v) for _, tl, ids in ts])
+    assert np.max(np.abs(obs.term_values(s) - want)) <= EV_TOL
+    assert abs(obs.get_expectation_value(s) - float(np.dot([t[0] for t in ts], want))) <= EV_TOL * len(ts)
