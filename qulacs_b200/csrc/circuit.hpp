@@ -122,8 +122,8 @@ void apply_gate_to_block(std::vector<std::complex<double>>& U, int kb, const Gat
 std::vector<GateRec> fuse_gates(const std::vector<GateRec>& G, int k);
 // fusion.cpp: each run of one-qubit unitaries on a qubit as a diagonal and a real rotation, the rotation's
 // second diagonal carried forward (through controls, CZ and other diagonals) into the next run.  `spec`: for
-// specialised passes; else a CNOT becomes H CZ H on its target and no RX is left, so that every phase of such
-// gates is rounds of diagonals and RY (run_rounds, staged.cu).
+// specialised passes; else no RX is left, so that phases of such gates are rounds of diagonals and RY (run_rounds,
+// staged.cu).
 std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec);
 // fusion.cpp: the gate list that the staged executors run at block size k; *blocks: gates after the fusion
 // (fuse_gates' count).

@@ -385,24 +385,11 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         k.post_unit = true;
         k.p0 = k.p1 = 1.L;
     };
-    const ld h = std::sqrt(0.5L);
-    const cl had[4] = {h, h, h, -h};
     for (const GateRec& g : G) {
         if (g.targets.size() == 1 && g.controls.empty() && g.kind != QS_GATE_DEPOLARIZING) {
             cl m[4];
             xmatrix(g, m);
             add_matrix(g.targets[0], g.kind, m);
-            continue;
-        }
-        if (g.kind == QS_GATE_CNOT && !spec) {
-            add_matrix(g.targets[1], QS_GATE_DENSE, had);
-            end_run(g.targets[0]);
-            end_run(g.targets[1]);
-            GateRec z;
-            z.kind = QS_GATE_CZ;
-            z.targets = g.targets;
-            out.push_back(z);
-            add_matrix(g.targets[1], QS_GATE_DENSE, had);
             continue;
         }
         for (UINT q : g.qubits()) end_run(q);

@@ -82,11 +82,24 @@ struct PassScalar {
 };
 
 struct Builder {
-    uint8_t F[4] = {1, 2, 4, 8}, V[4] = {1, 2, 4, 8}, A[4] = {};
+    // each qubit's functional, vector and constant over the register's index
+    uint8_t F[4], V[4], A[4] = {};
     std::vector<Node> nodes;
     PassScalar& S;
     const bool move;  // CNOT, SWAP and X are steps; the map stays the identity
-    Builder(PassScalar& s, bool m, size_t gates) : S(s), move(m) { nodes.reserve(gates); }
+    Builder(PassScalar& s, bool m, size_t gates, const uint8_t* in) : S(s), move(m) {
+        nodes.reserve(gates);
+        for (int b = 0; b < 4; ++b) {
+            F[b] = 0;
+            for (int k = 0; k < 4; ++k) F[b] |= (uint8_t)(((in[k] >> b) & 1) << k);
+        }
+        for (int j = 0; j < 16; ++j) {
+            int i = 0;
+            for (int k = 0; k < 4; ++k)
+                if ((j >> k) & 1) i ^= in[k];
+            if (i && !(i & (i - 1))) V[__builtin_ctz(i)] = (uint8_t)j;
+        }
+    }
 
     // qubit i of the node's step is register bit b; x, z: whether the node moves and reads it
     void set_qubit(Node& n, int i, int b, bool x = true, bool z = true) {
@@ -333,7 +346,7 @@ std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count
             const bool diag = one && m[1].x == 0. && m[1].y == 0. && m[2].x == 0. && m[2].y == 0.;
             move = move || o->kind == ST_DENSE2 || o->kind == ST_DEPOL1 || o->kind == ST_DEPOL2 || (one && !flip && !diag);
         }
-        Builder B(S, move, (size_t)(end - begin));
+        Builder B(S, move, (size_t)(end - begin), phases[ph].in);
         for (const StOp* op = begin; op != end; ++op) {
             const StOp& o = *op;
             const double2* p = pool + o.param;
@@ -381,55 +394,64 @@ std::vector<PhaseProgram> build_pass_program(const StPhase* phases, size_t count
     return out;
 }
 
-// The program as rounds, if it holds nothing else than signs, diagonals and scaled RY on register bits.
+// The program as rounds, if it holds nothing else than signs, diagonals and scaled RY (on register bits: the
+// planner starts a new phase where a CNOT has relabelled a register that turns again).
 static bool encode_rounds(const PhaseProgram& P, StPhase* phase, std::vector<double2>* pool) {
     for (const ProgStep& s : P.steps) {
-        const bool ry = s.kind == SP_ROT && s.form == RF_Y_TAN && !(s.v[0] & (s.v[0] - 1)) && s.f[0] == s.v[0];
+        const bool ry = s.kind == SP_ROT && s.form == RF_Y_TAN;
         if (!ry && s.kind != SP_DIAG && s.kind != SP_SIGN && s.kind != SP_SCALE) return false;
     }
-    const double2 one = make_double2(1., 0.);
-    double2 d[16];
-    double t[4];
-    int used;    // register bits with a rotation in this round
-    bool diag;
-    auto clear = [&]() {
-        for (double2& v : d) v = one;
-        for (double& v : t) v = 0.;
-        used = 0;
-        diag = false;
+    // turns (4 tangents) and factors in the order in which they run
+    struct Part {
+        bool turns;
+        double2 v[16];
     };
-    auto close = [&]() {
-        pool->insert(pool->end(), d, d + 16);
-        pool->push_back(make_double2(t[0], t[1]));
-        pool->push_back(make_double2(t[2], t[3]));
-        ++phase->rounds;
-        clear();
+    std::vector<Part> parts;
+    auto open = [&](bool turns) {
+        parts.emplace_back();
+        parts.back().turns = turns;
+        for (double2& v : parts.back().v) v = turns ? make_double2(0., 0.) : make_double2(1., 0.);
     };
-    clear();
-    phase->param = (uint32_t)pool->size();
-    phase->rounds = phase->tail = 0;
+    int used = 0;  // register bits that the open turns have
     for (const ProgStep& s : P.steps) {
         if (s.kind == SP_ROT) {
             const int b = __builtin_ctz(s.v[0]);
-            if (used >> b) close();  // ascending: the order in which a round runs them
+            if (parts.empty() || !parts.back().turns || used >> b) {  // ascending: the order in which they run
+                open(true);
+                used = 0;
+            }
             used |= 1 << b;
-            t[b] = s.a[0] ? -s.par[0].x : s.par[0].x;
+            double2& t = parts.back().v[b / 2];
+            (b & 1 ? t.y : t.x) = s.a[0] ? -s.par[0].x : s.par[0].x;
             continue;
         }
-        if (used) close();
-        diag = true;
+        if (parts.empty() || parts.back().turns) open(false);
         for (int j = 0; j < 16; ++j) {
             if (s.kind != SP_SCALE && !((s.mask >> j) & 1)) continue;
             const double2 z = s.kind == SP_SIGN ? make_double2(-1., 0.) : s.par[s.kind == SP_SCALE ? 0 : j];
+            double2& d = parts.back().v[j];
             // signs next to factors stay exact
-            d[j] = make_double2(z.x * d[j].x - z.y * d[j].y, z.x * d[j].y + z.y * d[j].x);
+            d = make_double2(z.x * d.x - z.y * d.y, z.x * d.y + z.y * d.x);
         }
     }
-    if (used) close();
-    else if (diag) {
-        pool->insert(pool->end(), d, d + 16);
-        phase->tail = 1;
+    phase->param = (uint32_t)pool->size();
+    phase->rounds = 0;
+    if (parts.empty()) return true;
+    // the order of a round that leaves fewer sets of factors 1
+    const bool turns_first = parts.front().turns && !parts.back().turns;
+    bool turns = turns_first;  // the kind of the next part of a round
+    auto put = [&](const Part* q) {
+        for (int j = 0; j < (turns ? 2 : 16); ++j)
+            pool->push_back(q ? q->v[j] : turns ? make_double2(0., 0.) : make_double2(1., 0.));
+        if (turns) ++phase->rounds;
+        turns = !turns;
+    };
+    for (const Part& q : parts) {
+        if (q.turns != turns) put(nullptr);
+        put(&q);
     }
+    if (turns_first) phase->flags |= PH_TURNS_FIRST;
+    else if (turns) phase->flags |= PH_TAIL;
     return true;
 }
 
@@ -441,7 +463,7 @@ void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vect
     for (int k = 0; k < 4; ++k) phase->out[k] = P.out[1 << k] ^ P.out[0];
     phase->step_count = 0;
     if (encode_rounds(P, phase, pool)) return;
-    phase->rounds = phase->tail = 0;
+    phase->rounds = 0;
     for (const ProgStep& s : P.steps) {
         StStep t{};
         t.param = (uint32_t)pool->size();
@@ -455,10 +477,7 @@ void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vect
             case SP_X: t.code = (uint8_t)(16 + a * 5); break;
             case SP_SWAP: t.code = (uint8_t)(32 + std::min(a, b) * 4 + std::max(a, b)); break;
             case SP_DENSE1: t.code = (uint8_t)(32 + a * 5); break;
-            case SP_DEPOL1:
-                t.code = (uint8_t)(32 + std::max(a, b) * 4 + std::min(a, b));
-                t.mask = s.form;
-                break;
+            case SP_DEPOL1: t.code = (uint8_t)((s.form ? 80 : 32) + std::max(a, b) * 4 + std::min(a, b)); break;
             case SP_DENSE2: t.code = (uint8_t)(48 + a * 4 + b); break;
             case SP_DEPOL2: {  // by the partner of register bit 0: 1, 2 or 3
                 const int c = bit(s.v[2]), d = bit(s.v[3]);
@@ -467,19 +486,16 @@ void encode_program(const PhaseProgram& P, std::vector<StStep>* steps, std::vect
                 t.mask = s.form;
                 break;
             }
-            case SP_ROT: {
-                const bool tan = s.form == RF_Y_TAN || s.form == RF_X_TAN, x = s.form >= RF_X_TAN;
-                t.code = (uint8_t)(64 + 32 * x + 16 * !tan + s.v[0]);
-                const int low = s.v[0] & -s.v[0];
-                for (int j = 0, k = 0; j < 16; ++j)
-                    if (!(j & low)) t.mask |= (uint16_t)(step_bit(s, 0, j) << k++);
-                break;
-            }
+            case SP_ROT: t.code = (uint8_t)(64 + (s.form == RF_Y_TAN ? 0 : 4) + a); break;
         }
-        if (s.kind == SP_ROT && (s.form == RF_Y_COT || s.form == RF_X_COT))
-            pool->push_back(make_double2(s.par[0].x, 1.));  // c = cot, s = 1: the same products and sums
-        else
+        if (s.kind == SP_ROT) {  // rotation_form leaves RY alone; a relabelled bit turns the other way
+            const double sign = s.a[0] ? -1. : 1.;
+            if (s.form == RF_Y_TAN) pool->push_back(make_double2(sign * s.par[0].x, 0.));
+            else if (s.form == RF_Y_COT) pool->push_back(make_double2(s.par[0].x, sign));  // cosine and sine over the sine
+            else pool->push_back(make_double2(s.par[0].x, sign * s.par[0].y));
+        } else {
             pool->insert(pool->end(), s.par.begin(), s.par.end());
+        }
         steps->push_back(t);
     }
     phase->step_count = (uint32_t)(steps->size() - phase->step_begin);

@@ -11,7 +11,7 @@
 //    factors per coset (4 per amplitude) for every diagonal that can meet there, or sign flips alone (0);
 //  * CNOT, SWAP and X only relabel registers (an affine map over GF(2) of the register index), 0.  In a
 //    phase with dense matrices or channels they are steps that move registers, so that those act on
-//    register bits.
+//    register bits.  The generic kernels rotate along register bits only (relabel_segments, csrc/staged.cu).
 #pragma once
 
 #include <complex>

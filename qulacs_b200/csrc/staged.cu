@@ -10,15 +10,19 @@
 // per gate.  A phase's gates run as a program of rotations, collected diagonals and register relabellings
 // (phase_program.hpp), which the kernels here interpret step by step; the specialised pass kernels
 // (pass_codegen.cpp) run the same programs as straight-line code.  The host scheduler (below) builds passes
-// and phases greedily from the gate list in rotation form (fusion.cpp); a gate is only moved past gates
-// on disjoint qubits, so the result equals gate-by-gate application up to rounding (~1e-16).  Gates the
-// pass kernel does not cover (more than 2 targets, controls, Pauli strings, multi-qubit diagonals) run
+// and phases greedily from the gate list in rotation form (fusion.cpp).  The scheduler moves a gate only past
+// gates on disjoint qubits; rotation form carries unitary diagonals past controls, CZ, SWAP, diagonals and
+// depolarizing channels, with which they commute, and a phase's program reorders steps that commute.  So the
+// result equals gate-by-gate application up to rounding (~1e-16), and exactly where gates only permute.  Gates
+// the pass kernel does not cover (more than 2 targets, controls, Pauli strings, multi-qubit diagonals) run
 // between passes with the gate-by-gate kernels.
 //
-// What bounds the generic kernel on small states is the chain of steps in a CTA: one coset per thread (256
-// threads for a 2^12-amplitude tile, where 128 threads took two in turn) and rotations in place of matrices
-// brought the 16-qubit layered circuit (16 tiles, 454 gates) from 0.43 to 0.23 ms, rounds (run_rounds) to 0.21;
-// 20 layers of U3 + CZ on 26 qubits took 46.9 ms step by step and 29.2 in rounds (specialised: 16.0).
+// What bounds the generic kernel on small states is the chain of rounds in a CTA: one coset per thread (256
+// threads for a 2^12-amplitude tile, where 128 threads took two in turn), rotations in place of matrices and
+// rounds (run_rounds) brought the layered circuit on 16 qubits from 0.43 to 0.20 ms; CNOTs as relabellings of the
+// coset's addresses (relabel_segments; H CZ H on the target before, 42 phases with 197 rounds against 87 with 81)
+// further, with the record of a phase read as four words (some forty loads field by field).  20 layers of
+// U3 + CZ on 26 qubits took 46.9 ms step by step and 26.5 in rounds (specialised: 16.0).
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -61,49 +65,27 @@ __device__ __forceinline__ double2 ld_par(const double2* p) {
 __device__ __forceinline__ double flipped(double t, unsigned odd) {  // -t where odd is 1
     return __hiloint2double(__double2hiint(t) ^ (int)(odd << 31), __double2loint(t));
 }
-// Rotations: register pairs (lo, lo ^ V), lo without V's lowest bit.  A pair whose lo has the qubit's value 1
-// (bit k of `rev`) runs with the sine's sign reversed.
-template <int V, class F>
-__device__ __forceinline__ void for_pairs(double2 (&r)[16], F f) {
-    constexpr int low = V & -V;
-    int k = 0;
+template <int B>
+__device__ __forceinline__ void r_ry_tan(double2 (&r)[16], double t) {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
-        if (!(j & low)) f(r[j], r[j ^ V], k++);
+        if (!(j & (1 << B))) {
+            double2 &x = r[j], &y = r[j | (1 << B)];
+            const double2 X = x;
+            x = make_double2(fma(t, y.x, X.x), fma(t, y.y, X.y));
+            y = make_double2(fma(-t, X.x, y.x), fma(-t, X.y, y.y));
+        }
 }
-template <int V>
-__device__ __forceinline__ void r_ry_tan(double2 (&r)[16], double t0, unsigned rev) {
-    for_pairs<V>(r, [&](double2& x, double2& y, int k) {
-        const double t = flipped(t0, (rev >> k) & 1u);
-        const double2 X = x;
-        x = make_double2(fma(t, y.x, X.x), fma(t, y.y, X.y));
-        y = make_double2(fma(-t, X.x, y.x), fma(-t, X.y, y.y));
-    });
-}
-template <int V>
-__device__ __forceinline__ void r_ry_full(double2 (&r)[16], double c, double s0, unsigned rev) {
-    for_pairs<V>(r, [&](double2& x, double2& y, int k) {
-        const double s = flipped(s0, (rev >> k) & 1u);
-        const double2 X = x;
-        x = make_double2(fma(c, X.x, s * y.x), fma(c, X.y, s * y.y));
-        y = make_double2(fma(c, y.x, -s * X.x), fma(c, y.y, -s * X.y));
-    });
-}
-template <int V>
-__device__ __forceinline__ void r_rx_tan(double2 (&r)[16], double t) {
-    for_pairs<V>(r, [&](double2& x, double2& y, int) {
-        const double2 X = x;
-        x = make_double2(fma(-t, y.y, X.x), fma(t, y.x, X.y));
-        y = make_double2(fma(-t, X.y, y.x), fma(t, X.x, y.y));
-    });
-}
-template <int V>
-__device__ __forceinline__ void r_rx_full(double2 (&r)[16], double c, double s) {
-    for_pairs<V>(r, [&](double2& x, double2& y, int) {
-        const double2 X = x;
-        x = make_double2(fma(c, X.x, -s * y.y), fma(c, X.y, s * y.x));
-        y = make_double2(fma(c, y.x, -s * X.y), fma(c, y.y, s * X.x));
-    });
+template <int B>
+__device__ __forceinline__ void r_ry_full(double2 (&r)[16], double c, double s) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (!(j & (1 << B))) {
+            double2 &x = r[j], &y = r[j | (1 << B)];
+            const double2 X = x;
+            x = make_double2(fma(c, X.x, s * y.x), fma(c, X.y, s * y.y));
+            y = make_double2(fma(c, y.x, -s * X.x), fma(c, y.y, -s * X.y));
+        }
 }
 __device__ __forceinline__ void r_diag(double2 (&r)[16], const double2* __restrict__ p, unsigned mask) {
 #pragma unroll
@@ -182,16 +164,9 @@ __device__ __forceinline__ void r_swap(double2 (&r)[16]) {
             r[k] = t;
         }
 }
-// One-qubit depolarizing channel (column and row bit A, B): populations mix, coherences shrink.  `full` (the
-// channel itself, not scaled): the factor by which the populations shrink first.
+// One-qubit depolarizing channel, scaled (column and row bit A, B): populations mix, coherences shrink.
 template <int A, int B>
-__device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k, const double2* __restrict__ full) {
-    if (full) {
-        const double d = full->x;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (!(j & (1 << A)) == !(j & (1 << B))) r[j] = make_double2(d * r[j].x, d * r[j].y);
-    }
+__device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k) {
 #pragma unroll
     for (int j = 0; j < 16; ++j)
         if (!(j & (1 << A)) && !(j & (1 << B))) {
@@ -202,6 +177,14 @@ __device__ __forceinline__ void r_depol1(double2 (&r)[16], double t, double k, c
             r[j | (1 << A)] = make_double2(k * r[j | (1 << A)].x, k * r[j | (1 << A)].y);
             r[j | (1 << B)] = make_double2(k * r[j | (1 << B)].x, k * r[j | (1 << B)].y);
         }
+}
+// The channel itself: the populations shrink by d before they mix.
+template <int A, int B>
+__device__ __forceinline__ void r_depol1_full(double2 (&r)[16], double t, double k, double d) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (!(j & (1 << A)) == !(j & (1 << B))) r[j] = make_double2(d * r[j].x, d * r[j].y);
+    r_depol1<A, B>(r, t, k);
 }
 // Two-qubit depolarizing channel on pairs of register bits (0, MATE) and the other two: the four populations
 // have equal bits in each pair.
@@ -220,7 +203,7 @@ __device__ __forceinline__ void r_depol2(double2 (&r)[16], double t, double k, b
 //   0 diagonal, 1 signs, 2 real and 3 complex scale;  16..31 CNOT a * 4 + b, X at a = b;
 //   32..47 SWAP (a < b), one-qubit matrix (a = b), one-qubit channel (a > b);
 //   48..63 two-qubit matrix, two-qubit channel at a = b (register bit 0's partner a + 1);
-//   64.. RY scaled by the pair vector, 80.. RY with cosine and sine, 96.. RX, 112.. RX with cosine and sine.
+//   64..67 RY scaled, 68..71 RY with cosine and sine;  80.. one-qubit channel unscaled (a > b).
 template <int CODE>
 __device__ __forceinline__ void run_step(double2 (&r)[16], const double2* __restrict__ p, unsigned mask) {
     constexpr int kind = CODE >> 4, V = CODE & 15, A = V >> 2, B = V & 3;
@@ -238,13 +221,12 @@ __device__ __forceinline__ void run_step(double2 (&r)[16], const double2* __rest
     else if constexpr (kind == 1) r_x<A>(r);
     else if constexpr (kind == 2 && A < B) r_swap<A, B>(r);
     else if constexpr (kind == 2 && A == B) r_dense1<A>(r, p);
-    else if constexpr (kind == 2) r_depol1<A, B>(r, p[0].x, p[0].y, mask ? p + 1 : nullptr);
+    else if constexpr (kind == 2) r_depol1<A, B>(r, p[0].x, p[0].y);
     else if constexpr (kind == 3 && A != B) r_dense2<A, B>(r, p);
     else if constexpr (kind == 3 && A < 3) r_depol2<A + 1>(r, p[0].x, p[0].y, mask != 0);
-    else if constexpr (kind == 4 && V) r_ry_tan<V>(r, p[0].x, mask);
-    else if constexpr (kind == 5 && V) r_ry_full<V>(r, p[0].x, p[0].y, mask);
-    else if constexpr (kind == 6 && V) r_rx_tan<V>(r, p[0].x);
-    else if constexpr (kind == 7 && V) r_rx_full<V>(r, p[0].x, p[0].y);
+    else if constexpr (kind == 4 && A == 0) r_ry_tan<B>(r, p[0].x);
+    else if constexpr (kind == 4 && A == 1) r_ry_full<B>(r, p[0].x, p[0].y);
+    else if constexpr (kind == 5 && A > B) r_depol1_full<A, B>(r, p[0].x, p[0].y, p[1].x);
 }
 #define QS_CODE1(c) \
     case c: run_step<c>(r, p, s.mask); break;
@@ -257,10 +239,9 @@ __device__ __forceinline__ void apply_step(const StStep& s, double2 (&r)[16], co
         QS_CODE16(16)
         QS_CODE16(32)
         QS_CODE16(48)
-        QS_CODE16(64)
+        QS_CODE4(64)
+        QS_CODE4(68)
         QS_CODE16(80)
-        QS_CODE16(96)
-        QS_CODE16(112)
         default: break;
     }
 }
@@ -268,53 +249,65 @@ __device__ __forceinline__ void apply_step(const StStep& s, double2 (&r)[16], co
 #undef QS_CODE4
 #undef QS_CODE1
 
-// Rounds of 16 diagonal factors and a scaled rotation on each register bit (factor 1, tangent 0 where there is
-// none): straight-line code on fixed registers.  Conditions around the parts, or the switch over step kinds,
-// cost moves of the whole coset at every join: the FP64 pipe was 15 % busy at 63 % issue with the switch, 20 %
-// with conditions, 35 % (46 % in the fullest passes) with rounds.  Reading factors ahead across rounds gained
-// 3 % at 14 qubits and lost 3 % at 26, and was not kept.
+// Rounds of 16 diagonal factors and a scaled rotation on each register bit, in either order (factor 1, tangent 0
+// where there is none): straight-line code on fixed registers.  Conditions around the parts, or the switch over
+// step kinds, cost moves of the whole coset at every join: the FP64 pipe was 15 % busy at 63 % issue with the
+// switch, 20 % with conditions, 35 % (46 % in the fullest passes) with rounds.  A condition between rotations and
+// factors, in place of the two orders, cost 20 % of a 10-qubit circuit: the factors' loads waited behind it.
+// Reading factors ahead across rounds gained 3 % at 14 qubits and lost 3 % at 26, and was not kept.
+__device__ __forceinline__ void r_turns(double2 (&r)[16], const double2* __restrict__ p) {
+    const double2 t01 = ld_par(p), t23 = ld_par(p + 1);
+    r_ry_tan<0>(r, t01.x);
+    r_ry_tan<1>(r, t01.y);
+    r_ry_tan<2>(r, t23.x);
+    r_ry_tan<3>(r, t23.y);
+}
 __device__ __forceinline__ void run_rounds(const StPhase& P, double2 (&r)[16], const double2* __restrict__ p) {
+    if (P.flags & PH_TURNS_FIRST) {
+#pragma unroll 1
+        for (UINT o = 0; o < P.rounds; ++o, p += 18) {
+            r_turns(r, p);
+            r_diag(r, p + 2, 0xffffu);
+        }
+        return;
+    }
 #pragma unroll 1
     for (UINT o = 0; o < P.rounds; ++o, p += 18) {
         r_diag(r, p, 0xffffu);
-        const double2 t01 = ld_par(p + 16), t23 = ld_par(p + 17);
-        r_ry_tan<1>(r, t01.x, 0);
-        r_ry_tan<2>(r, t01.y, 0);
-        r_ry_tan<4>(r, t23.x, 0);
-        r_ry_tan<8>(r, t23.y, 0);
+        r_turns(r, p + 16);
     }
-    if (P.tail) r_diag(r, p, 0xffffu);
+    if (P.flags & PH_TAIL) r_diag(r, p, 0xffffu);
 }
 
 __device__ __forceinline__ UINT swz(UINT u) { return QS_SWZ(u); }
 
-// Tile index u = tid + k * THREADS has global offset base | lo_off | hi_off[k]: lo_off takes tid's bits to
+// Tile index u = tid + k * threads has global offset base | lo_off | hi_off[k]: lo_off takes tid's bits to
 // the lowest tile qubits, hi_off[k] takes k's bits to the others.
 
 // Global rows of 16 amplitudes per thread from the swizzled tile to HBM.
-template <int THREADS, class T>
+template <UINT threads, class T>
 __device__ __forceinline__ void tile_rows_store(T* __restrict__ s, const double2* tile, ITYPE off,
     const ITYPE* hi_off, UINT tsize) {
     const UINT tid = threadIdx.x;
     double2 v[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-        if (tid + (UINT)k * THREADS < tsize) v[k] = tile[swz(tid + (UINT)k * THREADS)];
+        if (tid + (UINT)k * threads < tsize) v[k] = tile[swz(tid + (UINT)k * threads)];
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-        if (tid + (UINT)k * THREADS < tsize) st_amp(s + (off | hi_off[k]), v[k]);
+        if (tid + (UINT)k * threads < tsize) st_amp(s + (off | hi_off[k]), v[k]);
 }
 
 // One tile of one pass: load, apply every phase, store.  Shared by the per-pass kernel and the
 // persistent multi-circuit kernel.  `tile` holds 2^m amplitudes (m <= MAX_BITS) in FP64 whatever the
-// state's type E (complex128, or complex64 widened on load and rounded on store).  THREADS is the largest
-// tile's coset count: one 16-amplitude coset per thread and phase.  Ends with a CTA barrier so the shared
-// buffers can be reused immediately.
-template <int MAX_BITS, int THREADS, class E>
+// state's type E (complex128, or complex64 widened on load and rounded on store).  One 16-amplitude coset per
+// thread and phase, for the cosets of the largest tile.  Ends with a CTA barrier so the shared buffers can be
+// reused immediately.
+template <int MAX_BITS, class E>
 __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs& a, ITYPE T, double2* tile,
     ITYPE* hi_off) {
-    static_assert(THREADS == 1 << (MAX_BITS - kPhaseBits), "one coset per thread");
-    constexpr int TB = MAX_BITS - kPhaseBits;
+    constexpr int tb = MAX_BITS - kPhaseBits;
+    constexpr UINT threads = 1u << tb;
     const int m = a.m;
     const UINT tsize = 1u << m;
     // base: insert zeros at the tile qubits into the tile index
@@ -326,11 +319,11 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
     if (!hbm_first || !hbm_last) {
         if (tid < 16) {
             ITYPE o = 0;
-            for (int j = TB; j < m; ++j)
-                if ((tid >> (j - TB)) & 1) o |= 1ULL << a.q[j];
+            for (int j = tb; j < m; ++j)
+                if ((tid >> (j - tb)) & 1) o |= 1ULL << a.q[j];
             hi_off[tid] = o;
         }
-        for (int j = 0; j < TB && j < m; ++j)
+        for (int j = 0; j < tb && j < m; ++j)
             if ((tid >> j) & 1) lo_off |= 1ULL << a.q[j];
         __syncthreads();
     }
@@ -341,9 +334,9 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
             // once, without holding registers
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                if ((UINT)tid + (UINT)k * THREADS < tsize) {
+                if ((UINT)tid + (UINT)k * threads < tsize) {
                     const unsigned dst =
-                        (unsigned)__cvta_generic_to_shared(tile + swz((UINT)tid + (UINT)k * THREADS));
+                        (unsigned)__cvta_generic_to_shared(tile + swz((UINT)tid + (UINT)k * threads));
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(s + (off | hi_off[k]))
                                  : "memory");
                 }
@@ -355,11 +348,11 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
                 double2 v[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    if ((UINT)tid + (UINT)(k0 + k) * THREADS < tsize) v[k] = ld_amp(s + (off | hi_off[k0 + k]));
+                    if ((UINT)tid + (UINT)(k0 + k) * threads < tsize) v[k] = ld_amp(s + (off | hi_off[k0 + k]));
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    if ((UINT)tid + (UINT)(k0 + k) * THREADS < tsize)
-                        tile[swz((UINT)tid + (UINT)(k0 + k) * THREADS)] = v[k];
+                    if ((UINT)tid + (UINT)(k0 + k) * threads < tsize)
+                        tile[swz((UINT)tid + (UINT)(k0 + k) * threads)] = v[k];
             }
         }
         __syncthreads();
@@ -367,7 +360,13 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
     const UINT ncos = tsize >> kPhaseBits;  // cosets per phase
     char* tile_bytes = reinterpret_cast<char*>(tile);
     for (int ph = 0; ph < a.nphases; ++ph) {
-        const StPhase P = a.phases[ph];
+        StPhase P;
+        {  // whole words: field by field it is some forty loads
+            uint4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = reinterpret_cast<const uint4*>(a.phases + ph)[i];
+            memcpy(&P, w, sizeof(P));
+        }
         // The first phase may gather its cosets straight from HBM and the last scatter them straight to
         // HBM (the host sets this when the phase's bits are all >= 4, so that a coset's lanes 0..15 cover
         // 16 consecutive amplitudes): no tile load or store round through shared memory.
@@ -375,30 +374,36 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
         if ((UINT)tid < ncos) {
             UINT u0 = 0;
 #pragma unroll
-            for (int k = 0; k < TB; ++k) u0 |= ((tid >> k) & 1u) << P.order[k];
+            for (int k = 0; k < tb; ++k) u0 |= ((tid >> k) & 1u) << P.order[k];
             ITYPE g0 = base;  // global index of the coset's first amplitude (only for HBM phases)
             if (from_hbm || to_hbm)
                 for (int j = 0; j < m; ++j)
                     if ((u0 >> j) & 1) g0 |= 1ULL << a.q[j];
+            auto global_bits = [&](UINT i) {  // qubits of coset index i
+                ITYPE u = 0;
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if ((i >> p) & 1u) u |= 1ULL << a.q[P.bits[p]];
+                return u;
+            };
             double2 r[16];
-            // Offset of coset index j from the coset's first amplitude: the XOR of one offset per set bit of
-            // j (the swizzle is XOR-linear).  The 16 amplitudes are visited in Gray-code order, so that each
-            // address is the previous one with one offset XORed in.
+            // Offset of register j from the coset's first amplitude: the XOR of one offset per set bit of j (the
+            // relabelling and the swizzle are XOR-linear).  The 16 amplitudes are visited in Gray-code order, so
+            // that each address is the previous one with one offset XORed in.
             if (from_hbm) {
-                ITYPE gi = g0;
+                ITYPE gb[4], gi = g0;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) gb[p] = global_bits(P.in[p]);
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
-                    if (g) gi ^= 1ULL << a.q[P.bits[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3]];
+                    if (g) gi ^= gb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     r[g ^ (g >> 1)] = ld_amp(s + gi);
                 }
             } else {
-                UINT sb[4];
-#pragma unroll
-                for (int p = 0; p < 4; ++p) sb[p] = swz(1u << P.bits[p]) << 4;
                 UINT addr = swz(u0) << 4;
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
-                    if (g) addr ^= sb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
+                    if (g) addr ^= P.in_at[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     r[g ^ (g >> 1)] = *reinterpret_cast<const double2*>(tile_bytes + addr);
                 }
             }
@@ -406,42 +411,27 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
             else
                 for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
             // register j goes to coset index out0 ^ (XOR of out[k] over the bits k of j)
-            auto tile_index = [&](UINT i) {
-                UINT u = 0;
-#pragma unroll
-                for (int p = 0; p < 4; ++p) u |= ((i >> p) & 1u) << P.bits[p];
-                return u;
-            };
             if (to_hbm) {
-                ITYPE gb[4], gi = g0;
+                ITYPE gb[4], gi = g0 | global_bits(P.out0);
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    gb[p] = 0;
-#pragma unroll
-                    for (int b = 0; b < 4; ++b)
-                        if ((P.out[p] >> b) & 1) gb[p] |= 1ULL << a.q[P.bits[b]];
-                    if ((P.out0 >> p) & 1) gi |= 1ULL << a.q[P.bits[p]];
-                }
+                for (int p = 0; p < 4; ++p) gb[p] = global_bits(P.out[p]);
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
                     if (g) gi ^= gb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     st_amp(s + gi, r[g ^ (g >> 1)]);
                 }
             } else {
-                UINT sb[4];
-#pragma unroll
-                for (int p = 0; p < 4; ++p) sb[p] = swz(tile_index(P.out[p])) << 4;
-                UINT addr = swz(u0 | tile_index(P.out0)) << 4;
+                UINT addr = (swz(u0) << 4) ^ P.out0_at;
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
-                    if (g) addr ^= sb[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
+                    if (g) addr ^= P.out_at[(g & 1) ? 0 : (g & 2) ? 1 : (g & 4) ? 2 : 3];
                     *reinterpret_cast<double2*>(tile_bytes + addr) = r[g ^ (g >> 1)];
                 }
             }
         }
-        if (!to_hbm) __syncthreads();
+        if (!to_hbm && !(P.flags & PH_SAME_NEXT)) __syncthreads();  // the next phase's cosets are these: each thread's own
     }
-    if (!hbm_last) tile_rows_store<THREADS>(s, tile, base | lo_off, hi_off, tsize);
+    if (!hbm_last) tile_rows_store<threads>(s, tile, base | lo_off, hi_off, tsize);
     __syncthreads();
 }
 
@@ -450,7 +440,7 @@ template <class E>
 __global__ void __launch_bounds__(kStThreads, 2) k_staged_pass(E* __restrict__ s, const __grid_constant__ StPassArgs a) {
     extern __shared__ double2 st_tile[];
     __shared__ ITYPE hi_off[16];
-    staged_tile<kTileBits, kStThreads>(s, a, blockIdx.x, st_tile, hi_off);
+    staged_tile<kTileBits>(s, a, blockIdx.x, st_tile, hi_off);
 }
 
 // Opt k_staged_pass in to 64 KiB of dynamic shared memory, once per device.
@@ -462,10 +452,9 @@ static int staged_allow_smem() {
     std::lock_guard<std::mutex> lock(mu);
     if ((int)done.size() <= dev) done.resize(dev + 1, 0);
     if (!done[dev]) {
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int)(sizeof(double2) << kTileBits)));
-        QS_CUDA_CHECK(cudaFuncSetAttribute(k_staged_pass<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int)(sizeof(double2) << kTileBits)));
+        for (const void* f : {(const void*)k_staged_pass<double2>, (const void*)k_staged_pass<float2>})
+            QS_CUDA_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                (int)(sizeof(double2) << kTileBits)));
         done[dev] = 1;
     }
     return QS_OK;
@@ -489,6 +478,15 @@ static bool stageable(const GateRec& g) {
         case QS_GATE_DIAGONAL: return g.targets.size() == 1;
         default: return false;
     }
+}
+
+// Whether a gate acts on a phase's registers as a matrix or a channel (build_pass_program's `move`): one that
+// flips, or is diagonal, does not.
+static bool mixes_registers(const GateRec& g) {
+    if (g.depol) return true;
+    if (g.kind != QS_GATE_DENSE) return false;
+    const cd zero(0.);
+    return g.targets.size() > 1 || !((g.matrix[0] == zero && g.matrix[3] == zero) || (g.matrix[1] == zero && g.matrix[2] == zero));
 }
 
 // A gate as the scheduler sees it.
@@ -648,6 +646,81 @@ static void lane_order(StPhase* P, int m) {
     for (int i = 0; i < 8; ++i) P->order[i] = i < k ? rest[i] : 0;
 }
 
+// A phase's gates for the generic kernels, which rotate along register bits only.  A CNOT relabels registers (for
+// nothing: the coset is read or written under another order), so a rotation must come after those relabellings
+// that the phase can start with and before the others; where it cannot, a new phase starts on the same tile bits
+// (the coset goes through shared memory).  Phases with matrices or channels stay whole: their CNOTs are steps.
+struct Segment {
+    std::vector<int> gates;
+    uint8_t in[4] = {1, 2, 4, 8};  // StPhase::in
+};
+template <class F>
+static std::vector<Segment> relabel_segments(const std::vector<GateRec>& gates, const std::vector<int>& phase, F reg) {
+    std::vector<Segment> out;
+    for (int gi : phase)
+        if (mixes_registers(gates[gi])) {
+            out.emplace_back();
+            out.back().gates = phase;
+            return out;
+        }
+    struct Labels {  // functional and vector of each qubit over the register's index
+        UINT f[4] = {1, 2, 4, 8}, v[4] = {1, 2, 4, 8};
+        void relabel(int kind, int a, int b) {
+            if (kind == QS_GATE_CNOT) {
+                f[b] ^= f[a];
+                v[a] ^= v[b];
+            } else if (kind == QS_GATE_SWAP) {
+                std::swap(f[a], f[b]);
+                std::swap(v[a], v[b]);
+            }
+        }
+    };
+    struct Item {
+        int gate, kind, a, b;
+    };
+    std::vector<Item> todo, left;
+    for (int gi : phase) {
+        const GateRec& g = gates[gi];
+        const int a = reg(g.targets[0]);
+        todo.push_back({gi, g.kind, a, g.targets.size() > 1 ? reg(g.targets[1]) : a});
+    }
+    while (!todo.empty()) {
+        // relabellings before any rotation of their qubits: the phase starts with them undone, so that they end
+        // on register bits
+        Labels L;
+        UINT turned = 0;
+        std::vector<const Item*> lead;
+        for (const Item& i : todo) {
+            const UINT bits = (1u << i.a) | (1u << i.b);
+            const bool moves = i.kind == QS_GATE_CNOT || i.kind == QS_GATE_SWAP;
+            if (i.kind == QS_GATE_RX || i.kind == QS_GATE_RY || (bits & turned)) turned |= bits;
+            else if (moves) lead.push_back(&i);
+        }
+        for (size_t k = lead.size(); k-- > 0;) L.relabel(lead[k]->kind, lead[k]->a, lead[k]->b);
+        out.emplace_back();
+        Segment& S = out.back();
+        for (int k = 0; k < 4; ++k) {
+            S.in[k] = 0;
+            for (int b = 0; b < 4; ++b) S.in[k] |= (uint8_t)(((L.f[b] >> k) & 1u) << b);
+        }
+        UINT blocked = 0;
+        left.clear();
+        for (const Item& i : todo) {
+            const UINT bits = (1u << i.a) | (1u << i.b);
+            const bool rotation = i.kind == QS_GATE_RX || i.kind == QS_GATE_RY;
+            if ((bits & blocked) || (rotation && (L.f[i.a] != L.v[i.a] || (L.v[i.a] & (L.v[i.a] - 1))))) {
+                blocked |= bits;
+                left.push_back(i);
+                continue;
+            }
+            S.gates.push_back(i.gate);
+            L.relabel(i.kind, i.a, i.b);
+        }
+        todo.swap(left);
+    }
+    return out;
+}
+
 void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int tile_bits, bool spec) {
     H->passes = plan_passes(gates, n, tile_bits);
     const std::vector<PassPlan>& passes = H->passes;
@@ -723,11 +796,17 @@ void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int 
                     regbit[b] = nb;
                     ph.bits[nb++] = (uint8_t)b;
                 }
+            lane_order(&ph, m);
+            auto rb = [&](UINT gq) { return (uint8_t)regbit[local[gq]]; };
+            std::vector<Segment> segments(1);
+            if (spec) segments[0].gates = best;
+            else segments = relabel_segments(gates, best, rb);
+            for (const Segment& segment : segments) {
+            std::copy(segment.in, segment.in + 4, ph.in);
             ph.op_begin = (uint32_t)ops.size();
-            for (int gi : best) {
+            for (int gi : segment.gates) {
                 const GateRec& g = gates[gi];
                 StOp op{};
-                auto rb = [&](UINT gq) { return (uint8_t)regbit[local[gq]]; };
                 op.param = (uint32_t)pool.size();
                 if (g.depol) {
                     op.kind = g.depol == 1 ? ST_DEPOL1 : ST_DEPOL2;
@@ -781,8 +860,9 @@ void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int 
                 ops.push_back(op);
             }
             ph.op_count = (uint32_t)(ops.size() - ph.op_begin);
-            lane_order(&ph, m);
+            ph.flags = &segment != &segments.back() ? PH_SAME_NEXT : 0;
             phases.push_back(ph);
+            }
             size_t at = 0;  // best lists todo's gates in order
             todo.erase(std::remove_if(todo.begin(), todo.end(),
                            [&](const Todo& t) { return at < best.size() && best[at] == t.gate && (++at, true); }),
@@ -790,8 +870,22 @@ void make_host_plan(const std::vector<GateRec>& gates, UINT n, HostPlan* H, int 
         }
         std::vector<PhaseProgram> prog = build_pass_program(phases.data() + ph0, phases.size() - ph0, ops.data(), pool.data());
         for (size_t i = 0; i < prog.size(); ++i) {
-            if (!spec) encode_program(prog[i], &H->steps, &H->params, &phases[ph0 + i]);
-            else H->programs.push_back(std::move(prog[i]));
+            if (spec) {
+                H->programs.push_back(std::move(prog[i]));
+                continue;
+            }
+            StPhase& ph = phases[ph0 + i];
+            encode_program(prog[i], &H->steps, &H->params, &ph);
+            auto at = [&](UINT index) {  // QS_SWZ is linear: the offset of an index is the XOR of its bits' offsets
+                UINT u = 0;
+                for (int b = 0; b < kPhaseBits; ++b) u |= ((index >> b) & 1u) << ph.bits[b];
+                return (uint16_t)(QS_SWZ(u) << 4);
+            };
+            for (int k = 0; k < 4; ++k) {
+                ph.in_at[k] = at(ph.in[k]);
+                ph.out_at[k] = at(ph.out[k]);
+            }
+            ph.out0_at = at(ph.out0);
         }
         pp.push_back({ph0, phases.size() - ph0});
     }
@@ -1354,7 +1448,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) k_batch_staged(const BatchRe
             s_state = (E*)recs[s_rec].state;
         }
         __syncthreads();
-        staged_tile<kBatchTileBits, kBatchThreads>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
+        staged_tile<kBatchTileBits>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
         if (tid == 0) {
             __threadfence();
             atomicAdd(done + s_rec, 1u);
@@ -1463,20 +1557,19 @@ struct BatchLayout {
     int* err(void* b) const { return (int*)(head(b) + 1); }
 };
 
-static int batch_kernel(void* buf, const BatchLayout& L, int nrec, ITYPE total, unsigned long long wait_ns, bool c64,
-    cudaStream_t st) {
+static int batch_kernel(void* buf, const BatchLayout& L, int nrec, ITYPE total, unsigned long long wait_ns,
+    bool c64, cudaStream_t st) {
+    auto kernel = c64 ? (const void*)k_batch_staged<float2> : (const void*)k_batch_staged<double2>;
     int per_sm = 0;
-    if (c64)
-        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<float2>, kBatchThreads, 0));
-    else
-        QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_staged<double2>, kBatchThreads, 0));
+    QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchThreads, 0));
     const ITYPE resident = (ITYPE)std::max(1, per_sm) * sm_count();
     const unsigned grid = (unsigned)std::min<ITYPE>(resident, total);
     const BatchRec* drec = (const BatchRec*)buf;
-    if (c64)
-        k_batch_staged<float2><<<grid, kBatchThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
-    else
-        k_batch_staged<double2><<<grid, kBatchThreads, 0, st>>>(drec, nrec, total, L.head(buf), L.done(buf), L.err(buf), wait_ns);
+    unsigned long long* head = L.head(buf);
+    unsigned* done = L.done(buf);
+    int* err = L.err(buf);
+    void* args[] = {&drec, &nrec, &total, &head, &done, &err, &wait_ns};
+    QS_CUDA_CHECK(cudaLaunchKernel(kernel, dim3(grid), dim3(kBatchThreads), args, 0, st));
     return check_launch("k_batch_staged");
 }
 

@@ -45,19 +45,31 @@ struct StOp {
 // A step of a phase's program for the generic kernels.
 struct StStep {
     uint8_t code, pad;
-    uint16_t mask;   // registers of a diagonal or of signs, or the register pairs of a rotation that run reversed
+    uint16_t mask;   // registers of a diagonal or of signs; a channel's form
     uint32_t param;  // index into the steps' parameter pool
 };
-struct StPhase {
-    uint8_t bits[4];  // tile-local bit positions, ascending
-    uint8_t order[8];  // tile bit of bit k of the coset number
-    uint8_t out0, out[4];  // after the steps register j holds coset index out0 ^ (XOR of out[k] over the bits k of j)
-    uint32_t op_begin, op_count;      // its gates (host)
-    // Its program for the generic kernels: `rounds` of 16 diagonal factors and 4 tangents (16 + 2 entries of the
-    // parameter pool from `param`), then 16 more factors if `tail`; or, where it needs other steps, those.
-    uint32_t rounds, tail, param;
-    uint32_t step_begin, step_count;
+// Bits of StPhase::flags.
+enum PhaseFlag : uint8_t {
+    PH_TURNS_FIRST = 1,  // rounds of tangents, then factors
+    PH_TAIL = 2,         // factors after the last round
+    PH_SAME_NEXT = 4     // the next phase has the same tile bits (relabel_segments)
 };
+// Four 16-byte words, as the kernels read them.
+struct alignas(16) StPhase {
+    uint8_t bits[4];   // tile-local bit positions, ascending
+    uint8_t order[8];  // tile bit of bit k of the coset number
+    uint8_t in[4];     // register j starts with coset index XOR of in[k] over the bits k of j (specialised: j)
+    uint8_t out0, out[4];  // after the steps it holds coset index out0 ^ (XOR of out[k] over the bits k of j)
+    uint8_t flags;
+    uint16_t out0_at, in_at[4], out_at[4];  // in, out0 and out as swizzled byte offsets into the tile
+    // Its program for the generic kernels, from `param` of the parameter pool: `rounds` of 16 diagonal factors and 4
+    // tangents (16 + 2 entries), then 16 more factors (PH_TAIL); or rounds of 4 tangents and 16 factors
+    // (PH_TURNS_FIRST); or, where it needs other steps, those.
+    uint32_t rounds, param;
+    uint32_t step_begin, step_count;
+    uint32_t op_begin, op_count;  // its gates (host)
+};
+static_assert(sizeof(StPhase) == 64, "four words");
 
 // One pass as the code generator sees it: tile qubits, the HBM-direct first/last phase flags, and the
 // programs of its phases.

@@ -121,7 +121,7 @@ void run_code(const StStep& s, const double2* p, cd* r) {
     const int kind = s.code >> 4, V = s.code & 15, A = V >> 2, B = V & 3, a = 1 << A, b = 1 << B;
     for (int j = 0; j < 16; ++j) {
         const int o[4] = {j, j | a, j | b, j | a | b};
-        const bool base1 = !(j & a), base2 = base1 && !(j & b);
+        const bool base1 = !(j & a), base1b = !(j & b), base2 = base1 && base1b;
         if (s.code == 0) {
             if ((s.mask >> j) & 1) r[j] = mul(at(p[j]), r[j]);
         } else if (s.code == 1) {
@@ -137,21 +137,17 @@ void run_code(const StStep& s, const double2* p, cd* r) {
         } else if (kind == 2 && A == B) {
             if (base1) dense(r, o, 2, p);
         } else if (kind == 2) {
-            if (base2) channel1(r[j], r[o[3]], r[o[1]], r[o[2]], p[0].x, p[0].y, s.mask ? p + 1 : nullptr);
+            if (base2) channel1(r[j], r[o[3]], r[o[1]], r[o[2]], p[0].x, p[0].y, nullptr);
+        } else if (kind == 5) {
+            if (base2) channel1(r[j], r[o[3]], r[o[1]], r[o[2]], p[0].x, p[0].y, p + 1);
         } else if (kind == 3 && A != B) {
             if (base2) dense(r, o, 4, p);
         } else if (kind == 3) {
             const int mate = 1 | (1 << (A + 1)), pop[4] = {0, mate, 15 ^ mate, 15};
             if (j == 0) channel2(r, pop, p[0].x, p[0].y, s.mask != 0);
-        } else {
-            const int low = V & -V;
-            if (j & low) continue;
-            int k = 0;  // the pair's number: pairs in ascending order of their lower register
-            for (int i = 0; i < j; ++i) k += !(i & low);
-            const double sign = (s.mask >> k) & 1 ? -1. : 1.;
-            const bool rx = kind >= 6;
-            if (kind == 4 || kind == 6) scaled_rotation(r[j], r[j ^ V], rx ? p[0].x : sign * p[0].x, rx);
-            else rotate(r[j], r[j ^ V], p[0].x, rx ? p[0].y : sign * p[0].y, rx);
+        } else if (base1b) {
+            if (A == 0) scaled_rotation(r[j], r[j | b], p[0].x, false);
+            else rotate(r[j], r[j | b], p[0].x, p[0].y, false);
         }
     }
 }
@@ -163,15 +159,20 @@ void run_generic(const StPhase& P, const HostPlan& H, cd* r) {
     }
     if (P.step_count) return;
     const double2* p = H.params.data() + P.param;
-    for (uint32_t o = 0; o < P.rounds; ++o, p += 18) {
+    auto factors = [&]() {
         for (int j = 0; j < 16; ++j) r[j] = mul(at(p[j]), r[j]);
-        const double t[4] = {p[16].x, p[16].y, p[17].x, p[17].y};
+        p += 16;
+    };
+    for (uint32_t o = 0; o < P.rounds; ++o) {
+        if (!(P.flags & PH_TURNS_FIRST)) factors();
+        const double t[4] = {p[0].x, p[0].y, p[1].x, p[1].y};
         for (int b = 0; b < 4; ++b)
             for (int j = 0; j < 16; ++j)
                 if (!((j >> b) & 1)) scaled_rotation(r[j], r[j | (1 << b)], t[b], false);
+        p += 2;
+        if (P.flags & PH_TURNS_FIRST) factors();
     }
-    if (P.tail)
-        for (int j = 0; j < 16; ++j) r[j] = mul(at(p[j]), r[j]);
+    if (P.flags & PH_TAIL) factors();
 }
 
 void apply_single(const GateRec& g, cd* state, ITYPE dim) {
@@ -227,7 +228,12 @@ void run_pass(const HostPlan& H, size_t pass, bool spec, cd* state, ITYPE dim) {
                     return global(base, v);
                 };
                 cd r[16];
-                for (UINT i = 0; i < 16; ++i) r[i] = state[index(i)];
+                for (UINT j = 0; j < 16; ++j) {
+                    UINT i = 0;
+                    for (int b = 0; b < kPhaseBits; ++b)
+                        if ((j >> b) & 1) i ^= P.in[b];
+                    r[j] = state[index(i)];
+                }
                 if (spec)
                     for (const ProgStep& s : H.programs[at].steps) run_spec(s, r);
                 else

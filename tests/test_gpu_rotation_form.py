@@ -223,3 +223,33 @@ def test_failed_fused_planning_leaves_no_schedule():
     c.set_fusion(0)
     c.update_quantum_state(s, mode="staged_fused")
     assert c.fusion_info()[0] == 0
+
+
+@pytest.mark.parametrize("n", [4, 7, 13, 19])
+@pytest.mark.parametrize("spec", [1, 0])
+def test_permutations_are_exact(n, spec):
+    """CNOT, SWAP and X move amplitudes without arithmetic, tiny ones beside large ones included."""
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=1 << n) * 10.0 ** rng.uniform(-18, 0, size=1 << n) + 0j
+    idx = np.arange(1 << n)
+    c = QuantumCircuit(n)
+    if n >= 7:
+        c.set_specialized(spec)
+    for i in range(8 * n):
+        a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+        if i % 4 < 2:
+            c.add_gate(G.CNOT(a, b))
+            idx = np.where((idx >> a) & 1, idx ^ (1 << b), idx)
+        elif i % 4 == 2:
+            c.add_gate(G.SWAP(a, b))
+            x = ((idx >> a) ^ (idx >> b)) & 1
+            idx = idx ^ (x << a) ^ (x << b)
+        else:
+            c.add_gate(G.X(a))
+            idx = idx ^ (1 << a)
+    want = np.empty_like(v)
+    want[idx] = v
+    s = QuantumState(n)
+    s.load(v)
+    c.update_quantum_state(s)
+    assert np.array_equal(s.get_vector(), want)

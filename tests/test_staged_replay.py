@@ -92,6 +92,32 @@ def test_random_state_circuits(port, spec, k, tile_bits):
         assert np.max(np.abs(got - want)) <= TOL * max(1.0, float(np.max(np.abs(want))))
 
 
+def edge_gate(q, rng):
+    """One-qubit gates at the edges of the rotation form: flips, signs, near-flips, zero angles, non-unitary."""
+    tiny = 2.0 ** -24
+    pool = [G.X(q), G.Y(q), G.Z(q), G.H(q), G.S(q), G.RX(q, np.pi), G.RY(q, np.pi), G.RY(q, np.pi - tiny),
+            G.RX(q, np.pi + tiny), G.RY(q, 0.0), G.RZ(q, np.pi), G.U3(q, np.pi, 0.3, -1.0), G.U3(q, 1e-9, 2.0, 1.0),
+            G.DenseMatrix(q, np.array([[1.1, 0.2j], [0.3, 0.8 - 0.1j]])), G.DiagonalMatrix([q], [0.9j, -1.1]),
+            G.DenseMatrix(q, np.array([[0.0, 0.9], [-1.2j, 0.0]])), G.DenseMatrix(q, np.array([[0.0, 0.9], [1e-3, 0.0]]))]
+    return pool[int(rng.integers(len(pool)))]
+
+
+@pytest.mark.parametrize("spec", [True, False])
+def test_edge_gates_between_relabellings(port, spec):
+    rng = np.random.default_rng(1)
+    for trial in range(400):
+        n = 4
+        gates = []
+        for _ in range(trial % 25 + 1):
+            a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+            gates.append(edge_gate(int(rng.integers(n)), rng))
+            gates += [[G.CNOT(a, b)], [G.CZ(a, b)], [G.SWAP(a, b)], []][int(rng.choice(4, p=[0.35, 0.25, 0.1, 0.3]))]
+        v = random_state(n, rng)
+        want = v.copy()
+        c = apply_vector(port, gates, want)
+        assert np.max(np.abs(replay(c, v, spec=spec) - want)) <= TOL * max(1.0, float(np.max(np.abs(want))))
+
+
 @pytest.mark.parametrize("spec", [True, False])
 @pytest.mark.parametrize("k,tile_bits", [(0, 12), (0, 5), (2, 11)])
 def test_random_noisy_matrix_circuits(port, spec, k, tile_bits):
@@ -163,3 +189,31 @@ def test_long_products_of_non_unitary_diagonals_in_one_pass(port, spec):
     got = replay(c, v, spec=spec)
     assert 0 < np.max(np.abs(want)) < 1e-180
     assert np.max(np.abs(got - want)) <= 10 * TOL * float(np.max(np.abs(want)))
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("k", [0, 2])
+def test_permutations_are_exact(spec, k):
+    """CNOT, SWAP and X move amplitudes without arithmetic: a tiny amplitude beside a large one stays as it is,
+    between rotations on other qubits too."""
+    n = 7
+    rng = np.random.default_rng(6)
+    v = rng.normal(size=1 << n) * 10.0 ** rng.uniform(-18, 0, size=1 << n) + 0j
+    idx = np.arange(1 << n)
+    c = QuantumCircuit(n)
+    for _ in range(60):
+        a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+        r = rng.random()
+        if r < 0.6:
+            c.add_gate(G.CNOT(a, b))
+            idx = np.where((idx >> a) & 1, idx ^ (1 << b), idx)
+        elif r < 0.8:
+            c.add_gate(G.SWAP(a, b))
+            x = ((idx >> a) ^ (idx >> b)) & 1
+            idx = idx ^ (x << a) ^ (x << b)
+        else:
+            c.add_gate(G.X(a))
+            idx = idx ^ (1 << a)
+    want = np.empty_like(v)
+    want[idx] = v
+    assert np.array_equal(replay(c, v, k, spec), want)
