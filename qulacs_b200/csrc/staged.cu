@@ -21,7 +21,7 @@
 // threads for a 2^12-amplitude tile, where 128 threads took two in turn), rotations in place of matrices and
 // rounds (run_rounds) brought the layered circuit on 16 qubits from 0.43 to 0.20 ms; CNOTs as relabellings of the
 // coset's addresses (relabel_segments; H CZ H on the target before, 42 phases with 197 rounds against 87 with 81)
-// further, with the record of a phase read as four words (some forty loads field by field).  20 layers of
+// to 0.151, with the record of a phase read as four words (some forty loads field by field: 0.157).  20 layers of
 // U3 + CZ on 26 qubits took 46.9 ms step by step and 26.5 in rounds (specialised: 16.0).
 #include <algorithm>
 #include <atomic>
@@ -303,7 +303,8 @@ __device__ __forceinline__ void tile_rows_store(T* __restrict__ s, const double2
 // state's type E (complex128, or complex64 widened on load and rounded on store).  One 16-amplitude coset per
 // thread and phase, for the cosets of the largest tile.  Ends with a CTA barrier so the shared buffers can be
 // reused immediately.
-template <int MAX_BITS, class E>
+// STEPS: whether a phase may be a list of steps; without, every phase is rounds.
+template <int MAX_BITS, bool STEPS, class E>
 __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs& a, ITYPE T, double2* tile,
     ITYPE* hi_off) {
     constexpr int tb = MAX_BITS - kPhaseBits;
@@ -407,9 +408,15 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
                     r[g ^ (g >> 1)] = *reinterpret_cast<const double2*>(tile_bytes + addr);
                 }
             }
-            if (P.step_count == 0) run_rounds(P, r, a.pool + P.param);
-            else
-                for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
+            if constexpr (STEPS) {
+                if (P.step_count == 0) {
+                    run_rounds(P, r, a.pool + P.param);
+                } else {
+                    for (UINT o = 0; o < P.step_count; ++o) apply_step(a.steps[P.step_begin + o], r, a.pool);
+                }
+            } else {
+                run_rounds(P, r, a.pool + P.param);
+            }
             // register j goes to coset index out0 ^ (XOR of out[k] over the bits k of j)
             if (to_hbm) {
                 ITYPE gb[4], gi = g0 | global_bits(P.out0);
@@ -435,12 +442,24 @@ __device__ __forceinline__ void staged_tile(E* __restrict__ s, const StPassArgs&
     __syncthreads();
 }
 
-// One CTA per tile; the tile (2^m x 16 bytes, up to 64 KiB) is dynamic shared memory.
-template <class E>
-__global__ void __launch_bounds__(kStThreads, 2) k_staged_pass(E* __restrict__ s, const __grid_constant__ StPassArgs a) {
+// One CTA per tile; the tile (2^m x 16 bytes, up to 64 KiB) is dynamic shared memory.  CTAS: per SM.
+template <class E, bool STEPS, int CTAS>
+__global__ void __launch_bounds__(kStThreads, CTAS) k_staged_pass(E* __restrict__ s, const __grid_constant__ StPassArgs a) {
     extern __shared__ double2 st_tile[];
     __shared__ ITYPE hi_off[16];
-    staged_tile<kTileBits>(s, a, blockIdx.x, st_tile, hi_off);
+    staged_tile<kTileBits, STEPS>(s, a, blockIdx.x, st_tile, hi_off);
+}
+template <class E>
+using PassKernel = void (*)(E* __restrict__, StPassArgs);
+// Two CTAs of 256 threads per SM leave 128 registers: enough for rounds, not for lists of steps (1.2 KB of spill).
+// A state of no more tiles than SMs has one CTA on each either way: without the bound its kernels need 184 to 190
+// registers and read further ahead.  In us with one bound for all, and so: 10 qubits, layered 65 48, U3 + CZ 75 56;
+// 32 two-qubit matrices at 8 qubits 44 36, 64 at 16 qubits 124 110.
+template <class E>
+static PassKernel<E> pass_kernel(bool steps, ITYPE tiles) {
+    const bool few = tiles <= (ITYPE)sm_count();
+    return steps ? (few ? k_staged_pass<E, true, 1> : k_staged_pass<E, true, 2>)
+                 : (few ? k_staged_pass<E, false, 1> : k_staged_pass<E, false, 2>);
 }
 
 // Opt k_staged_pass in to 64 KiB of dynamic shared memory, once per device.
@@ -452,7 +471,10 @@ static int staged_allow_smem() {
     std::lock_guard<std::mutex> lock(mu);
     if ((int)done.size() <= dev) done.resize(dev + 1, 0);
     if (!done[dev]) {
-        for (const void* f : {(const void*)k_staged_pass<double2>, (const void*)k_staged_pass<float2>})
+        for (const void* f : {(const void*)k_staged_pass<double2, false, 1>, (const void*)k_staged_pass<double2, false, 2>,
+                 (const void*)k_staged_pass<double2, true, 1>, (const void*)k_staged_pass<double2, true, 2>,
+                 (const void*)k_staged_pass<float2, false, 1>, (const void*)k_staged_pass<float2, false, 2>,
+                 (const void*)k_staged_pass<float2, true, 1>, (const void*)k_staged_pass<float2, true, 2>})
             QS_CUDA_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                 (int)(sizeof(double2) << kTileBits)));
         done[dev] = 1;
@@ -596,6 +618,7 @@ struct DevPass {
     int gate;
     StPassArgs args;
     size_t phase_begin = 0;  // the pass's phases in StagedPlan::phases
+    bool steps = false;      // a phase is a list of steps
     void* spec = nullptr;    // specialised kernel of this pass (pass_codegen.cpp), if compiled
     std::vector<double2> spec_params;  // its parameter block
 };
@@ -603,7 +626,7 @@ struct DevPass {
 template <class E>
 static void launch_pass(E* state, const DevPass& d, ITYPE tiles, cudaStream_t st) {
     const size_t smem = sizeof(double2) << d.args.m;  // the tile is FP64 for either state type
-    k_staged_pass<E><<<(unsigned)tiles, kStThreads, smem, st>>>(state, d.args);
+    pass_kernel<E>(d.steps, tiles)<<<(unsigned)tiles, kStThreads, smem, st>>>(state, d.args);
 }
 
 struct StagedPlan {
@@ -943,6 +966,7 @@ static int upload_plan(const HostPlan& H, ITYPE dim, std::shared_ptr<StagedPlan>
             }
             d.args.phases = dph + pp[i].phase_begin;
             d.phase_begin = pp[i].phase_begin;
+            for (size_t ph = 0; ph < pp[i].nphases; ++ph) d.steps = d.steps || phases[d.phase_begin + ph].step_count;
             d.args.steps = dst;
             d.args.pool = dpa;
         }
@@ -1404,7 +1428,7 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     return v;
 }
 
-template <class E>
+template <class E, bool STEPS>
 __global__ void __launch_bounds__(kBatchThreads, 3) k_batch_staged(const BatchRec* __restrict__ recs, int nrec,
     ITYPE total, unsigned long long* head, unsigned* done, int* err, unsigned long long wait_ns) {
     __shared__ double2 tile[1 << kBatchTileBits];
@@ -1448,7 +1472,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) k_batch_staged(const BatchRe
             s_state = (E*)recs[s_rec].state;
         }
         __syncthreads();
-        staged_tile<kBatchTileBits>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
+        staged_tile<kBatchTileBits, STEPS>(s_state, s_args, s_item - recs[s_rec].prefix, tile, hi_off);
         if (tid == 0) {
             __threadfence();
             atomicAdd(done + s_rec, 1u);
@@ -1472,9 +1496,10 @@ static int ensure_batch_plan(Circuit& c, ITYPE dim) {
 // `wait_ns`: the dependency wait limit; `self_dep` >= 0 makes that work record depend on itself (a
 // counter nothing can complete), which only the wait-expiry check below uses.
 // The work records of a batch (plans missing from the circuits' caches built first: FP64 fusion and
-// host planning on host threads in parallel, uploads afterwards) and the number of work items.
+// host planning on host threads in parallel, uploads afterwards), the number of work items, and whether any
+// of their phases is a list of steps.
 static int batch_records(Circuit* const* cs, void* const* states, UINT count, std::vector<BatchRec>* recs,
-    ITYPE* total_out) {
+    ITYPE* total_out, bool* steps) {
     for (UINT i = 0; i < count; ++i)
         if (cs[i]->n < kPhaseBits) return set_error(QS_ERR_NOT_SUPPORTED, "batch: circuits need at least 4 qubits");
     {
@@ -1534,6 +1559,7 @@ static int batch_records(Circuit* const* cs, void* const* states, UINT count, st
             r.dep = last[i];
             last[i] = (int)recs->size();
             total += r.tiles;
+            *steps = *steps || passes[i][p]->steps;
             recs->push_back(r);
         }
     *total_out = total;
@@ -1557,9 +1583,10 @@ struct BatchLayout {
     int* err(void* b) const { return (int*)(head(b) + 1); }
 };
 
-static int batch_kernel(void* buf, const BatchLayout& L, int nrec, ITYPE total, unsigned long long wait_ns,
+static int batch_kernel(void* buf, const BatchLayout& L, int nrec, ITYPE total, bool steps, unsigned long long wait_ns,
     bool c64, cudaStream_t st) {
-    auto kernel = c64 ? (const void*)k_batch_staged<float2> : (const void*)k_batch_staged<double2>;
+    auto kernel = c64 ? (steps ? (const void*)k_batch_staged<float2, true> : (const void*)k_batch_staged<float2, false>)
+                      : (steps ? (const void*)k_batch_staged<double2, true> : (const void*)k_batch_staged<double2, false>);
     int per_sm = 0;
     QS_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchThreads, 0));
     const ITYPE resident = (ITYPE)std::max(1, per_sm) * sm_count();
@@ -1592,8 +1619,9 @@ int batch_update(Circuit* const* cs, void* const* states, UINT count, cudaStream
     for (size_t i = 0; i < solo_cs.size(); ++i) QS_TRY(ensure_c64_plan(*solo_cs[i], 1ULL << solo_cs[i]->n));
     std::vector<BatchRec> recs;
     ITYPE total = 0;
+    bool steps = false;
     if (!shared_cs.empty())
-        QS_TRY(batch_records(shared_cs.data(), shared_st.data(), (UINT)shared_cs.size(), &recs, &total));
+        QS_TRY(batch_records(shared_cs.data(), shared_st.data(), (UINT)shared_cs.size(), &recs, &total, &steps));
     if (!solo_cs.empty()) QS_TRY(staged_allow_smem());
     for (size_t i = 0; i < solo_cs.size(); ++i) {
         const ITYPE dim = 1ULL << solo_cs[i]->n;
@@ -1616,7 +1644,7 @@ int batch_update(Circuit* const* cs, void* const* states, UINT count, cudaStream
     QS_TRY(scratch(st, L.bytes, &buf));
     QS_CUDA_CHECK(cudaMemcpyAsync(buf, recs.data(), L.brec, cudaMemcpyHostToDevice, st));
     QS_CUDA_CHECK(cudaMemsetAsync(L.done(buf), 0, L.zero_bytes, st));
-    QS_TRY(batch_kernel(buf, L, (int)recs.size(), total, wait_ns, c64, st));
+    QS_TRY(batch_kernel(buf, L, (int)recs.size(), total, steps, wait_ns, c64, st));
     int err = 0;
     QS_CUDA_CHECK(cudaMemcpyAsync(&err, L.err(buf), sizeof(int), cudaMemcpyDeviceToHost, st));
     QS_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -1721,7 +1749,8 @@ extern "C" QS_API int qs_batch_graph_create(const qs_circuit_t* circuits, void* 
     }
     std::vector<qs::BatchRec> recs;
     ITYPE total = 0;
-    QS_TRY(qs::batch_records(cs.data(), states, count, &recs, &total));
+    bool steps = false;
+    QS_TRY(qs::batch_records(cs.data(), states, count, &recs, &total, &steps));
     if (recs.empty()) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "batch graph: no passes to run");
     auto G = std::make_unique<qs::GraphExec>();
     const qs::BatchLayout L(recs.size());
@@ -1739,7 +1768,7 @@ extern "C" QS_API int qs_batch_graph_create(const qs_circuit_t* circuits, void* 
                            : qs_initialize_quantum_state(states[i], dim, st));
             }
         QS_CUDA_CHECK(cudaMemsetAsync(L.done(dev), 0, L.zero_bytes, st));
-        QS_TRY(qs::batch_kernel(dev, L, (int)recs.size(), total, qs::kBatchWaitNs, c64 != 0, st));
+        QS_TRY(qs::batch_kernel(dev, L, (int)recs.size(), total, steps, qs::kBatchWaitNs, c64 != 0, st));
         QS_CUDA_CHECK(cudaMemcpyAsync(host_err, L.err(dev), sizeof(int), cudaMemcpyDeviceToHost, st));
         return QS_OK;
     }));

@@ -77,3 +77,22 @@ def test_kernels_depend_on_structure_not_angles():
         srcs.append(c.specialized_source(0))
     assert srcs[0] == srcs[1]
     assert "__grid_constant__ PassParams P" in srcs[0]
+
+
+@pytest.mark.skipif(not os.path.exists(NVCC) and shutil.which("nvcc") is None, reason="nvcc not available")
+def test_generic_pass_kernels_do_not_spill(tmp_path):
+    """k_staged_pass keeps a coset and its temporaries in registers wherever its phases are rounds, and for step
+    lists where one CTA has an SM to itself."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([NVCC, "-cubin", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3",
+                        "--expt-relaxed-constexpr", "-Xptxas", "-v", f"-I{root}/include", "-o", str(tmp_path / "s.cubin"),
+                        os.path.join(root, "qulacs_b200", "csrc", "staged.cu")], capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stderr[-3000:]
+    spill = {}
+    for name, stores in re.findall(r"Compiling entry function '(\S*k_staged_pass\S*)'.*?(\d+) bytes spill stores", r.stderr, re.S):
+        # template arguments: amplitude type, steps, CTAs per SM
+        spill[re.search(r"I(\S*?)Lb(\d)ELi(\d)E", name).groups()] = int(stores)
+    assert len(spill) == 8
+    for (kind, steps, ctas), stores in spill.items():
+        if steps == "0" or ctas == "1":
+            assert stores == 0, (kind, steps, ctas, stores)
