@@ -162,12 +162,15 @@ static cl xdiv(const cl& x, const cl& y) {  // |y| near 1
     return cl(z.real() / n, z.imag() / n);
 }
 
-// Whether |z| is 1 up to the rounding of a few double-precision operations.
-static bool is_unit(const cl& z) { return std::abs(xnorm(z) - 1.L) <= 0x1p-49L; }
+// What rounding leaves of the unitarity of a matrix computed in double precision (16 ulp: QR factors are off by up
+// to 6, matrix exponentials by 11).  A matrix further off is applied as it is given.
+constexpr ld kUnitTol = 0x1p-48L;
+static bool is_unit(const cl& z) { return std::abs(xnorm(z) - 1.L) <= kUnitTol; }
 
-static bool is_unitary2(const cl* u) {
+// `gates`: how many matrices were multiplied.
+static bool is_unitary2(const cl* u, int gates = 1) {
     const cl d = xmul(std::conj(u[0]), u[1]) + xmul(std::conj(u[2]), u[3]);
-    constexpr ld tol = 1e-13L;
+    const ld tol = kUnitTol * gates;
     return std::abs(xnorm(u[0]) + xnorm(u[2]) - 1.L) <= tol && std::abs(xnorm(u[1]) + xnorm(u[3]) - 1.L) <= tol &&
            xnorm(d) <= tol * tol;
 }
@@ -221,6 +224,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
     enum Core { NONE, REAL, RX, MATRIX };
     struct Qubit {
         Core core = NONE;
+        int len = 0;          // matrices in it
         ld c = 1.L, s = 0.L;  // REAL: {c, s; -s, c}; RX: {c, i s; i s, c}
         cl m[4];              // MATRIX
         bool post = false, post_free = false, post_unit = true;
@@ -282,7 +286,9 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         const bool post = k.post, post_free = k.post_free, post_unit = k.post_unit;
         const cl p0 = k.p0, p1 = k.p1;
         Core core = k.core;
+        const int len = k.len;
         k.core = NONE;
+        k.len = 0;
         k.post = k.post_free = false;
         k.post_unit = true;
         k.p0 = k.p1 = 1.L;
@@ -313,7 +319,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
                 out.push_back(x);
                 if (is_unit(u[1]) && is_unit(u[2])) carry(q, u[1], u[2], false);
                 else diagonal(q, u[1], u[2], false);
-            } else if (is_unitary2(u)) {
+            } else if (is_unitary2(u, len)) {
                 ld c, s;
                 cl q1, e0, e1;
                 zyz(u, &c, &s, &q1, &e0, &e1);
@@ -338,6 +344,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
     auto add_matrix = [&](UINT q, int kind, const cl* m) {
         Qubit& k = Q[q];
         const cl zero(0.L);
+        ++k.len;
         if (m[1] == zero && m[2] == zero) {
             k.p0 = xmul(m[0], k.p0);
             k.p1 = xmul(m[3], k.p1);

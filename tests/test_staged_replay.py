@@ -217,3 +217,34 @@ def test_permutations_are_exact(spec, k):
     want = np.empty_like(v)
     want[idx] = v
     assert np.array_equal(replay(c, v, k, spec), want)
+
+
+@pytest.mark.parametrize("spec", [True, False])
+@pytest.mark.parametrize("kind", ["scaled", "column", "skewed", "real", "diagonal"])
+def test_matrices_near_unitary_are_applied_as_given(port, kind, spec):
+    """A deviation from unitarity of 5e-14 is in the matrix that a caller gave: 200 of them show as 1e-11."""
+    n, eps = 4, 5e-14
+    rng = np.random.default_rng(9)
+    u = random_unitary(1, rng)
+    if kind == "real":
+        c, s = np.cos(0.7), np.sin(0.7)
+        u = np.array([[c, s], [-s * (1 + eps), c * (1 + eps)]])
+    elif kind == "diagonal":
+        u = np.diag([1.0, (1 + eps) * np.exp(0.3j)])
+    else:
+        u = u @ {"scaled": np.eye(2) * (1 + eps), "column": np.diag([1.0, 1 + 2 * eps]),
+                 "skewed": np.array([[1.0, 2 * eps], [0.0, 1.0]])}[kind]
+    gates = []
+    for i in range(200):
+        gates += [G.DenseMatrix(i % n, u), G.CNOT(i % n, (i + 1) % n)]
+    v = random_state(n, rng)
+    want = v.copy()
+    c = apply_vector(port, gates, want)
+    assert np.max(np.abs(replay(c, v, spec=spec) - want)) <= 5 * TOL
+    rho = random_density_matrix(2, rng)
+    gates = []
+    for i in range(100):
+        gates += [G.DenseMatrix(i % 2, u), G.DepolarizingNoise(i % 2, 0.01), G.RY(i % 2, 0.1)]
+    want = rho.copy()
+    c = apply_matrix(port, gates, want)
+    assert np.max(np.abs(replay(c, rho, spec=spec, dm=True) - want)) <= 5 * TOL
