@@ -450,9 +450,10 @@ QS_API int qs_circuit_add_gate(qs_circuit_t circuit, int kind, const QS_UINT* ta
 QS_API int qs_circuit_gate_count(qs_circuit_t circuit, QS_UINT* out);
 QS_API int qs_circuit_update_quantum_state(
     qs_circuit_t circuit, void* state, QS_ITYPE dim, int exec_mode, void* stream);
-/* Number of HBM passes (kernel launches over the whole state) the staged schedule uses. */
+/* Number of HBM passes (kernel launches over the whole state) of the QS_EXEC_STAGED schedule that runs at dim
+ * amplitudes: the specialised kernels' or the generic kernel's, as qs_circuit_set_specialized has it. */
 QS_API int qs_circuit_pass_count(qs_circuit_t circuit, QS_ITYPE dim, QS_UINT* out);
-/* Host-only statistics of the staged schedule (no reference counterpart): HBM passes, register
+/* Host-only statistics of the same schedule at 2^n amplitudes (no reference counterpart): HBM passes, register
  * phases, operations inside phases, gates run by the gate-by-gate kernels between passes. */
 QS_API int qs_circuit_staged_stats(qs_circuit_t circuit, QS_UINT* passes, QS_UINT* phases, QS_UINT* ops,
     QS_UINT* single_gates);

@@ -1059,13 +1059,21 @@ static bool want_specialized(const Circuit& c, ITYPE dim) {
 // 129), from 19 on there are tiles enough (19: 308 206 255 against 305 218 269; 21: 1118 652 952, 818 586 743).
 static int generic_tile_bits(UINT n) { return n >= 13 && n <= 18 ? kTileBits - 1 : kTileBits; }
 
+// The unfused schedule of a circuit, host part: its gates in rotation form and their plan.
+static void staged_host_plan(const Circuit& c, ITYPE dim, std::vector<GateRec>* gates, HostPlan* H) {
+    const bool spec = want_specialized(c, dim);
+    *gates = rotation_form(c.gates, spec);
+    make_host_plan(*gates, c.n, H, spec ? kTileBits : generic_tile_bits(c.n), spec);
+}
+
 static int ensure_plan(Circuit& c, ITYPE dim) {
     if (c.plan && c.plan->dim == dim) return QS_OK;
-    const bool spec = want_specialized(c, dim);
     std::shared_ptr<StagedPlan> P;
-    std::vector<GateRec> g = rotation_form(c.gates, spec);
-    QS_TRY(build_plan(g, c.n, dim, &P, spec ? kTileBits : generic_tile_bits(c.n), spec));
-    if (spec) QS_TRY(specialize_plan(*P));
+    std::vector<GateRec> g;
+    HostPlan H;
+    staged_host_plan(c, dim, &g, &H);
+    QS_TRY(upload_plan(H, dim, &P));
+    if (want_specialized(c, dim)) QS_TRY(specialize_plan(*P));
     c.rgates.swap(g);
     c.plan = P;
     return QS_OK;
@@ -1271,21 +1279,29 @@ int staged_pass_count(Circuit& c, ITYPE dim, UINT* out) {
         return QS_OK;
     }
     HostPlan H;
-    make_host_plan(rotation_form(c.gates, true), c.n, &H, kTileBits, true);
+    std::vector<GateRec> g;
+    staged_host_plan(c, dim, &g, &H);
     *out = (UINT)H.passes.size();
     return QS_OK;
 }
 
 }  // namespace qs
 
-// Host-only statistics of the staged schedule: HBM passes, register phases, operations in phases,
-// and gates run by the gate-by-gate kernels between passes.
+// Host-only statistics of the QS_EXEC_STAGED schedule that runs at 2^n amplitudes (the specialised kernels' or
+// the generic one's): HBM passes, register phases, operations in phases, and gates run by the gate-by-gate
+// kernels between passes.
 extern "C" QS_API int qs_circuit_staged_stats(qs_circuit_t circuit, QS_UINT* passes, QS_UINT* phases, QS_UINT* ops,
     QS_UINT* single_gates) {
     qs::Circuit* c = reinterpret_cast<qs::Circuit*>(circuit);
     if (!c || !passes || !phases || !ops || !single_gates) return qs::set_error(QS_ERR_INVALID_ARGUMENT, "null argument");
+    if (c->n < (UINT)qs::kPhaseBits) {  // gate by gate
+        *passes = *single_gates = (QS_UINT)c->gates.size();
+        *phases = *ops = 0;
+        return QS_OK;
+    }
     qs::HostPlan H;
-    qs::make_host_plan(qs::rotation_form(c->gates, true), c->n, &H, qs::kTileBits, true);
+    std::vector<qs::GateRec> gates;
+    qs::staged_host_plan(*c, 1ULL << c->n, &gates, &H);
     UINT single = 0;
     for (const qs::PassPlan& p : H.passes) single += p.single ? 1 : 0;
     *passes = (QS_UINT)H.passes.size();

@@ -1,5 +1,6 @@
 """Host logic: synthetic workload shapes, Pauli masks, gate matrices (CPU only)."""
 import numpy as np
+import pytest
 
 from qulacs_b200 import gate as G
 from qulacs_b200 import observable as OB
@@ -65,3 +66,23 @@ def test_staged_planner_pass_counts():
     assert 1 <= p <= 40  # vs 1190 gate-by-gate passes
     c = W.to_circuit(W.layered_rotation_circuit(3, 2, 1), 3)
     assert c.pass_count() == c.get_gate_count()  # below 4 qubits: gate by gate
+
+
+@pytest.mark.parametrize("n", [4, 10, 16, 18, 21, 22])
+def test_staged_statistics_describe_the_schedule_that_runs(n):
+    """Pass counts follow the kernels that a state of this size runs: the generic kernel's tiles and program below
+    2^22 amplitudes, the specialised kernels' from there on, or as the circuit forces them."""
+    c = W.to_circuit(W.layered_rotation_circuit(n, 10, 1), n)
+    default = c.staged_stats()
+    assert c.pass_count() == default[0]
+    c.set_specialized(1)
+    spec = c.staged_stats()
+    c.set_specialized(0)
+    generic = c.staged_stats()
+    assert default == (spec if n >= 22 else generic)
+    assert generic[1] > spec[1]  # phases split where a CNOT relabels
+    if 13 <= n <= 18:
+        assert generic[0] > spec[0]  # smaller tiles
+    three = W.to_circuit(W.layered_rotation_circuit(3, 2, 1), 3)
+    gates = three.get_gate_count()
+    assert three.staged_stats() == (gates, 0, 0, gates)
