@@ -575,11 +575,12 @@ def timed_region(step, steps: int, warmup: int, dist=None, sync=None, make_timer
 
 
 def fp64_per_amplitude(circ) -> float:
-    """FP64 instructions per amplitude of the circuit's staged schedule, counted from the generated pass
-    kernels: per 16-amplitude coset, 4 per diagonal factor or scaled rotation pair, 8 per unscaled one, 16 per
-    pair of a 2 x 2 matrix, 64 per quadruple of a 4 x 4 matrix, 2 per real scale."""
+    """FP64 instructions per amplitude of the circuit's unfused specialised schedule (no gate outside its passes),
+    counted from the generated pass kernels: per 16-amplitude coset, 4 per diagonal factor or scaled rotation
+    pair, 8 per unscaled one, 16 per pair of a 2 x 2 matrix, 64 per quadruple of a 4 x 4 matrix, 2 per real
+    scale; channels: 4 per mixed pair, 6 per sum of populations, 2 per population."""
     cost = {"cmul": 4, "ry_tan": 4, "ry_cot": 4, "rx_tan": 4, "rx_cot": 4, "ry_full": 8, "rx_full": 8,
-            "dense1": 16, "dense2": 64, "rscale": 2}
+            "dense1": 16, "dense2": 64, "rscale": 2, "mix2": 4, "sum4": 6, "axpy": 2}
     total = 0
     for p in range(circ.pass_count()):
         src = circ.specialized_source(p)
@@ -772,7 +773,13 @@ def main():
     # FP64 view of the same work: the instructions of the generated pass kernels (unscaled rotations gate by
     # gate: 4 per amplitude); B200 FP64 CUDA-core peak = 148 SMs x 64 FMA/clk.
     rot = sum(1 for g in gates if g[0] in ("RX", "RY", "RZ"))
-    fp64_instr = (fp64_per_amplitude(circ) if staged_kernel and n >= 7 else 4.0 * rot) * (1 << n)
+    staged_spec, fused_spec, _ = circ.specialized_info()
+    if mode == "gate_by_gate":
+        fp64_instr = 4.0 * rot * (1 << n)
+    elif staged_spec if mode == "staged" else fused_spec and fusion["k"] == 0:
+        fp64_instr = fp64_per_amplitude(circ) * (1 << n)
+    else:  # the generic kernel, or fused blocks: not the schedule that the sources show
+        fp64_instr = None
     fp64_peak = 148 * 64 * 1.965e9
     kernels = kernel_table(state, n, stream) if not args.no_kernel_table else None
 
@@ -893,7 +900,8 @@ def main():
                               "peak_tinstr_s": fp64_peak / 1e12,
                               "frac": fp64_instr / (ms / 1e3) / fp64_peak,
                               "note": "FP64 instructions of the generated pass kernels (scaled rotation 2 per "
-                                      "amplitude, collected diagonals up to 4); nominal 64 FP64 FMA/clk/SM at 1965 MHz"},
+                                      "amplitude, collected diagonals up to 4); nominal 64 FP64 FMA/clk/SM at 1965 MHz"}
+            if fp64_instr is not None else None,
             "kernels": kernels,
             "e2e": {"value": world * len(gates) / (e2e_ms / 1e3), "unit": "gates/s", "ms_per_step": e2e_ms,
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
