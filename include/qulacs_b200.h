@@ -281,8 +281,9 @@ QS_API int qs_expectation_value_pauli_batch(const QS_ITYPE* x_masks, const QS_IT
 QS_API int qs_expectation_value_pauli_weighted(const QS_ITYPE* x_masks, const QS_ITYPE* z_masks,
     const QS_UINT* y_counts, const double* coefs, QS_UINT term_count, const void* state, QS_ITYPE dim,
     void* stream, double out[2]);
-/* The plan qs_expectation_value_pauli_weighted follows for these terms on a state of dim amplitudes,
- * host only (diagnostic; no reference counterpart): *passes_out = passes over the state;
+/* The passes of qs_expectation_value_pauli_weighted for these terms on a state of dim amplitudes (of up to 2^12:
+ * with qs_set_expectation_specialized 0 or 2; by default their strings are one launch of jobs), host only
+ * (diagnostic; no reference counterpart): *passes_out = passes over the state;
  * kind_counts = terms evaluated {Z-only, bit flips within a thread's registers, partner amplitudes
  * from shared memory, partner rows selected per thread, one value each outside the passes}. */
 QS_API int qs_expectation_value_pauli_weighted_plan(const QS_ITYPE* x_masks, const QS_ITYPE* z_masks,
@@ -438,7 +439,8 @@ typedef struct qs_circuit_s* qs_circuit_t;
 
 /* Execution modes of qs_circuit_update_quantum_state. */
 #define QS_EXEC_GATE_BY_GATE 0 /* one kernel per gate: the reference's method */
-#define QS_EXEC_STAGED 1       /* several gates per HBM pass, identical arithmetic per gate */
+#define QS_EXEC_STAGED 1       /* several gates per HBM pass; one-qubit gates as rotations and diagonals: equal to
+                                  gate by gate up to rounding, and exactly where gates only permute */
 #define QS_EXEC_STAGED_FUSED 2 /* runs of gates composed in FP64 into k-qubit dense blocks (k chosen per
                                   circuit by measurement, or forced by qs_circuit_set_fusion), then staged */
 

@@ -12,8 +12,9 @@ class QuantumCircuit:
     """Gate list applied in order by ``update_quantum_state`` (cppsim circuit.cpp:46-57).
 
     ``mode="gate_by_gate"`` launches one kernel per gate (the reference's method);
-    ``mode="staged"`` applies several gates per HBM pass, each with its own arithmetic (specialised passes
-    write one-qubit gates as rotations and diagonals: equal up to rounding);
+    ``mode="staged"`` applies several gates per HBM pass; runs of one-qubit gates are multiplied out and written
+    as rotations and diagonals, so results equal gate-by-gate ones up to rounding (exactly where gates only
+    permute amplitudes);
     ``mode="staged_fused"`` first composes runs of gates into k-qubit dense blocks in FP64 (k chosen
     per circuit by timing, or forced with ``set_fusion``), then stages them.
     """

@@ -1,11 +1,10 @@
 // Specialised staged-pass kernels: one kernel per pass, generated as CUDA C from the pass's schedule and
 // compiled for sm_100a with NVRTC at plan time.
 //
-// The generic pass kernel (k_staged_pass, staged.cu) interprets each phase's op list: per op it loads
-// the op record and its matrix from memory, branches through a 128-case switch, and returns its 16
-// amplitudes to the registers the switch fixed, which costs register moves at every op boundary and an
-// instruction footprint larger than the instruction cache.  Here every tile qubit, phase bit, address offset
-// and register index is a compile-time constant: a phase is the straight-line code of its program
+// The generic pass kernel (k_staged_pass, staged.cu) reads each phase's program from memory: rounds in which a
+// rotation or factor that is not there costs as much as one that is, or, with matrices and channels, steps
+// behind a switch that returns the 16 amplitudes to fixed registers.  Here every tile qubit, phase bit, address
+// offset and register index is a compile-time constant: a phase is the straight-line code of its program
 // (phase_program.hpp), and gate parameters are constant-bank operands.
 //
 // What bounds it: a pass needs one read and one write of the state, 16 bytes through shared memory each
@@ -17,7 +16,6 @@
 //    (12 warps, and the coset loop turned parameters into separate constant loads).
 //  * Lanes run over tile bits whose swizzle vectors are independent (lane_order): the density-matrix
 //    circuit of 12 qubits went from 3.6 to 3.1 ms.
-//
 //  * Plain loads and stores: with streaming hints (.cs) the layered circuit took 141 ms, without them 137.
 //
 // NVRTC is opened at run time (libnvrtc.so.12); the compiled cubin is loaded with cudaLibraryLoadData,
@@ -442,8 +440,8 @@ std::string pass_source(const PassDesc& d, std::vector<double2>* params) {
         if (!to_hbm) o << "  __syncthreads();\n";
     }
     if (!hbm_last) {
-        // batches of 16 rows per thread: the batch's shared-memory loads first, then its streaming
-        // stores; row k's global offset takes k's bits to the tile qubits q[7..]
+        // batches of 16 rows per thread: the batch's shared-memory loads first, then its stores; row k's
+        // global offset takes k's bits to the tile qubits q[tb..]
         const int batch = rows < 16 ? rows : 16;
         o << "#pragma unroll 1\n  for (unsigned k0 = 0; k0 < " << rows << "u; k0 += " << batch << "u) {\n";
         o << "    D2 v[" << batch << "];\n#pragma unroll\n    for (unsigned k = 0; k < " << batch

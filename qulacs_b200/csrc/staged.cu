@@ -1054,9 +1054,10 @@ static bool want_specialized(const Circuit& c, ITYPE dim) {
 
 // Tile size of the generic kernel for a circuit alone.  From 13 to 18 qubits there are at most 64 tiles of 2^12
 // amplitudes for 148 SMs: 2^11 spreads each pass over twice the SMs, at about a third more passes.  U3 + CZ (20
-// layers), HEA (8), layered (10), in us: 16 qubits 215 144 197 against 247 189 214; 18 qubits 267 177 229
-// against 314 215 236.  Up to 12 qubits one tile of the whole state needs one pass (12: 119 72 140 against 127 114
-// 129), from 19 on there are tiles enough (19: 308 206 255 against 305 218 269; 21: 1118 652 952, 818 586 743).
+// layers), HEA (8), layered (10), U3 + random CNOT and CZ (10), in us by 2^12 and 2^11: 13 qubits 145 129 121 132, 118
+// 111 95 106; 16 qubits 218 171 147 203, 190 136 151 187; 18 qubits 282 194 181 225, 231 157 172 202; from 19 on
+// there are tiles enough: 273 202 192 277, 308 203 260 321.  Up to 12 qubits one tile of the whole state needs one
+// pass.
 static int generic_tile_bits(UINT n) { return n >= 13 && n <= 18 ? kTileBits - 1 : kTileBits; }
 
 // The unfused schedule of a circuit, host part: its gates in rotation form and their plan.

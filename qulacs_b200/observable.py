@@ -271,8 +271,9 @@ class Observable:
         return masks_of(self.terms)
 
     def weighted_plan(self, qubit_count: int | None = None) -> dict:
-        """How get_expectation_value evaluates these terms on a state of `qubit_count` qubits (host
-        only): passes over the state and terms per kind of evaluation."""
+        """The passes in which get_expectation_value evaluates these terms on a state of `qubit_count` qubits
+        (host only): passes over the state and terms per kind of evaluation.  Up to 12 qubits it has them only
+        with forced kernels (set_expectation_specialized 0 or 2); by default the strings are one launch of jobs."""
         n = self.qubit_count if qubit_count is None else int(qubit_count)
         xm, zm, ny = self._masks()
         passes = C.c_uint()

@@ -1,8 +1,8 @@
 """Specialised pass kernels, host side: the generated CUDA C of staged passes (plain gates, FP64-fused
 dense blocks, CNOT-folded ops, CZ, SWAP, HBM-direct first/last phases and tile round trips) compiles for
-sm_100a at the pass kernel's occupancy (128 threads, 3 CTAs per SM) with at most a few bytes of spill,
-and gate parameters passed as a kernel-parameter block, so circuits that differ only in angles share a
-kernel."""
+sm_100a at the pass kernel's occupancy (256 threads, 2 CTAs per SM; 128 and 3 with two-qubit matrices) with at
+most a few bytes of spill, and gate parameters passed as a kernel-parameter block, so circuits that differ only
+in angles share a kernel.  The generic pass kernels compile without spill where they can."""
 import os
 import re
 import shutil
