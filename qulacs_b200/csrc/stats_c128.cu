@@ -2040,12 +2040,14 @@ int ev_weighted(const PauliTerm* terms, const double2* coefs, UINT count, const 
     // A small state's terms in one launch, one job per bit-flip string: they read it from the L2 cache, and a pass
     // of the weighted kernel over one or two tiles is a chain of strings in one or two CTAs.  8, 32, 64 and 200
     // strings in us, by passes and so: 11 qubits 61 78 127 210, 58 74 114 183; 12 qubits 53 74 119 217, 52 68 115
-    // 167; 13 qubits 52 76 118 204, 64 78 128 188; 15 qubits 52 74 130 216, 77 92 143 214.  (Forced modes keep the
-    // passes at every size.)
+    // 167; 13 qubits 52 76 118 204, 64 78 128 188; 15 qubits 52 74 130 216, 77 92 143 214.  Where there are passes
+    // (11 and 12 qubits, at least 4 bit flips), they are ahead up to 8 bit flips: 4, 6 and 8 at 12 qubits 41 43 45
+    // against 47 49 51, 12 54 against 52.  (Forced modes keep the passes at every size.)
     std::vector<int> zidx, xidx;
     if (n <= kEvOneLaunchQubits && g_ev_spec_mode.load() == 1)
         for (UINT k = 0; k < count; ++k) (terms[k].x == 0 ? zidx : xidx).push_back((int)k);
-    if (ev_one_launch(zidx.size(), xidx.size())) {
+    const bool passes_ahead = n >= (UINT)kEvTileBits && xidx.size() >= 4 && xidx.size() <= 8;
+    if (ev_one_launch(zidx.size(), xidx.size()) && !passes_ahead) {
         std::vector<double> v(count);
         QS_TRY(ev_listed<T>(terms, zidx, xidx, s, dim, st, v.data()));
         out[0] = out[1] = 0.;

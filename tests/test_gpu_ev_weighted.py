@@ -214,3 +214,23 @@ def test_small_states_at_the_edges_of_one_launch(port, n, flips, z_only, c64):
     want = np.array([port.expectation_value(tl, ids, v) for _, tl, ids in ts])
     assert np.max(np.abs(obs.term_values(s) - want)) <= EV_TOL
     assert abs(obs.get_expectation_value(s) - float(np.dot([t[0] for t in ts], want))) <= EV_TOL * len(ts)
+
+
+@pytest.mark.parametrize("c64", [False, True])
+@pytest.mark.parametrize("n", [10, 11, 12])
+@pytest.mark.parametrize("flips", [3, 4, 8, 9])
+def test_few_strings_by_passes_or_in_one_launch(port, n, flips, c64):
+    """Both sides of the rule that keeps 4 to 8 bit-flip strings at 11 and 12 qubits in passes, with Z-only ones."""
+    rng = np.random.default_rng(31 * n + flips)
+    v = random_state(n, rng)
+    if c64:
+        v = v.astype(np.complex64).astype(np.complex128)
+    s = QuantumStateC64(n) if c64 else QuantumState(n)
+    s.load(v)
+    ts = []
+    for i in range(flips):
+        a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+        ts.append((float(rng.normal()), [a, b], [1 + i % 2, 1 + i % 3]))
+    ts += [(0.5, [q], [3]) for q in range(2)]
+    want = sum(t[0] * port.expectation_value(t[1], t[2], v) for t in ts)
+    assert abs(W.to_observable(ts, n).get_expectation_value(s) - want) <= EV_TOL * len(ts)
