@@ -1095,16 +1095,20 @@ int run_staged(Circuit& c, void* state, ITYPE dim, cudaStream_t st) {
 // when the circuit runs specialised passes, else the generic one -- on a scratch buffer of whole tiles
 // (the pass's ops only see tile-local bits, so its tile qubits are remapped to 0..m-1); a pass costs at
 // least its HBM time, and gates left outside passes cost one HBM pass each (dense 5- and 6-qubit
-// kernels more).  The best k is then also tried with 2^11-amplitude tiles (the tile shape).
+// kernels more), or their launch.  The best k is then also tried with 2^11-amplitude tiles (the tile shape).
 constexpr int kTuneMaxK = 6;
 constexpr int kTuneSlots = kTuneMaxK + 2;  // k = 0..6 at 2^12 tiles, then the best k at 2^11 tiles
 constexpr double kTuneHbmBytesPerSec = 6.5e12;  // B200 streaming copy bandwidth
 
-static double single_gate_factor(const GateRec& g) {
+// A gate outside the passes: HBM passes, but at least what its launch and arithmetic take on a state in the L2
+// cache (8 to 18 qubits: 3 to 4.2 us up to three targets, 6.2 to 7.8 for four, 10 to 13 for five, 26 to 27 for
+// six).  By the HBM time alone 30 five-qubit blocks at 14 qubits cost nothing: 412 us were chosen over 122.
+static double single_gate_ms(const GateRec& g, double hbm_ms) {
     const size_t k = g.targets.size() + g.controls.size();
-    if (g.kind == QS_GATE_DENSE && k == 5) return 2.0;
-    if (g.kind == QS_GATE_DENSE && k >= 6) return 6.5;  // k_denseK_blk: 33 ms against a 5.3 ms pass at 30 qubits
-    return 1.0;
+    const bool dense = g.kind == QS_GATE_DENSE;
+    if (dense && k == 5) return std::max(0.012, 2.0 * hbm_ms);
+    if (dense && k >= 6) return std::max(0.026, 6.5 * hbm_ms);  // k_denseK_blk: 33 ms against a 5.3 ms pass at 30 qubits
+    return std::max(dense && k == 4 ? 0.0065 : 0.0042, hbm_ms);
 }
 
 static int estimate_plan_ms(const std::vector<GateRec>& gates, const StagedPlan& P, ITYPE dim, cudaStream_t st,
@@ -1146,7 +1150,7 @@ static int estimate_plan_ms(const std::vector<GateRec>& gates, const StagedPlan&
     for (size_t i = 0; i < P.passes.size(); ++i) {
         const DevPass& d = P.passes[i];
         if (d.single) {
-            total += hbm_ms * single_gate_factor(gates[d.gate]);
+            total += single_gate_ms(gates[d.gate], hbm_ms);
             continue;
         }
         const ITYPE tiles = dim >> d.args.m;

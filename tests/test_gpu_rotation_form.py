@@ -253,3 +253,14 @@ def test_permutations_are_exact(n, spec):
     s.load(v)
     c.update_quantum_state(s)
     assert np.array_equal(s.get_vector(), want)
+
+
+@pytest.mark.parametrize("n", [8, 13, 16])
+def test_block_size_of_small_states_counts_launches(n):
+    """Blocks of three and more qubits run outside the passes, one launch each: on states that fit the L2 cache the
+    autotuner must not take them for free."""
+    from qulacs_b200 import workloads as W
+    for gates in (W.layered_rotation_circuit(n, 10, 1), W.hea_circuit(n, 8, 1), W.u3_cz_circuit(n, 20, 1)):
+        c = W.to_circuit(gates, n)
+        c.update_quantum_state(QuantumState(n), mode="staged_fused")
+        assert 0 <= c.fusion_info()[0] <= 2
