@@ -16,8 +16,15 @@ using cd = std::complex<double>;
 
 static ITYPE qubit_mask(const GateRec& g) {
     ITYPE m = 0;
-    for (UINT q : g.qubits()) m |= 1ULL << q;
+    for (UINT q : g.targets) m |= 1ULL << q;
+    for (UINT q : g.controls) m |= 1ULL << q;
     return m;
+}
+// One more than the highest qubit of a gate list.
+static UINT qubit_range(const std::vector<GateRec>& G) {
+    ITYPE m = 0;
+    for (const GateRec& g : G) m |= qubit_mask(g);
+    return m ? 64u - (UINT)__builtin_clzll(m) : 0u;
 }
 
 void apply_gate_to_block(std::vector<cd>& U, int kb, const GateRec& g, const std::vector<int>& pos) {
@@ -205,6 +212,9 @@ static void xmatrix(const GateRec& g, cl* m) {
         case QS_GATE_RX: m[0] = m[3] = c; m[1] = m[2] = cl(0.L, s); return;
         case QS_GATE_RY: m[0] = m[3] = c; m[1] = s; m[2] = -s; return;
         case QS_GATE_RZ: m[0] = cl(c, s); m[3] = cl(c, -s); m[1] = m[2] = 0.L; return;
+        case QS_GATE_DENSE:
+            for (int i = 0; i < 4; ++i) m[i] = cl(g.matrix[i].real(), g.matrix[i].imag());
+            return;
         default: break;
     }
     const std::vector<cd> d = g.dense_matrix();
@@ -232,9 +242,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         bool any = false, any_free = false;
         cl d = 1.L;           // carried; a product of quotients of unit entries
     };
-    UINT n = 0;
-    for (const GateRec& g : G)
-        for (UINT q : g.qubits()) n = std::max(n, q + 1);
+    const UINT n = qubit_range(G);
     std::vector<Qubit> Q(n);
     std::vector<GateRec> out;
     out.reserve(2 * G.size() + 4);
@@ -249,7 +257,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         d.xd[0] = d0;
         d.xd[1] = d1;
         d.free_phase = free_phase;
-        out.push_back(d);
+        out.push_back(std::move(d));
     };
     auto carry = [&](UINT q, const cl& d0, const cl& d1, bool free_phase) {  // diag(d0, d1) after the carried one
         Qubit& k = Q[q];
@@ -273,7 +281,7 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
         r.extended = true;
         r.xc = c;
         r.xs = s;
-        out.push_back(r);
+        out.push_back(std::move(r));
     };
     auto core_matrix = [](const Qubit& k, cl* m) {
         if (k.core == MATRIX) std::copy(k.m, k.m + 4, m);
@@ -399,7 +407,8 @@ std::vector<GateRec> rotation_form(const std::vector<GateRec>& G, bool spec) {
             add_matrix(g.targets[0], g.kind, m);
             continue;
         }
-        for (UINT q : g.qubits()) end_run(q);
+        for (UINT q : g.targets) end_run(q);
+        for (UINT q : g.controls) end_run(q);
         switch (g.kind) {
             case QS_GATE_CZ:
             case QS_GATE_DIAGONAL: break;
@@ -461,9 +470,7 @@ std::vector<GateRec> executor_gates(const std::vector<GateRec>& G, int k, bool s
 // q1, q2 compose to 1 - (1 - q1)(1 - q2), so runs of (gate, channel) pairs on a qubit become the gates and
 // one channel.
 std::vector<GateRec> merge_depolarizing(const std::vector<GateRec>& G) {
-    UINT n = 0;
-    for (const GateRec& g : G)
-        for (UINT q : g.qubits()) n = std::max(n, q + 1);
+    const UINT n = qubit_range(G);
     std::vector<ld> keep(n, 1.L);  // 1 - strength carried on each qubit
     std::vector<GateRec> out;
     auto flush = [&](UINT q) {
