@@ -776,9 +776,10 @@ def main():
     staged_spec, fused_spec, _ = circ.specialized_info()
     if mode == "gate_by_gate":
         fp64_instr = 4.0 * rot * (1 << n)
-    elif staged_spec if mode == "staged" else fused_spec and fusion["k"] == 0:
+    elif staged_spec if mode == "staged" else fused_spec and fusion["k"] <= 2 and passes == circ.pass_count():
+        # k = 1 and 2 leave this circuit's passes as they are: its blocks are cheaper gate by gate
         fp64_instr = fp64_per_amplitude(circ) * (1 << n)
-    else:  # the generic kernel, or fused blocks: not the schedule that the sources show
+    else:  # the generic kernel, or larger blocks: not the schedule that the sources show
         fp64_instr = None
     fp64_peak = 148 * 64 * 1.965e9
     kernels = kernel_table(state, n, stream) if not args.no_kernel_table else None
